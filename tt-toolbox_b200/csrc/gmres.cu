@@ -1,17 +1,22 @@
 // Device GMRES with Householder orthogonalisation (FP64).
 //
-// Restates dgmresr_hh (fmex/solve3d.c:339-518).  The Arnoldi work outside
-// the matvec is done by three cooperative kernels, each one launch covering
-// a whole sequence of reflector applications:
-//   hh_build  : v_j = P_0 ... P_{j-1} (P_j e_j), normalised       (:396-406)
-//   hh_tail   : w = P_j ... P_0 (B v_j), next reflector, Givens     (:421-473)
-//   hh_correct: upper-triangular solve and the correction x += Q y  (:487-507)
-// plus hh_init for the restart vector (:376-392).  Each reflector needs a
-// global dot product before its update, so the blocks meet at a grid barrier
-// per reflector; the partial sums are reduced in a fixed order, so results
-// are deterministic run to run.  Every barrier wait is bounded: on timeout
-// the kernel raises the context error flag and runs to completion, and the
-// host returns TTG_ERR_TIMEOUT.
+// Restates dgmresr_hh (fmex/solve3d.c:339-518).  The reference applies the
+// reflectors P_r = I - 2 u_r u_r' one after another; each needs a global
+// inner product before its update, so a step that applies j of them one by
+// one meets j grid barriers.  Here the product of the reflectors is kept in
+// compact WY form (Schreiber and Van Loan, SIAM J. Sci. Stat. Comput. 10
+// (1989) 53-57), P_0 ... P_j = I - U T U' with U = [u_0 .. u_j] and T upper
+// triangular, T(j,j) = 2, T(0:j,j) = -2 T U(:,0:j)' u_j: all inner products
+// of a step are taken at once.  Outside the matvec one Arnoldi step is one
+// cooperative launch with two grid barriers:
+//   hh_init   : restart vector, u_0, v_0 = P_0 e_0                 (:376-392)
+//   hh_step   : w = P_j ... P_0 (B v_j), next reflector, Givens    (:421-473),
+//               then v_{j+1} = P_0 ... P_{j+1} e_{j+1}             (:396-406)
+//   hh_correct: triangular solve and the correction x += Q y       (:487-507)
+// Partial sums are reduced in a fixed order, so results are deterministic
+// run to run.  Every barrier wait is bounded: on timeout the kernel raises
+// the context error flag and runs to completion, and the host returns
+// TTG_ERR_TIMEOUT.
 #include <cmath>
 #include <cstring>
 
@@ -22,20 +27,20 @@ namespace ttg {
 
 namespace {
 
-constexpr int HH_THREADS = 256;
+constexpr int HH_THREADS = 512;
+constexpr int HH_WARPS = HH_THREADS / 32;
 constexpr long long BAR_SPIN_LIMIT = 1LL << 24;
 
-// Restart lengths up to which k_hh_tail / k_hh_correct stage their serial
-// sections in shared memory (3 nrestart + 1, nrestart^2 + 2 nrestart doubles).
-constexpr int64_t HH_STAGE_MAX = 1024;
+// Restart lengths up to which k_hh_correct stages R in shared memory.
 constexpr int64_t HH_CORRECT_STAGE_MAX = 64;
 
-size_t hh_tail_smem(int64_t nrestart) {
-  return nrestart <= HH_STAGE_MAX ? sizeof(double) * size_t(3 * nrestart + 1) : 0;
+// Shared memory of k_hh_step: three vectors over the reflectors and the
+// per-warp partial inner products (the Givens section reuses the space).
+size_t hh_step_smem(int64_t nrestart) {
+  return sizeof(double) * size_t(4 * (nrestart + 1) + 4 * HH_WARPS);
 }
-size_t hh_correct_smem(int64_t nrestart) {
-  return sizeof(double) * size_t(nrestart + (nrestart <= HH_CORRECT_STAGE_MAX
-                                                 ? nrestart * nrestart + nrestart : 0));
+size_t hh_correct_smem(int64_t nrestart, int64_t ni) {
+  return sizeof(double) * size_t(3 * ni + (nrestart <= HH_CORRECT_STAGE_MAX ? ni * ni : 0));
 }
 
 struct HhArgs {
@@ -49,9 +54,11 @@ struct HhArgs {
   double* tau;   // nrestart+1
   double* J;     // 2 x nrestart
   double* R;     // nrestart x nrestart
+  double* T;     // (nrestart+1)^2: the WY factor, and its transpose
+  double* TT;
   double* scal;  // [0] nrmrhs [1] curres [2] nrmr [3] exact-flag [4] w[j+1]
-  double* part;  // 2 * gridDim.x
-  unsigned* bar; // [0] count [1] generation [2] reduction parity
+  double* part;  // 2 x (nrestart+2) x gridDim.x partial sums
+  unsigned* bar; // [0] count [1] generation
   int* err;
   int* stop;     // [0] converged flag, [1] step at which it converged
   double tol;    // relative stopping tolerance of the current solve
@@ -109,151 +116,228 @@ __device__ void grid_barrier(TTG_BLOCK, unsigned* bar, int* err,
   __syncthreads();
 }
 
-// Grid-wide deterministic sum; every thread of every block gets the result.
-// Partial buffers alternate so one barrier per reduction suffices.
-__device__ double grid_sum(TTG_BLOCK, double v, const HhArgs& a, unsigned& parity) {
-  v = block_sum_all(v);
-  double* part = a.part + (parity & 1u) * gridDim.x;
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
-  grid_barrier(blockIdx, gridDim, a.bar, a.err);
-  double s = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) s += __ldcg(part + i);
-  s = block_sum_all(s);
-  parity ^= 1u;
-  return s;
+// First row and end of this block's share of the rows.
+__device__ __forceinline__ int64_t row_at(int64_t sz, int64_t b, int64_t nb) { return sz * b / nb; }
+
+// part[r * nb + b] = sum over this block's rows [i0, i1) of U_r[i] w[i],
+// r < nr.  Four columns per warp share the loads of w; with fewer column
+// groups than warps the rows of a group are split over several warps.
+__device__ void hh_dots(const double* U, int64_t sz, int64_t nr, const double* w, int64_t i0,
+                        int64_t i1, double* sp, double* part, int64_t b, int64_t nb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t G = (nr + 3) / 4, RP = G >= HH_WARPS ? 1 : HH_WARPS / G;
+  for (int64_t unit = warp; unit < G * RP; unit += HH_WARPS) {
+    const int64_t g = unit / RP, p = unit % RP;
+    const double* u0 = U + 4 * g * sz;
+    const double* u1 = U + min(4 * g + 1, nr - 1) * sz;
+    const double* u2 = U + min(4 * g + 2, nr - 1) * sz;
+    const double* u3 = U + min(4 * g + 3, nr - 1) * sz;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    const int64_t lo = i0 + (i1 - i0) * p / RP, hi = i0 + (i1 - i0) * (p + 1) / RP;
+#pragma unroll 4
+    for (int64_t i = lo + lane; i < hi; i += 32) {
+      const double x = w[i];
+      s0 = fma(u0[i], x, s0);
+      s1 = fma(u1[i], x, s1);
+      s2 = fma(u2[i], x, s2);
+      s3 = fma(u3[i], x, s3);
+    }
+    s0 = warp_sum(s0);
+    s1 = warp_sum(s1);
+    s2 = warp_sum(s2);
+    s3 = warp_sum(s3);
+    if (lane < 4 && 4 * g + lane < nr)
+      sp[(4 * g + lane) * RP + p] = lane == 0 ? s0 : lane == 1 ? s1 : lane == 2 ? s2 : s3;
+  }
+  __syncthreads();
+  for (int64_t r = threadIdx.x; r < nr; r += blockDim.x) {
+    double s = 0.0;
+    for (int64_t p = 0; p < RP; ++p) s += sp[r * RP + p];
+    part[r * nb + b] = s;
+  }
 }
 
-#define GRID_LOOP(idx, n)                                                           \
-  for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < (n);    \
-       idx += int64_t(gridDim.x) * blockDim.x)
+// out[r] = sum over the blocks of part[r * nb + b] in a fixed order, r < nr.
+__device__ void hh_gather(const double* part, int64_t nb, int64_t nr, double* out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t r = warp; r < nr; r += HH_WARPS) {
+    double s = 0.0;
+    for (int64_t b = lane; b < nb; b += 32) s += __ldcg(part + r * nb + b);
+    s = warp_sum(s);
+    if (lane == 0) out[r] = s;
+  }
+  __syncthreads();
+}
 
-// w = rhs - w2 ; U_0 = Householder vector of w ; tau_0 = -beta  (:376-392)
+// v - sum_r U_r[i] y[r], r < nr
+__device__ __forceinline__ double hh_row(const double* U, int64_t sz, int64_t nr, int64_t i,
+                                         const double* y, double v) {
+  const double* u = U + i;
+#pragma unroll 8
+  for (int64_t r = 0; r < nr; ++r) v = fma(-u[r * sz], y[r], v);
+  return v;
+}
+
+// w = rhs - w2 ; U_0 = Householder vector of w ; tau_0 = -beta  (:376-392);
+// then v_0 = P_0 e_0 into w.
 TTG_BODY(k_hh_init)(TTG_BLOCK, HhArgs a, int it) {
-  unsigned parity = 0;
-  const int64_t sz = a.sz;
+  const int64_t sz = a.sz, nb = gridDim.x, b = blockIdx.x;
+  const int64_t i0 = row_at(sz, b, nb), i1 = row_at(sz, b + 1, nb);
+  __shared__ double tot;
   double s = 0.0;
-  GRID_LOOP(i, sz) {
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     const double v = a.rhs[i] - a.w2[i];
     a.w[i] = v;
-    s += v * v;
+    s = fma(v, v, s);
+    if (i == 0) a.scal[4] = v;  // read by every block after the barrier
   }
-  const double nrmr = sqrt(grid_sum(blockIdx, gridDim, s, a, parity));
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  s = block_sum_all(s);
+  if (threadIdx.x == 0) a.part[b] = s;
+  grid_barrier(blockIdx, gridDim, a.bar, a.err);
+  hh_gather(a.part, nb, 1, &tot);
+  const double nrmr = sqrt(tot);
+  if (b == 0 && threadIdx.x == 0) {
     if (it == 0) a.scal[0] = nrmr;
     a.scal[2] = nrmr;
     a.scal[3] = (nrmr == 0.0) ? 1.0 : 0.0;
   }
   if (nrmr == 0.0) return;
-  const double w0 = __ldcg(a.w);
+  const double w0 = __ldcg(a.scal + 4);
   const double beta = (w0 < 0.0) ? -nrmr : nrmr;
   const double nu = sqrt(2.0 * nrmr * nrmr + 2.0 * beta * w0);
-  GRID_LOOP(i, sz) {
-    const double v = (i == 0) ? (a.w[i] + beta) : a.w[i];
-    a.U[i] = v / nu;
+  const double u0 = (w0 + beta) / nu;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    const double u = i == 0 ? u0 : a.w[i] / nu;
+    a.U[i] = u;
+    a.w[i] = fma(-2.0 * u0, u, i == 0 ? 1.0 : 0.0);
   }
-  if (blockIdx.x == 0) {
+  if (b == 0) {
     for (int64_t k = threadIdx.x; k <= a.nrestart; k += blockDim.x) a.tau[k] = 0.0;
     __syncthreads();
-    if (threadIdx.x == 0) a.tau[0] = -beta;
+    if (threadIdx.x == 0) {
+      a.tau[0] = -beta;
+      a.T[0] = a.TT[0] = 2.0;
+    }
   }
 }
 TTG_COOP_KERNEL(k_hh_init, HH_THREADS);
 
-// v_j = P_0 ... P_{j-1} (P_j e_j), normalised, into w  (:396-406)
-TTG_BODY(k_hh_build)(TTG_BLOCK, HhArgs a, int64_t j) {
+// One Arnoldi step around the matvec w2 = B v_j:
+//   w2 = P_j ... P_0 w2 = w2 - U T' (U' w2)                     (:421-427)
+//   next reflector u_{j+1} from w2 below row j                  (:428-443)
+//   Givens rotations, R(:,j), residual estimate                 (:445-473)
+//   v_{j+1} = P_0 ... P_{j+1} e_{j+1}, into w                   (:396-406)
+// Row j + 1 of U gives U' e_{j+1}, so v_{j+1} takes no further inner products
+// but those of the new column of T, U' u_{j+1}: they are formed from the
+// rows of w2 below j together with their norm, before u_{j+1} is known
+// (u_{j+1} = (w2 + alpha e_{j+1}) / nu there).  v_{j+1} has unit norm by
+// construction.  Bound by the four reads of U a step (41 columns of 64 x 64 x
+// 64 are 86 MB, mostly L2 hits): a local solve of two restarts of 40 at that
+// size takes 7.0 ms, 40 us of it this kernel per step, against 22.3 ms with
+// one grid barrier per reflector (225 us per step).
+TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
   if (*(volatile int*)a.stop) return;  // queued after convergence
-  unsigned parity = 0;
-  const int64_t sz = a.sz;
-  const double* Uj = a.U + j * sz;
-  const double ujj = __ldcg(Uj + j);
-  GRID_LOOP(i, sz) { a.w[i] = -2.0 * ujj * Uj[i] + (i == j ? 1.0 : 0.0); }
-  for (int64_t r = j - 1; r >= 0; --r) {
-    const double* Ur = a.U + r * sz;
-    double s = 0.0;
-    GRID_LOOP(i, sz) s += Ur[i] * a.w[i];
-    const double dot = grid_sum(blockIdx, gridDim, s, a, parity);
-    GRID_LOOP(i, sz) a.w[i] -= 2.0 * dot * Ur[i];
-  }
-  double s = 0.0;
-  GRID_LOOP(i, sz) s += a.w[i] * a.w[i];
-  const double inv = 1.0 / sqrt(grid_sum(blockIdx, gridDim, s, a, parity));
-  GRID_LOOP(i, sz) a.w[i] *= inv;
-}
-TTG_COOP_KERNEL(k_hh_build, HH_THREADS);
-
-// w2 = P_j ... P_0 w2 ; new reflector U_{j+1} ; Givens ; R(:,j) ; residual (:421-473)
-TTG_BODY(k_hh_tail)(TTG_BLOCK, HhArgs a, int64_t j) {
-  if (*(volatile int*)a.stop) return;  // queued after convergence
-  unsigned parity = 0;
-  const int64_t sz = a.sz;
+  extern __shared__ double hsm[];
+  const int64_t sz = a.sz, m1 = a.nrestart + 1, nr = j + 1;
+  const int64_t nb = gridDim.x, b = blockIdx.x;
+  const int64_t i0 = row_at(sz, b, nb), i1 = row_at(sz, b + 1, nb);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* sd = hsm;       // inner products
+  double* sy = sd + m1;   // coefficients of the columns of U
+  double* su = sy + m1;   // row j + 1 of U
+  double* sp = su + m1;   // per-warp partials
+  double* part2 = a.part + (m1 + 1) * nb;
   double* w = a.w2;
-  for (int64_t r = 0; r <= j; ++r) {
-    const double* Ur = a.U + r * sz;
-    double s = 0.0;
-    GRID_LOOP(i, sz) s += Ur[i] * w[i];
-    const double dot = grid_sum(blockIdx, gridDim, s, a, parity);
-    GRID_LOOP(i, sz) w[i] -= 2.0 * dot * Ur[i];
-  }
-  if (j < sz - 1) {
-    // The owner of w[j+1] publishes it before the barrier: after the barrier
-    // it rewrites w[j+1], so other blocks must not read w itself.
-    double s = 0.0;
-    GRID_LOOP(i, sz) {
-      if (i > j) s += w[i] * w[i];
-      if (i == j + 1) a.scal[4] = w[i];
-    }
-    double alpha = sqrt(grid_sum(blockIdx, gridDim, s, a, parity));
-    const double wj1 = __ldcg(a.scal + 4);
-    double* Un = a.U + (j + 1) * sz;
-    if (alpha != 0.0) {
-      if (wj1 < 0.0) alpha = -alpha;
-      const double nu = sqrt(2.0 * alpha * alpha + 2.0 * alpha * wj1);
-      GRID_LOOP(i, sz) {
-        double u;
-        if (i <= j)
-          u = 0.0;
-        else if (i == j + 1)
-          u = (w[i] + alpha) / nu;
-        else
-          u = w[i] / nu;
-        Un[i] = u;
-        if (i == j + 1)
-          w[i] = -alpha;
-        else if (i > j + 1)
-          w[i] = 0.0;
-      }
-    } else {
-      GRID_LOOP(i, sz) Un[i] = (i <= j) ? 0.0 : w[i];
-    }
-  }
+
+  hh_dots(a.U, sz, nr, w, i0, i1, sp, a.part, b, nb);
   grid_barrier(blockIdx, gridDim, a.bar, a.err);
-  if (blockIdx.x == 0) {
-    // Givens rotations to the top of w (:445-449) on one thread.  With
-    // staging (restart length up to HH_STAGE_MAX) the chain of dependent
-    // accesses runs on shared-memory copies of w's top entries and of the
-    // rotators, copied in and out by the block; the same operations in the
-    // same order as on the global arrays.
-    extern __shared__ double tsm[];
-    const bool staged = a.nrestart <= HH_STAGE_MAX;
-    const int64_t top = a.nrestart + 1 < sz ? a.nrestart + 1 : sz;
-    double* wl = staged ? tsm : w;
-    double* Jl = staged ? tsm + (a.nrestart + 1) : a.J;
-    if (staged) {
-      for (int64_t e = threadIdx.x; e < top; e += blockDim.x) wl[e] = __ldcg(w + e);
-      for (int64_t e = threadIdx.x; e < 2 * j; e += blockDim.x) Jl[e] = a.J[e];
-      __syncthreads();
+  hh_gather(a.part, nb, nr, sd);
+  for (int64_t r = warp; r < nr; r += HH_WARPS) {  // T' (U' w2)
+    double s = 0.0;
+    for (int64_t q = lane; q <= r; q += 32) s = fma(a.T[q + r * m1], sd[q], s);
+    s = warp_sum(s);
+    if (lane == 0) sy[r] = s;
+  }
+  __syncthreads();
+  const bool next = j < sz - 1;          // a new reflector exists
+  const bool build = j + 1 < a.nrestart;  // and another step follows
+  double s = 0.0;
+  for (int64_t i = i0 + tid; i < i1; i += blockDim.x) {
+    const double v = hh_row(a.U, sz, nr, i, sy, w[i]);
+    w[i] = v;
+    if (i > j) s = fma(v, v, s);
+    if (i == j + 1) a.scal[4] = v;
+  }
+  s = block_sum_all(s);  // and every thread's rows of w are written
+  if (next && build)
+    hh_dots(a.U, sz, nr, w, max(i0, min(nr, i1)), i1, sp, part2, b, nb);
+  if (tid == 0) part2[nr * nb + b] = s;
+  grid_barrier(blockIdx, gridDim, a.bar, a.err);
+
+  double alpha = 0.0;
+  if (next) {
+    if (build) {
+      hh_gather(part2, nb, nr + 1, sd);
+      alpha = sqrt(sd[nr]);
+    } else {
+      hh_gather(part2 + nr * nb, nb, 1, sd);
+      alpha = sqrt(sd[0]);
     }
-    if (threadIdx.x == 0) {
-      for (int64_t i = 0; i < j; ++i) {
-        const double b = staged ? wl[i] : __ldcg(w + i);
-        const double b1 = staged ? wl[i + 1] : __ldcg(w + i + 1);
-        const double c0 = Jl[2 * i], c1 = Jl[2 * i + 1];
-        wl[i] = c0 * b + c1 * b1;
-        wl[i + 1] = -c1 * b + c0 * b1;
+    const double wj1 = __ldcg(a.scal + 4);
+    if (wj1 < 0.0) alpha = -alpha;
+    if (build) {
+      const double nu = alpha != 0.0 ? sqrt(2.0 * alpha * alpha + 2.0 * alpha * wj1) : 1.0;
+      const double uj1 = (wj1 + alpha) / nu;
+      for (int64_t r = tid; r < nr; r += blockDim.x) {
+        const double ur = __ldcg(a.U + (j + 1) + r * sz);
+        su[r] = ur;
+        sd[r] = fma(alpha, ur, sd[r]) / nu;  // U' u_{j+1}
       }
-      if (j < sz - 1) {  // new rotator (:454-465)
-        const double wj = staged ? wl[j] : __ldcg(w + j);
-        const double wj1 = staged ? wl[j + 1] : __ldcg(w + j + 1);
+      __syncthreads();
+      for (int64_t q = warp; q < nr; q += HH_WARPS) {
+        double t = 0.0, y = 0.0;
+        for (int64_t r = q + lane; r < nr; r += 32) {
+          const double Tqr = a.TT[r + q * m1];
+          t = fma(Tqr, sd[r], t);
+          y = fma(Tqr, su[r], y);
+        }
+        t = -2.0 * warp_sum(t);
+        y = warp_sum(y);
+        if (lane == 0) {
+          sy[q] = fma(t, uj1, y);
+          if (b == 0) a.T[q + nr * m1] = a.TT[nr + q * m1] = t;
+        }
+      }
+      if (b == 0 && tid == 0) a.T[nr + nr * m1] = a.TT[nr + nr * m1] = 2.0;
+      __syncthreads();
+      double* Un = a.U + nr * sz;
+      const double yn = 2.0 * uj1;
+      for (int64_t i = i0 + tid; i < i1; i += blockDim.x) {
+        const double u = i <= j ? 0.0 : (i == j + 1 ? uj1 : w[i] / nu);
+        Un[i] = u;
+        a.w[i] = hh_row(a.U, sz, nr, i, sy, fma(-u, yn, i == j + 1 ? 1.0 : 0.0));
+      }
+    }
+  }
+  if (b == 0) {
+    // Givens rotations of the new Hessenberg column (:445-449) by one thread
+    // on shared-memory copies of the column and of the rotators.
+    __syncthreads();
+    double* wl = hsm;                 // nrestart + 1
+    double* Jl = hsm + a.nrestart + 1;  // 2 nrestart
+    for (int64_t e = tid; e <= j; e += blockDim.x) wl[e] = __ldcg(w + e);
+    for (int64_t e = tid; e < 2 * j; e += blockDim.x) Jl[e] = a.J[e];
+    __syncthreads();
+    if (tid == 0) {
+      if (next) wl[j + 1] = -alpha;
+      for (int64_t i = 0; i < j; ++i) {
+        const double x = wl[i], x1 = wl[i + 1];
+        const double c0 = Jl[2 * i], c1 = Jl[2 * i + 1];
+        wl[i] = c0 * x + c1 * x1;
+        wl[i + 1] = -c1 * x + c0 * x1;
+      }
+      if (next) {  // new rotator (:454-465)
+        const double wj = wl[j], wj1 = wl[j + 1];
         const double rho = sqrt(wj * wj + wj1 * wj1);
         const double c0 = wj / rho, c1 = wj1 / rho;
         a.J[2 * j] = c0;
@@ -261,11 +345,7 @@ TTG_BODY(k_hh_tail)(TTG_BLOCK, HhArgs a, int64_t j) {
         a.tau[j + 1] = -c1 * a.tau[j];
         a.tau[j] = c0 * a.tau[j];
         wl[j] = rho;
-        wl[j + 1] = 0.0;
       }
-      if (!staged)
-        for (int64_t k = 0; k < a.nrestart; ++k)
-          a.R[k + j * a.nrestart] = (k < sz) ? __ldcg(w + k) : 0.0;
       const double curres = fabs(a.tau[j + 1]) / a.scal[0];
       a.scal[1] = curres;
       if (curres < a.tol) {  // (:476) later queued steps see the flag and return
@@ -274,71 +354,72 @@ TTG_BODY(k_hh_tail)(TTG_BLOCK, HhArgs a, int64_t j) {
         a.stop[0] = 1;
       }
     }
-    if (staged) {
-      __syncthreads();
-      for (int64_t k = threadIdx.x; k < a.nrestart; k += blockDim.x)
-        a.R[k + j * a.nrestart] = (k < sz) ? wl[k] : 0.0;
-      for (int64_t e = threadIdx.x; e < top; e += blockDim.x) w[e] = wl[e];
-    }
+    __syncthreads();
+    for (int64_t k = tid; k < a.nrestart; k += blockDim.x)
+      a.R[k + j * a.nrestart] = k <= j ? wl[k] : 0.0;
   }
 }
-TTG_COOP_KERNEL(k_hh_tail, HH_THREADS);
+TTG_COOP_KERNEL(k_hh_step, HH_THREADS);
 
-// Triangular solve + correction sol += P_0..P_j (sum y_i e_i)  (:487-507)
-TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t j, int64_t ni) {
-  // y (nrestart); with staging also R's leading ni x ni block (ld ni) and
-  // tau, copied by the block so that the back-substitution on one thread
-  // reads shared memory (same operations, same order).
-  extern __shared__ double y[];
-  unsigned parity = 0;
-  const int64_t sz = a.sz;
+// y = R^{-1} tau, then sol += P_0 ... P_j (sum_i y_i e_i)
+//                        = sol + y - U T (U' y)                 (:487-507)
+// Every block solves the small system for itself; no barrier.
+TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t ni) {
+  pdl_begin();
+  extern __shared__ double y[];  // y (ni), U' y (ni), T U' y (ni), R when staged (ld ni)
+  const int64_t sz = a.sz, m1 = a.nrestart + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool staged = a.nrestart <= HH_CORRECT_STAGE_MAX;
-  double* Rs = y + a.nrestart;
-  double* ts = Rs + ni * ni;
-  if (staged) {
-    for (int64_t e = threadIdx.x; e < ni * ni; e += blockDim.x)
+  double* sc = y + ni;
+  double* st = sc + ni;
+  double* Rs = st + ni;
+  if (staged)
+    for (int64_t e = tid; e < ni * ni; e += blockDim.x)
       Rs[e] = a.R[(e % ni) + (e / ni) * a.nrestart];
-    for (int64_t e = threadIdx.x; e < ni; e += blockDim.x) ts[e] = a.tau[e];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    for (int64_t row = ni - 1; row >= 0; --row) {
-      double v = staged ? ts[row] : a.tau[row];
-      for (int64_t col = row + 1; col < ni; ++col)
-        v -= (staged ? Rs[row + col * ni] : a.R[row + col * a.nrestart]) * y[col];
-      y[row] = v / (staged ? Rs[row + row * ni] : a.R[row + row * a.nrestart]);
+  for (int64_t e = tid; e < ni; e += blockDim.x) y[e] = a.tau[e];
+  __syncthreads();
+  if (warp == 0) {  // back-substitution, one column at a time
+    const double* R = staged ? Rs : a.R;
+    const int64_t ldr = staged ? ni : a.nrestart;
+    for (int64_t c = ni - 1; c >= 0; --c) {
+      const double v = y[c] / R[c + c * ldr];
+      __syncwarp();
+      if (lane == 0) y[c] = v;
+      for (int64_t r = lane; r < c; r += 32) y[r] = fma(-R[r + c * ldr], v, y[r]);
+      __syncwarp();
     }
   }
   __syncthreads();
-  const double* Uj = a.U + j * sz;
-  const double ujj = __ldcg(Uj + j);
-  const double yj = y[j];
-  GRID_LOOP(i, sz) a.w[i] = -2.0 * ujj * yj * Uj[i] + (i == j ? yj : 0.0);
-  for (int64_t r = j - 1; r >= 0; --r) {
-    const double* Ur = a.U + r * sz;
+  for (int64_t r = warp; r < ni; r += HH_WARPS) {  // u_r has no entries above row r
     double s = 0.0;
-    GRID_LOOP(i, sz) {
-      if (i == r) a.w[i] += y[r];
-      s += Ur[i] * a.w[i];
-    }
-    const double dot = grid_sum(blockIdx, gridDim, s, a, parity);
-    GRID_LOOP(i, sz) a.w[i] -= 2.0 * dot * Ur[i];
+    for (int64_t i = r + lane; i < ni; i += 32) s = fma(a.U[i + r * sz], y[i], s);
+    s = warp_sum(s);
+    if (lane == 0) sc[r] = s;
   }
-  GRID_LOOP(i, sz) a.sol[i] += a.w[i];
+  __syncthreads();
+  for (int64_t q = warp; q < ni; q += HH_WARPS) {
+    double s = 0.0;
+    for (int64_t r = q + lane; r < ni; r += 32) s = fma(a.TT[r + q * m1], sc[r], s);
+    s = warp_sum(s);
+    if (lane == 0) st[q] = s;
+  }
+  __syncthreads();
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + tid; i < sz;
+       i += int64_t(gridDim.x) * blockDim.x)
+    a.sol[i] += hh_row(a.U, sz, ni, i, st, i < ni ? y[i] : 0.0);
 }
-TTG_COOP_KERNEL(k_hh_correct, HH_THREADS);
+TTG_KERNEL(k_hh_correct, HH_THREADS);
 
+// Blocks of the cooperative kernels: contiguous row ranges of at least HH_ROWS
+// rows, at most two blocks per SM.  Two keep twice the loads of U in flight
+// (64 x 64 x 64, 80 steps: 7.04 against 7.66 ms with one); small systems take
+// few blocks, and 256 or 512 rows as the least share measure the same.
+constexpr int64_t HH_ROWS = 256;
 int coop_blocks(Context* c, const void* kernel, size_t smem, int64_t sz) {
-  int occ = 0;
-  occ = max_active_blocks(kernel, HH_THREADS, smem);
-  if (occ < 1) occ = 1;
-  int64_t want = (sz + HH_THREADS * 4 - 1) / (HH_THREADS * 4);
-  int64_t cap = int64_t(c->num_sms) * std::min(occ, 2);
-  if (want > cap) want = cap;
-  if (want < 1) want = 1;
-  return int(want);
+  const int64_t cap =
+      int64_t(c->num_sms) * std::max(1, std::min(max_active_blocks(kernel, HH_THREADS, smem), 2));
+  return int(std::max<int64_t>(1, std::min((sz + HH_ROWS - 1) / HH_ROWS, cap)));
 }
-
 
 }  // namespace
 
@@ -348,12 +429,14 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
   TTG_REQUIRE(nrestart >= 1 && nrestart <= 4096, "nrestart %lld out of range",
               (long long)nrestart);
   DBuf<double> U(c, size_t(sz) * (nrestart + 1)), w(c, sz), w2(c, sz);
-  DBuf<double> small(c, (nrestart + 1) + 2 * nrestart + nrestart * nrestart + 8);
-  const int blocks = std::min(
-      std::min(coop_blocks(c, k_hh_init.fn(), 0, sz), coop_blocks(c, k_hh_build.fn(), 0, sz)),
-      std::min(coop_blocks(c, k_hh_tail.fn(), hh_tail_smem(nrestart), sz),
-               coop_blocks(c, k_hh_correct.fn(), hh_correct_smem(nrestart), sz)));
-  DBuf<double> part(c, 2 * blocks);
+  const int64_t m1 = nrestart + 1;
+  DBuf<double> small(c, m1 + 2 * nrestart + nrestart * nrestart + 2 * m1 * m1 + 8);
+  const size_t step_smem = hh_step_smem(nrestart);
+  ensure_smem_attr(k_hh_step.fn(), c->device, int(hh_step_smem(4096)));
+  ensure_smem_attr(k_hh_correct.fn(), c->device, int(hh_correct_smem(4096, 4096)));
+  const int blocks = std::min(coop_blocks(c, k_hh_init.fn(), 0, sz),
+                              coop_blocks(c, k_hh_step.fn(), step_smem, sz));
+  DBuf<double> part(c, 2 * (m1 + 1) * blocks);
   DBuf<unsigned> bar(c, 4);
   DBuf<int> stop(c, 4);
   memset_async(c, bar.p(), 0, 4 * sizeof(unsigned));
@@ -370,7 +453,9 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
   a.tau = small.p();
   a.J = a.tau + (nrestart + 1);
   a.R = a.J + 2 * nrestart;
-  a.scal = a.R + nrestart * nrestart;
+  a.T = a.R + nrestart * nrestart;
+  a.TT = a.T + m1 * m1;
+  a.scal = a.TT + m1 * m1;
   a.part = part.p();
   a.bar = bar.p();
   a.err = c->d_err;
@@ -379,8 +464,8 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
   fill_f64(c, sz, 0.0, sol);
 
   // Arnoldi steps are queued in chunks of growing length without a host
-  // round trip per step; k_hh_tail raises a device flag on convergence and
-  // every kernel queued after it (reflector kernels and the matvec GEMMs,
+  // round trip per step; k_hh_step raises a device flag on convergence and
+  // every kernel queued after it (further steps and the matvec GEMMs,
   // through Context::skip) returns at once.  The host reads the flag, the
   // converged step and the residual estimate once per chunk.
   struct Probe {
@@ -422,9 +507,8 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
     while (j < nrestart) {
       const int64_t jend = std::min(nrestart, j + chunk);
       for (int64_t jj = j; jj < jend; ++jj) {
-        launch(c, k_hh_build, blocks, HH_THREADS, 0, a, jj);
         apply(w.p(), w2.p());
-        launch(c, k_hh_tail, blocks, HH_THREADS, hh_tail_smem(nrestart), a, jj);
+        launch(c, k_hh_step, blocks, HH_THREADS, step_smem, a, jj);
       }
       Probe p;
       probe(p);
@@ -448,7 +532,7 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
     } else {
       ni = j + 1;
     }
-    launch(c, k_hh_correct, blocks, HH_THREADS, hh_correct_smem(nrestart), a, j, ni);
+    launch(c, k_hh_correct, blocks, HH_THREADS, hh_correct_smem(nrestart, ni), a, ni);
     if (curres < tol) break;
   }
   res.relres = curres;
