@@ -26,24 +26,28 @@ namespace ttg {
 
 namespace {
 
-constexpr int AR_THREADS = 256;
+constexpr int AR_THREADS = 512;
 constexpr int AR_WARPS = AR_THREADS / 32;
 constexpr long long AR_SPIN_LIMIT = 1LL << 24;
 constexpr int MAX_OUTER = 8;
 constexpr double INNER_TOL = 1e-3;
+// Least rows of a block of the cooperative Arnoldi kernels: 512 measures the
+// same, 2048 4% slower on solves of 97 x 64 x 83 and on batches of small ones.
+constexpr int64_t AR_ROWS = 1024;
 
 struct ArArgs {
   int64_t sz;
+  int64_t ldv;     // sz rounded up to a multiple of 4 (float4 loads)
   int m;           // restart length
-  float* V;        // sz x (m+1)
-  float* w;        // matvec output, orthogonalised in place
+  float* V;        // ldv x (m+1), zero in rows sz..ldv
+  float* w;        // matvec output (ldv, zero in rows sz..ldv), orthogonalised in place
   double* H;       // (m+1) x m, column-major
   double* cs;      // m
   double* sn;      // m
   double* g;       // m+1
   double* scal;    // [0] |g_{j+1}|  [1] norm of the new Arnoldi vector  [2] beta
                    // [3] norm of the solve's right-hand side  [4] stop threshold
-  double* part;    // 2 * (m+1) * gridDim.x
+  double* part;    // 2 * (m+2) * gridDim.x
   unsigned* bar;   // [0] count [1] generation
   int* err;
   int* stop;       // [0] converged flag, [1] step at which it converged (-1: at start)
@@ -56,17 +60,29 @@ struct ArArgs {
   int ldx;
 };
 
-__device__ __forceinline__ void put_x(const ArArgs& a, int64_t i, float v) {
+// Four consecutive entries i..i+3 of a new basis vector (those below sz).
+__device__ __forceinline__ void put_x4(const ArArgs& a, int64_t i, const float4& v) {
   if (!a.X) return;  // preconditioned solve: the operand is P v, written apart
-  const int64_t row = i / a.rx2, b = i - row * a.rx2;
-  a.X[b + int64_t(a.ldx) * row] = __float2bfloat16_rn(v);
+  int64_t row;
+  int b;
+  if (a.sz <= 0xffffffffll) {  // 32-bit division where it holds the index
+    row = unsigned(i) / unsigned(a.rx2);
+    b = int(unsigned(i) - unsigned(row) * unsigned(a.rx2));
+  } else {
+    row = i / a.rx2;
+    b = int(i - row * a.rx2);
+  }
+  const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (i + k < a.sz) a.X[b + int64_t(a.ldx) * row] = __float2bfloat16_rn(e[k]);
+    if (++b == a.rx2) {
+      b = 0;
+      ++row;
+    }
+  }
 }
 
-__device__ __forceinline__ float warp_sumf(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 __device__ __forceinline__ double warp_sumd(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -105,38 +121,54 @@ __device__ void ar_barrier(TTG_BLOCK, unsigned* bar, int* err, long long limit =
   for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < (n);    \
        idx += int64_t(gridDim.x) * blockDim.x)
 
-// part[c*nb + block] = block partial of V(:,c)'w, c < ncol.  red: AR_WARPS*(m+1) floats.
-// Columns go in groups of AR_COLS per pass over w, so that each thread has
-// AR_COLS independent loads in flight instead of one memory latency per
-// column; every column's sum is formed in the same order as one column per
-// pass would form it.
-constexpr int AR_COLS = 8;
-__device__ void partial_dots(TTG_BLOCK, const ArArgs& a, int ncol, double* part, float* red) {
+// This block's share of the rows, in groups of four.
+__device__ __forceinline__ int64_t quad_at(const ArArgs& a, int64_t b, int64_t nb) {
+  return (a.ldv / 4) * b / nb;
+}
+
+__device__ __forceinline__ float dot4(const float4& u, const float4& x) {
+  return fmaf(u.w, x.w, fmaf(u.z, x.z, fmaf(u.y, x.y, u.x * x.x)));
+}
+
+// part[c*nb + block] = block partial of V(:,c)'w, c < ncol.  Four columns per
+// warp share the loads of w; with fewer column groups than warps the rows of
+// a group are split over several warps.  Products of four rows are summed in
+// FP32, everything beyond in FP64.  sp: m + 1 + 4 AR_WARPS doubles.
+__device__ void partial_dots(const ArArgs& a, int ncol, int64_t q0, int64_t q1, int64_t b,
+                             int64_t nb, double* part, double* sp) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int c0 = 0; c0 < ncol; c0 += AR_COLS) {
-    const int nc = ncol - c0 < AR_COLS ? ncol - c0 : AR_COLS;
-    float s[AR_COLS];
-#pragma unroll
-    for (int k = 0; k < AR_COLS; ++k) s[k] = 0.f;
-    AR_LOOP(i, a.sz) {
-      const float wi = a.w[i];
-#pragma unroll
-      for (int k = 0; k < AR_COLS; ++k)
-        if (k < nc) s[k] += a.V[int64_t(c0 + k) * a.sz + i] * wi;
+  const int G = (ncol + 3) / 4, RP = G >= AR_WARPS ? 1 : AR_WARPS / G;
+  const int64_t ldq = a.ldv / 4;
+  const float4* V = reinterpret_cast<const float4*>(a.V);
+  const float4* w = reinterpret_cast<const float4*>(a.w);
+  for (int unit = warp; unit < G * RP; unit += AR_WARPS) {
+    const int g = unit / RP, p = unit % RP;
+    const float4* v0 = V + 4 * g * ldq;
+    const float4* v1 = V + min(4 * g + 1, ncol - 1) * ldq;
+    const float4* v2 = V + min(4 * g + 2, ncol - 1) * ldq;
+    const float4* v3 = V + min(4 * g + 3, ncol - 1) * ldq;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    const int64_t lo = q0 + (q1 - q0) * p / RP, hi = q0 + (q1 - q0) * (p + 1) / RP;
+#pragma unroll 2
+    for (int64_t q = lo + lane; q < hi; q += 32) {
+      const float4 x = w[q];
+      s0 += double(dot4(v0[q], x));
+      s1 += double(dot4(v1[q], x));
+      s2 += double(dot4(v2[q], x));
+      s3 += double(dot4(v3[q], x));
     }
-#pragma unroll
-    for (int k = 0; k < AR_COLS; ++k) {
-      if (k < nc) {
-        const float t = warp_sumf(s[k]);
-        if (lane == 0) red[warp * (a.m + 1) + c0 + k] = t;
-      }
-    }
+    s0 = warp_sumd(s0);
+    s1 = warp_sumd(s1);
+    s2 = warp_sumd(s2);
+    s3 = warp_sumd(s3);
+    if (lane < 4 && 4 * g + lane < ncol)
+      sp[(4 * g + lane) * RP + p] = lane == 0 ? s0 : lane == 1 ? s1 : lane == 2 ? s2 : s3;
   }
   __syncthreads();
   for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
     double s = 0.0;
-    for (int q = 0; q < AR_WARPS; ++q) s += double(red[q * (a.m + 1) + c]);
-    part[int64_t(c) * gridDim.x + blockIdx.x] = s;
+    for (int p = 0; p < RP; ++p) s += sp[c * RP + p];
+    part[c * nb + b] = s;
   }
 }
 
@@ -152,104 +184,165 @@ __device__ void reduce_parts(TTG_BLOCK, const double* part, int ncol, double* ou
   __syncthreads();
 }
 
-// Shared memory of k_arnoldi: hp (m+1 doubles), ht (m+2), red (AR_WARPS
-// (m+1) floats), then 2 m doubles for the rotations of the Givens update,
-// 8-byte aligned.
-__device__ __forceinline__ double* red_d(double* shd, int m) {
-  const size_t off = sizeof(double) * 2 * (m + 2) + sizeof(float) * AR_WARPS * (m + 1);
-  return reinterpret_cast<double*>(reinterpret_cast<char*>(shd) + ((off + 7) & ~size_t(7)));
+// Block-wide sum in thread 0; red: AR_WARPS doubles.
+__device__ __forceinline__ double block_sum0(double v, double* red) {
+  v = warp_sumd(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x == 0)
+    for (int q = 0; q < AR_WARPS; ++q) t += red[q];
+  return t;
+}
+
+// w - sum_c V(q, c) h[c] for the four rows of group q
+__device__ __forceinline__ float4 project4(const float4* V, int64_t ldq, int ncol, int64_t q,
+                                           const float* h, float4 w) {
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int c = 0; c < ncol; ++c) {
+    const float4 v = V[c * ldq + q];
+    const float hc = h[c];
+    s.x = fmaf(v.x, hc, s.x);
+    s.y = fmaf(v.y, hc, s.y);
+    s.z = fmaf(v.z, hc, s.z);
+    s.w = fmaf(v.w, hc, s.w);
+  }
+  w.x -= s.x;
+  w.y -= s.y;
+  w.z -= s.z;
+  w.w -= s.w;
+  return w;
+}
+
+// Shared memory of k_arnoldi, in doubles: hp (m+2), ht (m+2), partials
+// (m+1 + 4 AR_WARPS), the rotations of the Givens update (2 m), and hf (m+1
+// floats).
+__host__ __device__ __forceinline__ size_t arnoldi_doubles(int m) {
+  return size_t(2 * (m + 2) + (m + 1 + 4 * AR_WARPS) + 2 * m);
 }
 
 // One Arnoldi step for column j: w -= V h twice (CGS2), normalise into
 // V(:, j+1), Givens update of H(:, j) and g; scal[0] = |g_{j+1}|.
+// Two grid barriers, one per projection: with w1 the vector after the first
+// and h2 its coefficients, the norm after the second is |w1|^2 - |h2|^2; only
+// when the second projection removes more than a quarter of it (w lies in the
+// span of the basis to rounding) is the norm summed over the result, at a
+// third barrier.  Bound by reading V four times from L2 at large sizes (97 x
+// 64 x 83, mean over 40 columns: 24 us per step, against 50 us with three
+// barriers, scalar loads and the norm in a pass of its own) and by the two
+// barriers at small ones (13 against 22 us in a batch of twelve systems).
 TTG_BODY(k_arnoldi)(TTG_BLOCK, ArArgs a, int j) {
   if (*(volatile int*)a.stop) return;  // queued after convergence
   extern __shared__ double shd[];
-  double* hp = shd;                 // m+1 : this pass's coefficients
-  double* ht = shd + (a.m + 1);     // m+2 : accumulated coefficients
-  float* red = reinterpret_cast<float*>(shd + 2 * (a.m + 2));
-  const int ncol = j + 1;
+  const int m = a.m, ncol = j + 1;
+  const int64_t b = blockIdx.x, nb = gridDim.x;
+  const int64_t q0 = quad_at(a, b, nb), q1 = quad_at(a, b + 1, nb), ldq = a.ldv / 4;
+  const int tid = threadIdx.x;
+  double* hp = shd;              // this pass's coefficients, then |w1|^2
+  double* ht = hp + (m + 2);     // accumulated coefficients
+  double* sp = ht + (m + 2);
+  double* cl = sp + (m + 1 + 4 * AR_WARPS);
+  float* hf = reinterpret_cast<float*>(cl + 2 * m);
   double* part0 = a.part;
-  double* part1 = a.part + int64_t(a.m + 1) * gridDim.x;
-  for (int c = threadIdx.x; c <= ncol; c += blockDim.x) ht[c] = 0.0;
-  for (int pass = 0; pass < 2; ++pass) {
-    double* part = pass ? part1 : part0;
-    partial_dots(blockIdx, gridDim, a, ncol, part, red);
-    ar_barrier(blockIdx, gridDim, a.bar, a.err);
-    reduce_parts(blockIdx, gridDim, part, ncol, hp);
-    AR_LOOP(i, a.sz) {
-      float s = 0.f;
-      for (int c = 0; c < ncol; ++c) s += a.V[int64_t(c) * a.sz + i] * float(hp[c]);
-      a.w[i] -= s;
-    }
-    for (int c = threadIdx.x; c < ncol; c += blockDim.x) ht[c] += hp[c];
-    __syncthreads();
+  double* part1 = a.part + int64_t(m + 2) * nb;
+  const float4* V = reinterpret_cast<const float4*>(a.V);
+  float4* w = reinterpret_cast<float4*>(a.w);
+  float4* Vn = reinterpret_cast<float4*>(a.V) + int64_t(j + 1) * ldq;
+
+  partial_dots(a, ncol, q0, q1, b, nb, part0, sp);
+  ar_barrier(blockIdx, gridDim, a.bar, a.err);
+  reduce_parts(blockIdx, gridDim, part0, ncol, hp);
+  for (int c = tid; c < ncol; c += blockDim.x) {
+    ht[c] = hp[c];
+    hf[c] = float(hp[c]);
   }
-  // norm of w (reuses part0: every block finished reading it before the
-  // second pass's barrier)
-  {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float s = 0.f;
-    AR_LOOP(i, a.sz) s += a.w[i] * a.w[i];
-    s = warp_sumf(s);
-    if (lane == 0) red[warp] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int q = 0; q < AR_WARPS; ++q) t += double(red[q]);
-      part0[blockIdx.x] = t;
+  __syncthreads();
+  double n1 = 0.0;
+  for (int64_t q = q0 + tid; q < q1; q += blockDim.x) {
+    const float4 v = project4(V, ldq, ncol, q, hf, w[q]);
+    w[q] = v;
+    n1 += double(dot4(v, v));
+  }
+  n1 = block_sum0(n1, sp);  // and every thread's rows of w are written
+  __syncthreads();
+  if (tid == 0) part1[int64_t(ncol) * nb + b] = n1;
+  partial_dots(a, ncol, q0, q1, b, nb, part1, sp);
+  ar_barrier(blockIdx, gridDim, a.bar, a.err);
+  reduce_parts(blockIdx, gridDim, part1, ncol + 1, hp);
+  for (int c = tid; c < ncol; c += blockDim.x) {
+    ht[c] += hp[c];
+    hf[c] = float(hp[c]);
+  }
+  double n2 = hp[ncol];
+  for (int c = 0; c < ncol; ++c) n2 = fma(-hp[c], hp[c], n2);
+  __syncthreads();
+  const bool direct = n2 > 0.75 * hp[ncol];  // the same value in every block
+  if (!direct) {
+    double s = 0.0;
+    for (int64_t q = q0 + tid; q < q1; q += blockDim.x) {
+      const float4 v = project4(V, ldq, ncol, q, hf, w[q]);
+      w[q] = v;
+      s += double(dot4(v, v));
     }
+    s = block_sum0(s, sp);
+    if (tid == 0) part0[b] = s;  // every block is past its reads of part0
     ar_barrier(blockIdx, gridDim, a.bar, a.err);
     reduce_parts(blockIdx, gridDim, part0, 1, hp);
+    n2 = hp[0];
   }
-  const double nrm = sqrt(hp[0]);
-  float* Vn = a.V + int64_t(j + 1) * a.sz;
+  const double nrm = sqrt(n2);
   const float inv = nrm > 0.0 ? float(1.0 / nrm) : 0.f;
-  AR_LOOP(i, a.sz) {
-    const float v = a.w[i] * inv;
-    Vn[i] = v;
-    put_x(a, i, v);
-  }
-  if (blockIdx.x == 0) {
-    // The Givens update runs on one thread over a shared-memory copy of the
-    // column (ht) and of the previous rotations: a chain of dependent
-    // shared-memory accesses instead of global ones.  Same operations in the
-    // same order as on the global arrays.
-    double* cl = red_d(shd, a.m);
-    double* sl = cl + a.m;
-    for (int i = threadIdx.x; i < j; i += blockDim.x) {
-      cl[i] = a.cs[i];
-      sl[i] = a.sn[i];
+  // Block 0 leaves its rows to the other warps while warp 0 runs the Givens
+  // update: one thread over shared-memory copies of the column (ht) and of
+  // the previous rotations, a chain of dependent accesses.
+  const bool givens = b == 0 && tid < 32;
+  if (!givens) {
+    const int64_t t0 = b == 0 ? tid - 32 : tid, dt = b == 0 ? blockDim.x - 32 : blockDim.x;
+    for (int64_t q = q0 + t0; q < q1; q += dt) {
+      float4 v = direct ? project4(V, ldq, ncol, q, hf, w[q]) : w[q];
+      v.x *= inv;
+      v.y *= inv;
+      v.z *= inv;
+      v.w *= inv;
+      Vn[q] = v;
+      put_x4(a, 4 * q, v);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      ht[j + 1] = nrm;
-      for (int i = 0; i < j; ++i) {  // previous rotations
-        const double x = ht[i], y = ht[i + 1];
-        ht[i] = cl[i] * x + sl[i] * y;
-        ht[i + 1] = -sl[i] * x + cl[i] * y;
-      }
-      const double x = ht[j], y = ht[j + 1];
-      const double rho = sqrt(x * x + y * y);
-      const double c0 = rho > 0.0 ? x / rho : 1.0, s0 = rho > 0.0 ? y / rho : 0.0;
-      a.cs[j] = c0;
-      a.sn[j] = s0;
-      ht[j] = rho;
-      ht[j + 1] = 0.0;
-      a.g[j + 1] = -s0 * a.g[j];
-      a.g[j] = c0 * a.g[j];
-      a.scal[0] = fabs(a.g[j + 1]);
-      a.scal[1] = nrm;
-      if (a.scal[0] <= a.scal[4]) {
-        a.stop[1] = j;
-        __threadfence();
-        a.stop[0] = 1;
-      }
-    }
-    __syncthreads();
-    double* Hj = a.H + int64_t(a.m + 1) * j;
-    for (int c = threadIdx.x; c <= j + 1; c += blockDim.x) Hj[c] = ht[c];
+    return;
   }
+  double* sl = cl + m;
+  for (int i = tid; i < j; i += 32) {
+    cl[i] = a.cs[i];
+    sl[i] = a.sn[i];
+  }
+  __syncwarp();
+  if (tid == 0) {
+    ht[j + 1] = nrm;
+    for (int i = 0; i < j; ++i) {  // previous rotations
+      const double x = ht[i], y = ht[i + 1];
+      ht[i] = cl[i] * x + sl[i] * y;
+      ht[i + 1] = -sl[i] * x + cl[i] * y;
+    }
+    const double x = ht[j], y = ht[j + 1];
+    const double rho = sqrt(x * x + y * y);
+    const double c0 = rho > 0.0 ? x / rho : 1.0, s0 = rho > 0.0 ? y / rho : 0.0;
+    a.cs[j] = c0;
+    a.sn[j] = s0;
+    ht[j] = rho;
+    ht[j + 1] = 0.0;
+    a.g[j + 1] = -s0 * a.g[j];
+    a.g[j] = c0 * a.g[j];
+    a.scal[0] = fabs(a.g[j + 1]);
+    a.scal[1] = nrm;
+    if (a.scal[0] <= a.scal[4]) {
+      a.stop[1] = j;
+      __threadfence();
+      a.stop[0] = 1;
+    }
+  }
+  __syncwarp();
+  double* Hj = a.H + int64_t(m + 1) * j;
+  for (int c = tid; c <= j + 1; c += 32) Hj[c] = ht[c];
 }
 TTG_COOP_KERNEL(k_arnoldi, AR_THREADS);
 
@@ -257,31 +350,44 @@ TTG_COOP_KERNEL(k_arnoldi, AR_THREADS);
 // restart (first != 0) r is the right-hand side: scal[3] = ||r||.  The stop
 // threshold reltol * scal[3] goes to scal[4]; a residual already below it
 // (or zero) raises the stop flag with step -1, so the queued steps return at
-// once and the host learns it at its next read of the flags.
+// once and the host learns it at its next read of the flags.  The rows of V
+// and w beyond sz are cleared here.
 TTG_BODY(k_ar_init)(TTG_BLOCK, ArArgs a, const float* r, int first) {
-  __shared__ float red[AR_WARPS];
+  __shared__ double red[AR_WARPS];
   __shared__ double tot[1];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float s = 0.f;
-  AR_LOOP(i, a.sz) s += r[i] * r[i];
-  s = warp_sumf(s);
-  if (lane == 0) red[warp] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int q = 0; q < AR_WARPS; ++q) t += double(red[q]);
-    a.part[blockIdx.x] = t;
+  const int64_t b = blockIdx.x, nb = gridDim.x;
+  const int64_t q0 = quad_at(a, b, nb), q1 = quad_at(a, b + 1, nb);
+  auto load = [&](int64_t q) {  // r has sz entries
+    const int64_t i = 4 * q;
+    float4 v;
+    v.x = r[i];
+    v.y = i + 1 < a.sz ? r[i + 1] : 0.f;
+    v.z = i + 2 < a.sz ? r[i + 2] : 0.f;
+    v.w = i + 3 < a.sz ? r[i + 3] : 0.f;
+    return v;
+  };
+  double s = 0.0;
+  for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    const float4 v = load(q);
+    s += double(dot4(v, v));
   }
+  s = block_sum0(s, red);
+  if (threadIdx.x == 0) a.part[b] = s;
   ar_barrier(blockIdx, gridDim, a.bar, a.err);
   reduce_parts(blockIdx, gridDim, a.part, 1, tot);
   const double beta = sqrt(tot[0]);
   const float inv = beta > 0.0 ? float(1.0 / beta) : 0.f;
-  AR_LOOP(i, a.sz) {
-    const float v = r[i] * inv;
-    a.V[i] = v;
-    put_x(a, i, v);
+  for (int64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    float4 v = load(q);
+    v.x *= inv;
+    v.y *= inv;
+    v.z *= inv;
+    v.w *= inv;
+    reinterpret_cast<float4*>(a.V)[q] = v;
+    put_x4(a, 4 * q, v);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (b == 0 && threadIdx.x == 0) {
+    for (int64_t i = a.sz; i < a.ldv; ++i) a.w[i] = 0.f;
     for (int k = 0; k <= a.m; ++k) a.g[k] = 0.0;
     a.g[0] = beta;
     a.scal[2] = beta;
@@ -321,13 +427,20 @@ TTG_BODY(k_ar_update)(TTG_BLOCK, ArArgs a, int k, float* x) {
     }
   }
   __syncthreads();
-  AR_LOOP(i, a.sz) {
-    float s = 0.f;
-    for (int c = 0; c < k; ++c) s += a.V[int64_t(c) * a.sz + i] * float(y[c]);
-    x[i] += s;
+  float* yf = reinterpret_cast<float*>(Hs);  // H is done with
+  for (int e = threadIdx.x; e < k; e += blockDim.x) yf[e] = -float(y[e]);
+  __syncthreads();
+  const float4* V = reinterpret_cast<const float4*>(a.V);
+  AR_LOOP(q, a.ldv / 4) {
+    const int64_t i = 4 * q;
+    const float4 s = project4(V, a.ldv / 4, k, q, yf, make_float4(0.f, 0.f, 0.f, 0.f));
+    x[i] += s.x;
+    if (i + 1 < a.sz) x[i + 1] += s.y;
+    if (i + 2 < a.sz) x[i + 2] += s.z;
+    if (i + 3 < a.sz) x[i + 3] += s.w;
   }
 }
-TTG_KERNEL(k_ar_update, 0);
+TTG_KERNEL(k_ar_update, AR_THREADS);
 
 // Centre block-Jacobi on vectors in the reversed layout v[k + rx2 (j + n i)]:
 // out[k, j, i] = sum_m J[i, j, m, k] v[k, m, i] with the FP64 blocks J of
@@ -372,20 +485,22 @@ struct Gmres32 {
   ArArgs a{};
 
   Gmres32(Context* cc, int64_t n, int restart) : c(cc), sz(n), m(restart) {
-    V.reset(c, size_t(sz) * (m + 1));
-    w.reset(c, sz);
+    const int64_t ldv = (sz + 3) & ~int64_t(3);
+    V.reset(c, size_t(ldv) * (m + 1));
+    w.reset(c, ldv);
     r.reset(c, sz);
     small.reset(c, size_t(m + 1) * m + 2 * m + (m + 1) + 8);
     int occ = 0;
     occ = max_active_blocks(k_arnoldi.fn(), AR_THREADS, arnoldi_smem());
     if (occ < 1) occ = 1;
-    int64_t want = (sz + AR_THREADS * 4 - 1) / (AR_THREADS * 4);
+    const int64_t want = (sz + AR_ROWS - 1) / AR_ROWS;
     const int64_t cap = int64_t(c->num_sms) * std::min(occ, 2);
     blocks = int(std::max<int64_t>(1, std::min(want, cap)));
-    part.reset(c, size_t(2) * (m + 1) * blocks);
+    part.reset(c, size_t(2) * (m + 2) * blocks);
     bar.reset(c, 4);
     memset_async(c, bar.p(), 0, 4 * sizeof(unsigned));
     a.sz = sz;
+    a.ldv = ldv;
     a.m = m;
     a.V = V.p();
     a.w = w.p();
@@ -404,10 +519,8 @@ struct Gmres32 {
   }
 
   size_t arnoldi_smem() const {
-    return sizeof(double) * (2 * (m + 2)) + sizeof(float) * AR_WARPS * (m + 1) + 8 +
-           sizeof(double) * 2 * m + 16;
+    return sizeof(double) * arnoldi_doubles(m) + sizeof(float) * (m + 1);
   }
-
 
   // Right-preconditioned operand: X = bf16(P v) for the centre block-Jacobi
   // blocks J (FP64, natural layout), v in the reversed layout.
@@ -460,7 +573,7 @@ struct Gmres32 {
         for (int jj = j; jj < jend; ++jj) {
           const int jv = jj;
           seqs.push_back(c->ev_seq);
-          if (J) prec_x(op, J, V.p() + int64_t(jj) * sz);  // X = bf16(P V(:, jv))
+          if (J) prec_x(op, J, V.p() + int64_t(jj) * a.ldv);  // X = bf16(P V(:, jv))
           op.apply_converted(c, w.p());  // X holds V(:, jv) (k_ar_init / k_arnoldi)
           launch(c, k_arnoldi, blocks, AR_THREADS, arnoldi_smem(), a, jv);
         }
