@@ -4,10 +4,11 @@
 // The GEMM is the contraction engine of the FP64 (parity) path: every local
 // matvec (bfun3) and every interface update (compute_next_Phi) is written as
 // three batched column-major GEMMs whose operand layouts need no explicit
-// permutations (see local_ops.cu).  Tiles: 64x64x16 per CTA, 4 warps of
-// 32x32, each warp issuing mma.sync.m8n8k4 f64 (the FP64 tensor path; tcgen05
-// has no FP64 kind).  Global->shared staging with cp.async (8-byte granules so
-// any leading dimension works), double buffered.
+// permutations (see local_ops.cu).  CTA tiles of 64x64, 32x64 or 32x32 by 16,
+// four warps, each warp issuing mma.sync.m8n8k4 f64 (the FP64 tensor path;
+// tcgen05 has no FP64 kind, and the larger mma shapes run at the same rate).
+// Global->shared staging with cp.async through a ring of three tiles, 16-byte
+// granules where the operand's alignment allows, else 8-byte ones.
 #include "group.cuh"
 #include "kernels.h"
 #include "dmma.cuh"
@@ -16,9 +17,9 @@ namespace ttg {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, PADS = 8;
+constexpr int BK = 16, GEMM_STAGES = 3, GEMM_THREADS = 128;
 // Split-K partial values one CTA may sum in the GEMM kernel itself.
-constexpr int64_t SPLITK_INKERNEL_MAX = 4096;
+constexpr int64_t SPLITK_INKERNEL_MAX = 8192;
 
 struct GemmP {
   int64_t M, N, K;
@@ -30,6 +31,7 @@ struct GemmP {
   int64_t ldc, sC;
   double alpha, beta;
   const int* skip;  // optional: return at once when *skip != 0
+  int vecA, vecB;   // operand admits 16-byte loads (see vec16)
   // Split-K: nsplit > 1 slices of kc columns of K per batch item, blockIdx.z =
   // item * nsplit + slice.  Each slice writes its partial tile to `part`
   // ([item][slice] blocks of M x N, ld M).  With `cnt` (one arrival counter
@@ -41,11 +43,91 @@ struct GemmP {
   unsigned* cnt;
 };
 
-template <bool TA, bool TB>
+// One operand tile of T rows (of C) by BK in shared memory, in the order its
+// global layout has: k contiguous (KC) as rows of BK + 4, else k slices of
+// T + 4.  Either pitch is 4 mod 16 doubles, which puts the 16 doubles that a
+// half-warp reads for an mma fragment (4 of k by 4 rows) in different banks.
+template <int T, bool KC>
+struct TileS {
+  static constexpr int NT = GEMM_THREADS;
+  static constexpr int LD = KC ? BK + 4 : T + 4;
+  static constexpr int SIZE = KC ? T * LD : BK * LD;
+  static __device__ __forceinline__ double at(const double* s, int r, int k) {
+    return KC ? s[r * LD + k] : s[k * LD + r];
+  }
+  // Rows r0.. of R, k0.. of K of the operand g (element (r, k) at
+  // g[k + r ld] or g[r + k ld]); zeros outside.
+  static __device__ __forceinline__ void load(double* s, const double* __restrict__ g, int64_t ld,
+                                              int64_t r0, int64_t R, int64_t k0, int64_t K,
+                                              bool vec) {
+    const int tid = threadIdx.x;
+    if (KC) {
+      if (vec) {
+        const int k = (tid & 7) * 2, rb = tid >> 3;
+        const int64_t left = K - (k0 + k);
+        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+#pragma unroll
+        for (int i = 0; i < BK * T / (2 * NT); ++i) {
+          const int r = rb + NT / (BK / 2) * i;
+          const bool ok = bytes && r0 + r < R;
+          cp_async16(s + r * LD + k, ok ? g + (k0 + k) + (r0 + r) * ld : g, ok ? bytes : 0);
+        }
+      } else {
+        const int k = tid & 15, rb = tid >> 4;
+        const bool kok = k0 + k < K;
+#pragma unroll
+        for (int i = 0; i < BK * T / NT; ++i) {
+          const int r = rb + NT / BK * i;
+          const bool ok = kok && r0 + r < R;
+          cp_async8(s + r * LD + k, ok ? g + (k0 + k) + (r0 + r) * ld : g, ok);
+        }
+      }
+    } else {
+      if (vec) {
+        const int r = (tid % (T / 2)) * 2, kb = tid / (T / 2);
+        const int64_t left = R - (r0 + r);
+        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+#pragma unroll
+        for (int i = 0; i < BK * T / (2 * NT); ++i) {
+          const int k = kb + 2 * NT / T * i;
+          const bool ok = bytes && k0 + k < K;
+          cp_async16(s + k * LD + r, ok ? g + (r0 + r) + (k0 + k) * ld : g, ok ? bytes : 0);
+        }
+      } else {
+        const int r = tid % T, kb = tid / T;
+        const bool rok = r0 + r < R;
+#pragma unroll
+        for (int i = 0; i < BK * T / NT; ++i) {
+          const int k = kb + NT / T * i;
+          const bool ok = rok && k0 + k < K;
+          cp_async8(s + k * LD + r, ok ? g + (r0 + r) + (k0 + k) * ld : g, ok);
+        }
+      }
+    }
+  }
+};
+
+template <int BM, int BN, bool TA, bool TB>
+constexpr size_t gemm_smem() {
+  return sizeof(double) * GEMM_STAGES * (TileS<BM, TA>::SIZE + TileS<BN, !TB>::SIZE);
+}
+
+// Bound by the FP64 tensor rate where the tiles fill the device, by the chain
+// of launch, first loads and last stores where there are few.  Local matvec
+// (three products), measured against pitches of 72 (8-way bank conflicts on k-
+// contiguous stores), two stages, 8-byte copies and 64 x 64 tiles only:
+// 20 x 32 x 20 19.3 us / 28.0; 61 x 64 x 67 48 / 59; 128 x 64 x 128 138 / 184
+// (20.5 TFLOP/s); 187 x 64 x 203 368 / 440; 512 x 64 x 512 3.92 / 4.66 ms (31
+// TFLOP/s).  Four stages, eight warps per tile and the larger mma shapes
+// measure the same or slower.
+template <int BM, int BN, bool TA, bool TB>
 TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
   pdl_begin();
-  __shared__ double As[2][BK][BM + PADS];
-  __shared__ double Bs[2][BK][BN + PADS];
+  extern __shared__ __align__(16) double gsm[];
+  constexpr int NT = GEMM_THREADS;
+  using SA = TileS<BM, TA>;
+  using SB = TileS<BN, !TB>;
+  constexpr int MI = BM / 16, NI = BN / 16;  // 8 x 8 fragments of a warp
   if (p.skip && *p.skip) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool split = p.nsplit > 1;
@@ -58,94 +140,59 @@ TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
   const int64_t m0 = int64_t(blockIdx.x) * BM, n0 = int64_t(blockIdx.y) * BN;
   const int64_t M = p.M, N = p.N;
 
-  auto load_tile = [&](int64_t k0, int buf) {
-    if (!TA) {  // m contiguous
-      const int m = tid & 63, kb = tid >> 6;
-      const int64_t gm = m0 + m;
+  double acc[MI][NI][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int k = kb + 2 * i;
-        const int64_t gk = k0 + k;
-        const bool ok = gm < M && gk < K;
-        cp_async8(&As[buf][k][m], ok ? A + gm + gk * p.lda : A, ok);
-      }
-    } else {  // k contiguous: A(m,k) = A[k + m*lda]
-      const int k = tid & 15, mb = tid >> 4;
-      const int64_t gk = k0 + k;
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int m = mb + 8 * i;
-        const int64_t gm = m0 + m;
-        const bool ok = gm < M && gk < K;
-        cp_async8(&As[buf][k][m], ok ? A + gk + gm * p.lda : A, ok);
-      }
-    }
-    if (!TB) {  // k contiguous: B(k,n) = B[k + n*ldb]
-      const int k = tid & 15, nb = tid >> 4;
-      const int64_t gk = k0 + k;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int n = nb + 8 * i;
-        const int64_t gn = n0 + n;
-        const bool ok = gn < N && gk < K;
-        cp_async8(&Bs[buf][k][n], ok ? B + gk + gn * p.ldb : B, ok);
-      }
-    } else {  // n contiguous: B(k,n) = B[n + k*ldb]
-      const int n = tid & 63, kb = tid >> 6;
-      const int64_t gn = n0 + n;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int k = kb + 2 * i;
-        const int64_t gk = k0 + k;
-        const bool ok = gn < N && gk < K;
-        cp_async8(&Bs[buf][k][n], ok ? B + gn + gk * p.ldb : B, ok);
-      }
+    for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+
+  const int g = lane >> 2, t = lane & 3;
+  const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
+  const int ktiles = int((K + BK - 1) / BK);
+  auto load_tile = [&](int kt) {
+    if (kt < ktiles) {
+      double* s = gsm + (kt % GEMM_STAGES) * (SA::SIZE + SB::SIZE);
+      SA::load(s, A, p.lda, m0, M, int64_t(kt) * BK, K, p.vecA);
+      SB::load(s + SA::SIZE, B, p.ldb, n0, N, int64_t(kt) * BK, K, p.vecB);
     }
     cp_async_commit();
   };
-
-  double acc[4][4][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int s = 0; s < GEMM_STAGES - 1; ++s) load_tile(s);
+  for (int kt = 0; kt < ktiles; ++kt) {
+    cp_async_wait<GEMM_STAGES - 2>();
+    __syncthreads();  // tile kt has landed, tile kt - 1 is read out
+    load_tile(kt + GEMM_STAGES - 1);
+    const double* As = gsm + (kt % GEMM_STAGES) * (SA::SIZE + SB::SIZE);
+    const double* Bs = As + SA::SIZE;
+    // Fragments of the next k slice are read while the mma of this one run.
+    double a[2][MI], b[2][NI];
+    auto frag = [&](int kk) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-  const int g = lane >> 2, t = lane & 3;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-  const int64_t ktiles = (K + BK - 1) / BK;
-  if (ktiles > 0) load_tile(0, 0);
-  for (int64_t kt = 0; kt < ktiles; ++kt) {
-    const int buf = int(kt & 1);
-    if (kt + 1 < ktiles) {
-      load_tile((kt + 1) * BK, buf ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+      for (int i = 0; i < MI; ++i) a[kk & 1][i] = SA::at(As, wm + i * 8 + g, kk * 4 + t);
+#pragma unroll
+      for (int j = 0; j < NI; ++j) b[kk & 1][j] = SB::at(Bs, wn + j * 8 + g, kk * 4 + t);
+    };
+    frag(0);
 #pragma unroll
     for (int kk = 0; kk < BK / 4; ++kk) {
-      double a[4], b[4];
+      if (kk + 1 < BK / 4) frag(kk + 1);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk * 4 + t][wm + i * 8 + g];
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[buf][kk * 4 + t][wn + j * 8 + g];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+        for (int j = 0; j < NI; ++j)
+          dmma(acc[i][j][0], acc[i][j][1], a[kk & 1][i], b[kk & 1][j]);
     }
-    __syncthreads();
   }
 
   double* __restrict__ C = p.C + item * p.sC;
   if (!split) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < MI; ++i) {
       const int64_t row = m0 + wm + i * 8 + g;
       if (row >= M) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < NI; ++j) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int64_t col = n0 + wn + j * 8 + 2 * t + e;
@@ -166,11 +213,11 @@ TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
   const int64_t MN = M * N;
   double* Pme = p.part + blockIdx.z * MN;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < MI; ++i) {
     const int64_t row = m0 + wm + i * 8 + g;
     if (row >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < NI; ++j) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int64_t col = n0 + wn + j * 8 + 2 * t + e;
@@ -192,21 +239,38 @@ TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  // The last slice: every thread sums its elements over the slices in slice
+  // order, its loads of one slice in flight together.
   const double* P0 = p.part + item * p.nsplit * MN;
-  for (int e = tid; e < BM * BN; e += 128) {
-    const int64_t row = m0 + (e % BM), col = n0 + (e / BM);
-    if (row >= M || col >= N) continue;
-    const int64_t off = row + col * M;
-    double acc2 = 0.0;
-    for (int64_t z = 0; z < p.nsplit; ++z) acc2 += __ldcg(P0 + z * MN + off);
-    double* dst = C + row + col * p.ldc;
-    double v = p.alpha * acc2;
-    if (p.beta != 0.0) v += p.beta * *dst;
-    *dst = v;
+  constexpr int EPT = BM * BN / NT < 8 ? BM * BN / NT : 8;
+  for (int e0 = tid; e0 < BM * BN; e0 += NT * EPT) {
+    double acc2[EPT];
+    bool ok[EPT];
+    int64_t off[EPT];
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+      const int e = e0 + q * NT;
+      const int64_t row = m0 + e % BM, col = n0 + e / BM;
+      ok[q] = row < M && col < N;
+      off[q] = ok[q] ? row + col * M : 0;
+      acc2[q] = 0.0;
+    }
+    for (int64_t z = 0; z < p.nsplit; ++z)
+#pragma unroll
+      for (int q = 0; q < EPT; ++q) acc2[q] += __ldcg(P0 + z * MN + off[q]);
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+      if (!ok[q]) continue;
+      const int e = e0 + q * NT;
+      double* dst = C + (m0 + e % BM) + (n0 + e / BM) * p.ldc;
+      double v = p.alpha * acc2[q];
+      if (p.beta != 0.0) v += p.beta * *dst;
+      *dst = v;
+    }
   }
 }
-template <bool TA, bool TB>
-TTG_KERNEL_T(k_gemm_f64, 128, TA, TB);
+template <int BM, int BN, bool TA, bool TB>
+TTG_KERNEL_T(k_gemm_f64, GEMM_THREADS, BM, BN, TA, TB);
 
 // ---------------------------------------------------------------------------
 // Reductions
@@ -510,6 +574,84 @@ int grid_for(Context* c, int64_t n, int threads = 256) {
   return int(b);
 }
 
+// An operand whose columns (or rows, k contiguous) all start on 16 bytes.
+bool vec16(const double* p, int64_t ld, int64_t stride, int64_t batch) {
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 2 == 0 &&
+         (batch == 1 || stride % 2 == 0);
+}
+
+template <int BM, int BN, bool TA, bool TB>
+void gemm_launch(Context* c, dim3 grid, const GemmP& p) {
+  constexpr size_t smem = gemm_smem<BM, BN, TA, TB>();
+  if (smem > 48 * 1024) ensure_smem_attr(k_gemm_f64<BM, BN, TA, TB>.fn(), c->device, int(smem));
+  launch(c, k_gemm_f64<BM, BN, TA, TB>, grid, GEMM_THREADS, smem, p);
+}
+
+template <int BM, int BN>
+void gemm_launch(Context* c, bool tA, bool tB, dim3 grid, const GemmP& p) {
+  if (!tA && !tB)
+    gemm_launch<BM, BN, false, false>(c, grid, p);
+  else if (!tA && tB)
+    gemm_launch<BM, BN, false, true>(c, grid, p);
+  else if (tA && !tB)
+    gemm_launch<BM, BN, true, false>(c, grid, p);
+  else
+    gemm_launch<BM, BN, true, true>(c, grid, p);
+}
+
+struct GemmTile {
+  int bm, bn;
+  double cost;  // relative time per tile element
+};
+constexpr GemmTile GEMM_TILES[] = {{64, 64, 1.0}, {32, 64, 1.1}, {32, 32, 1.25}};
+
+struct GemmPlan {
+  GemmTile tile;
+  int64_t gx, gy, split, kc;
+};
+
+// CTA tile and number of K slices: the pair with the least estimated time, in
+// cycles.  An SM multiplies a 64 x 64 x 16 step in 1024 cycles (m8n8k4 at 37
+// TFLOP/s on the device) whichever of its CTAs issues it, so the product takes
+// the work of the fullest SM, tile edges that hang over the matrix included;
+// a smaller tile costs more per element (it loads more operand per product),
+// and an SM with fewer than four CTAs leaves the pipe idle between their steps.
+// Slices add their partials, written once and read once, and either the
+// last CTA's sum or a second kernel.  Interface update with this rule, against
+// split-K to two 64 x 64 CTAs per SM: 61 x 64 x 67 54 / 83 us, 128 x 64 x 128
+// 136 / 216, 512 x 64 x 512 4.4 / 8.0 ms.
+GemmPlan plan_gemm(Context* c, int64_t M, int64_t N, int64_t K, int64_t batch, bool may_split) {
+  const int64_t ktiles = (K + BK - 1) / BK;
+  GemmPlan best{};
+  double best_t = 0.0;
+  for (const GemmTile& t : GEMM_TILES) {
+    const int64_t gx = (M + t.bm - 1) / t.bm, gy = (N + t.bn - 1) / t.bn, ctas = gx * gy * batch;
+    if (&t != GEMM_TILES && (gy > 65535 || gx > 0x7fffffff)) continue;  // the grid's limits
+    int64_t smax = 1;
+    if (may_split && ctas < 4 * c->num_sms && ktiles >= 8 && ctas <= GEMM_TILE_COUNTERS)
+      smax = std::min({ktiles / 4, 8 * c->num_sms / ctas + 1, 65535 / batch});
+    int64_t prev = 0;
+    for (int64_t s = 1; s <= smax; s = s < 8 ? s + 1 : s + s / 4) {
+      const int64_t kt = (ktiles + s - 1) / s, ns = (ktiles + kt - 1) / kt;
+      if (ns == prev) continue;
+      prev = ns;
+      const int64_t per_sm = (ctas * ns + c->num_sms - 1) / c->num_sms;
+      const double idle = per_sm == 1 ? 2.2 : per_sm == 2 ? 1.45 : per_sm == 3 ? 1.15 : 1.0;
+      double est = double(per_sm * kt) * (t.bm * t.bn / 4) * t.cost * idle;
+      if (ns > 1) {
+        const int64_t te = std::min<int64_t>(M, t.bm) * std::min<int64_t>(N, t.bn);
+        est += 16.0 * double(ns * M * N * batch) / 2600.0 +
+               (ns * te <= SPLITK_INKERNEL_MAX ? 2500.0 : 4500.0);
+      }
+      if (best_t == 0.0 || est < best_t) {
+        best = GemmPlan{t, gx, gy, ns, kt * BK};
+        best_t = est;
+      }
+    }
+  }
+  return best;
+}
+
 }  // namespace
 
 void gemm_f64(Context* c, bool tA, bool tB, int64_t M, int64_t N, int64_t K, double alpha,
@@ -528,50 +670,34 @@ void gemm_f64(Context* c, bool tA, bool tB, int64_t M, int64_t N, int64_t K, dou
     return;
   }
   TTG_REQUIRE(batch <= 65535, "gemm batch %lld too large", (long long)batch);
-  const int64_t gx = (M + BM - 1) / BM, gy = (N + BN - 1) / BN;
-  TTG_REQUIRE(gy <= 65535 && gx <= 0x7fffffff, "gemm too large");
-  GemmP p{M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, alpha, beta, c->skip, 1, 0, nullptr,
-          nullptr};
-  dim3 grid{unsigned(gx), unsigned(gy), unsigned(batch)};
-  // Split-K when the output tiles (times the batch) cannot fill the SMs and
-  // K is long: one CTA's FP64 DMMA rate is a small share of the device's, so
-  // a few long-K CTAs (inner products of tall matrices: interface updates,
-  // Gram matrices, projections) would run for about K x 30 ns each.  K is cut
-  // into slices of at least 4 k-tiles so that about two CTAs per SM run.  The
-  // slices of a tile are summed in slice order: by the last slice to finish
-  // when the partials are few (no second launch), else by a reduction kernel
-  // spread over the device (one CTA reading many partials is latency-bound).
-  DBuf<double> part;
-  const int64_t ctas = gx * gy * batch;
-  const int64_t ktiles = (K + BK - 1) / BK;
+  TTG_REQUIRE((N + 63) / 64 <= 65535 && (M + 63) / 64 <= 0x7fffffff, "gemm too large");
+  // Split-K cuts a long K into slices of at least 4 k-tiles where the output
+  // tiles leave SMs idle (inner products of tall matrices: interface updates,
+  // Gram matrices, projections).  The slices of a tile are summed in slice
+  // order: by the last slice to finish when the partials are few (no second
+  // launch), else by a reduction kernel spread over the device (one CTA
+  // reading many partials is latency-bound).
   // (A context without an allocator -- the caller-scratch entry point -- runs
   // every product unsplit.)
-  if (c->alloc && c->d_tile_cnt && ctas < c->num_sms && ktiles >= 8 &&
-      ctas <= GEMM_TILE_COUNTERS) {
-    int64_t s = std::min<int64_t>((2 * c->num_sms + ctas - 1) / ctas, ktiles / 4);
-    if (s * batch > 65535) s = 65535 / batch;
-    if (s >= 2) {
-      const int64_t kc = (ktiles + s - 1) / s * BK;
-      s = (K + kc - 1) / kc;
-      if (s >= 2) {
-        part.reset(c, batch * s * M * N);
-        p.nsplit = s;
-        p.kc = kc;
-        p.part = part.p();
-        const int64_t tile_elems = std::min<int64_t>(M, BM) * std::min<int64_t>(N, BN);
-        if (s * tile_elems <= SPLITK_INKERNEL_MAX) p.cnt = c->d_tile_cnt;
-        grid.z = unsigned(batch * s);
-      }
-    }
+  const GemmPlan pl = plan_gemm(c, M, N, K, batch, c->alloc && c->d_tile_cnt);
+  GemmP p{M,  N,     K,       A,  lda, sA, B, ldb, sB, C, ldc, sC, alpha, beta, c->skip,
+          vec16(A, lda, sA, batch), vec16(B, ldb, sB, batch), 1, 0, nullptr, nullptr};
+  dim3 grid{unsigned(pl.gx), unsigned(pl.gy), unsigned(batch * pl.split)};
+  DBuf<double> part;
+  if (pl.split > 1) {
+    part.reset(c, batch * pl.split * M * N);
+    p.nsplit = pl.split;
+    p.kc = pl.kc;
+    p.part = part.p();
+    const int64_t te = std::min<int64_t>(M, pl.tile.bm) * std::min<int64_t>(N, pl.tile.bn);
+    if (pl.split * te <= SPLITK_INKERNEL_MAX) p.cnt = c->d_tile_cnt;
   }
-  if (!tA && !tB)
-    launch(c, k_gemm_f64<false, false>, grid, 128, 0, p);
-  else if (!tA && tB)
-    launch(c, k_gemm_f64<false, true>, grid, 128, 0, p);
-  else if (tA && !tB)
-    launch(c, k_gemm_f64<true, false>, grid, 128, 0, p);
+  if (pl.tile.bm == 64)
+    gemm_launch<64, 64>(c, tA, tB, grid, p);
+  else if (pl.tile.bn == 64)
+    gemm_launch<32, 64>(c, tA, tB, grid, p);
   else
-    launch(c, k_gemm_f64<true, true>, grid, 128, 0, p);
+    gemm_launch<32, 32>(c, tA, tB, grid, p);
   TTG_CHECK_LAUNCH();
   if (p.nsplit > 1 && !p.cnt) {
     launch(c, k_splitk_reduce, grid_for(c, M * N * batch), 256, 0, M, N, p.nsplit, batch,
