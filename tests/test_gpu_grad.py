@@ -240,3 +240,20 @@ def test_grad_d12_n32_r64_full_size(ctx):
                                                                              b.cores())[0])
         assert abs(v - vr) <= 1e-11 * scale, name
         assert grad_rel(split(G, xc), Gr) <= GRAD_TOL, name
+
+
+def test_grad_xAx_without_kept_intermediates(ctx):
+    """A core whose left products exceed what the sweep keeps (1 GiB) forms
+    them again.  f is quadratic in every core, so <x_k, g_k> = 2 f for all k;
+    inner products of 4.5e7 terms round at 1e-13 of their size."""
+    rng = np.random.default_rng(3)
+    n, r = [4, 172, 4], [1, 512, 512, 1]
+    xs = rand_cores(rng, n, r)
+    ra = [1, 3, 3, 1]
+    As = [np.asfortranarray(rng.standard_normal((ra[k], n[k], n[k], ra[k + 1]))) for k in range(3)]
+    for k in range(3):
+        As[k] = As[k] + np.transpose(As[k], (0, 2, 1, 3))
+    v, G = ttgpu.grad_xAx(to_tt(xs), to_mat(As), ctx=ctx)
+    for xk, gk in zip(xs, split(G, xs)):
+        scale = np.linalg.norm(xk) * np.linalg.norm(gk)
+        assert abs(np.vdot(xk, gk) - 2.0 * v) <= GRAD_TOL * scale

@@ -10,13 +10,13 @@
 // right of k contracted with everything that touched core k.
 //
 // <x, A x>: the interfaces are those of AMEn's local system (compute_next_Phi,
-//   solve/amen_solve2.m:834-920, without its normalisation).  With the left
-//   interface L_k [bra, ket, ra] and the right interface R_k [ket, ra, bra],
-//   the derivative through the bra copy of x_k is the local matvec bfun3
-//   (solve/amen_solve2.m:924-951) L_k x A_k x R_{k+1} applied to x_k, and the
-//   derivative through the ket copy is the same with bra and ket exchanged
-//   (transposed interfaces and A_k^T).  Both run on the DMMA GEMMs of the
-//   local matvec.
+//   solve/amen_solve2.m:834-920, without its normalisation), L_k [bra, ket, ra]
+//   from the left and R_k [ket, ra, bra] from the right.  The derivative
+//   through the bra copy of x_k is the local matvec bfun3
+//   (solve/amen_solve2.m:924-951) L_k x A_k x R_{k+1} applied to x_k, whose
+//   first two products are those of the update of R_k: it takes one product
+//   more in the right sweep.  The derivative through the ket copy, likewise,
+//   is the left update's last intermediate, W2_k, times R_{k+1}.
 // <x, b>:   two interface sweeps Psi_L [rx, rb], Psi_R [rx, rb]; three GEMMs
 //   per core.
 // sum_s (X[idx_s] - y_s)^2: per sample s, the row vector l_k(s) = product of
@@ -32,7 +32,6 @@
 #include "grad.h"
 #include "dmma.cuh"
 #include "kernels.h"
-#include "local_ops.h"
 
 namespace ttg {
 
@@ -43,41 +42,12 @@ constexpr int PT = 64;           // samples per propagation tile
 constexpr int GT = 512;          // samples per gradient (split-K) tile
 constexpr int SORT_CHUNK = 1024; // samples per sorting warp
 constexpr int64_t MAX_BUCKETS = 8192;
+// Bytes of intermediates the left sweep of <x, A x> keeps for the right one.
+constexpr int64_t KEEP_MAX = int64_t(1) << 30;
 
 int blocks_for(int64_t n, int threads = 256) {
   int64_t b = (n + threads - 1) / threads;
   return int(b < 1 ? 1 : (b > 65535 * 16 ? 65535 * 16 : b));
-}
-
-// ---------------------------------------------------------------------------
-// 4-D permutation: out[sum_a i_a * ostride_a] = in[i0 + d0*(i1 + d1*(i2 + d2*i3))]
-// ---------------------------------------------------------------------------
-struct Perm4 {
-  int64_t d0, d1, d2, d3;
-  int64_t o0, o1, o2, o3;
-};
-
-__global__ void k_permute4(Perm4 p, const double* __restrict__ in, double* __restrict__ out) {
-  const int64_t total = p.d0 * p.d1 * p.d2 * p.d3;
-  for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < total;
-       t += int64_t(gridDim.x) * blockDim.x) {
-    int64_t r = t;
-    const int64_t i0 = r % p.d0;
-    r /= p.d0;
-    const int64_t i1 = r % p.d1;
-    r /= p.d1;
-    const int64_t i2 = r % p.d2;
-    const int64_t i3 = r / p.d2;
-    out[i0 * p.o0 + i1 * p.o1 + i2 * p.o2 + i3 * p.o3] = in[t];
-  }
-}
-
-void permute4(Context* c, const Perm4& p, const double* in, double* out) {
-  const int64_t total = p.d0 * p.d1 * p.d2 * p.d3;
-  if (total <= 0) return;
-  k_permute4<<<blocks_for(total), 256, 0, c->stream>>>(p, in, out);
-  c->launches += 1;
-  TTG_CHECK_LAUNCH();
 }
 
 // ---------------------------------------------------------------------------
@@ -460,7 +430,10 @@ void check_tt_vector(const ttg_tt_s* x, const char* what) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// <x, A x>
+// <x, A x>: eight products per core (three each way for the interfaces, two
+// for the gradient).  Bound by the chain of some 120 dependent launches of
+// 5-10 us: d = 12, n = 32, rank 64 721 us, against 1151 us with two whole local
+// matvecs and three permutations per core.
 // ---------------------------------------------------------------------------
 void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, double* value) {
   check_tt_vector(x, "x");
@@ -474,48 +447,68 @@ void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, do
                 (long long)A->n[k], (long long)A->m[k], (long long)x->n[k]);
   const auto& r = x->r;
   const auto& ra = A->r;
-  // Interfaces: L[k] [r_k, r_k, ra_k] (k = 0..d), R[k] [r_k, ra_k, r_k].
-  std::vector<int64_t> off(d + 2, 0);
-  for (int64_t k = 0; k <= d; ++k) off[k + 1] = off[k] + r[k] * r[k] * ra[k];
-  DBuf<double> L(c, off[d + 1]), R(c, off[d + 1]);
-  fill_f64(c, 1, 1.0, L.p());
-  fill_f64(c, 1, 1.0, R.p() + off[d]);
-  for (int64_t k = 0; k < d; ++k) {
-    const double* xk = x->core + x->ps[k];
-    next_phi_f64(c, 0, r[k], x->n[k], r[k + 1], r[k], r[k + 1], ra[k], ra[k + 1], L.p() + off[k],
-                 xk, A->core + A->ps[k], xk, L.p() + off[k + 1]);
+  // Interfaces: L[k] [r_k, r_k, ra_k] (k = 0..d), R [r_k, ra_k, r_k] of the
+  // right sweep's current core.
+  std::vector<int64_t> off(d + 2, 0), woff(d + 1, 0);
+  int64_t nphi = 1, w1max = 1, w2max = 1;
+  for (int64_t k = 0; k <= d; ++k) {
+    off[k + 1] = off[k] + r[k] * r[k] * ra[k];
+    nphi = std::max(nphi, r[k] * r[k] * ra[k]);
   }
-  for (int64_t k = d - 1; k >= 0; --k) {
-    const double* xk = x->core + x->ps[k];
-    next_phi_f64(c, 1, r[k], x->n[k], r[k + 1], r[k], r[k + 1], ra[k], ra[k + 1],
-                 R.p() + off[k + 1], xk, A->core + A->ps[k], xk, R.p() + off[k]);
+  for (int64_t k = 0; k < d; ++k) {
+    const int64_t w2 = r[k] * x->n[k] * ra[k + 1] * r[k + 1];
+    woff[k + 1] = woff[k] + w2;
+    w2max = std::max(w2max, w2);
+    w1max = std::max(w1max, r[k] * ra[k] * x->n[k] * r[k + 1]);
+  }
+  // The left sweep's W2 of every core serve the right sweep, unless that
+  // would hold too much memory: then each is formed again.
+  const bool keep = woff[d] * int64_t(sizeof(double)) <= KEEP_MAX;
+  DBuf<double> L(c, off[d + 1]), R0(c, nphi), R1(c, nphi);
+  DBuf<double> W1(c, w1max), W2(c, keep ? woff[d] : w2max), Z1(c, w2max), Z2(c, w1max);
+  double* Rk = R0.p();
+  double* Rn = R1.p();
+  fill_f64(c, 1, 1.0, L.p());
+  fill_f64(c, 1, 1.0, Rk);
+  // W1[(y,al),(j,c)] = L^T x, W2_c[y,(m,be)] = W1_c[y,(al,j)] A[(al,j),(m,be)]
+  auto left_products = [&](int64_t k, double* w2) {
+    const int64_t r1 = r[k], r2 = r[k + 1], a1 = ra[k], a2 = ra[k + 1], n = x->n[k];
+    gemm_f64(c, true, false, r1 * a1, n * r2, r1, 1.0, L.p() + off[k], r1, 0, x->core + x->ps[k],
+             r1, 0, 0.0, W1.p(), r1 * a1, 0, 1);
+    gemm_f64(c, false, false, r1, n * a2, a1 * n, 1.0, W1.p(), r1, r1 * a1 * n,
+             A->core + A->ps[k], a1 * n, 0, 0.0, w2, r1, r1 * n * a2, r2);
+  };
+  for (int64_t k = 0; k < d; ++k) {
+    const int64_t r1 = r[k], r2 = r[k + 1], a2 = ra[k + 1], n = x->n[k];
+    double* w2 = W2.p() + (keep ? woff[k] : 0);
+    left_products(k, w2);
+    // L_{k+1},be [c, e] = W2[(y,m), be, c]^T x[(y,m), e]
+    gemm_f64(c, true, false, r2, r2, r1 * n, 1.0, w2, r1 * n * a2, r1 * n, x->core + x->ps[k],
+             r1 * n, 0, 0.0, L.p() + off[k + 1], r2, r2 * r2, a2);
   }
   if (value) copy_f64(c, 1, L.p() + off[d], value);
-  // Scratch for the two local matvecs of the largest core.
-  int64_t t1 = 0, t2 = 0, nx = 0, nphi = 0, na = 0;
-  for (int64_t k = 0; k < d; ++k) {
-    MvDims dm{r[k], r[k], ra[k], x->n[k], x->n[k], r[k + 1], ra[k + 1], r[k + 1]};
-    t1 = std::max(t1, dm.t1_size());
-    t2 = std::max(t2, dm.t2_size());
-    nx = std::max(nx, dm.out_size());
-    nphi = std::max(nphi, std::max(r[k] * r[k] * ra[k], r[k + 1] * r[k + 1] * ra[k + 1]));
-    na = std::max(na, ra[k] * x->n[k] * x->n[k] * ra[k + 1]);
-  }
-  DBuf<double> T1(c, t1), T2(c, t2), G2(c, nx), Ls(c, nphi), Rs(c, nphi), At(c, na);
-  for (int64_t k = 0; k < d; ++k) {
+  for (int64_t k = d - 1; k >= 0; --k) {
     const int64_t r1 = r[k], r2 = r[k + 1], a1 = ra[k], a2 = ra[k + 1], n = x->n[k];
-    MvDims dm{r1, r1, a1, n, n, r2, a2, r2};
     const double* xk = x->core + x->ps[k];
-    const double* Ak = A->core + A->ps[k];
     double* gk = grad + x->ps[k];
-    // through the bra copy: (L_k x A_k x R_{k+1}) x_k
-    local_matvec_f64(c, dm, L.p() + off[k], Ak, R.p() + off[k + 1], xk, gk, T1.p(), T2.p());
-    // through the ket copy: bra and ket exchanged
-    permute4(c, Perm4{r1, r1, a1, 1, r1, 1, r1 * r1, 0}, L.p() + off[k], Ls.p());
-    permute4(c, Perm4{r2, a2, r2, 1, r2 * a2, r2, 1, 0}, R.p() + off[k + 1], Rs.p());
-    permute4(c, Perm4{a1, n, n, a2, 1, a1 * n, a1, a1 * n * n}, Ak, At.p());
-    local_matvec_f64(c, dm, Ls.p(), At.p(), Rs.p(), xk, G2.p(), T1.p(), T2.p());
-    axpby_f64(c, dm.out_size(), 1.0, G2.p(), 1.0, gk);
+    double* w2 = W2.p() + (keep ? woff[k] : 0);
+    // Z1[(y,m),(be,c)] = x R_{k+1}, Z2_c[y,(al,j)] = Z1_c[y,(m,be)] A[(al,j),(m,be)]^T
+    gemm_f64(c, false, false, r1 * n, a2 * r2, r2, 1.0, xk, r1 * n, 0, Rk, r2, 0, 0.0, Z1.p(),
+             r1 * n, 0, 1);
+    gemm_f64(c, false, true, r1, a1 * n, n * a2, 1.0, Z1.p(), r1, r1 * n * a2,
+             A->core + A->ps[k], a1 * n, 0, 0.0, Z2.p(), r1, r1 * a1 * n, r2);
+    // through the bra copy: G[a,(j,c)] = L_k[a,(y,al)] Z2[(y,al),(j,c)]
+    gemm_f64(c, false, false, r1, n * r2, r1 * a1, 1.0, L.p() + off[k], r1, 0, Z2.p(), r1 * a1, 0,
+             0.0, gk, r1, 0, 1);
+    // through the ket copy: G[(y,m), e] += W2[(y,m),(be,c)] R_{k+1}[e,(be,c)]^T
+    if (!keep) left_products(k, w2);
+    gemm_f64(c, false, true, r1 * n, r2, a2 * r2, 1.0, w2, r1 * n, 0, Rk, r2, 0, 1.0, gk, r1 * n,
+             0, 1);
+    if (k == 0) break;
+    // R_k[(y,al), a] = Z2[(y,al),(j,c)] x[a,(j,c)]^T
+    gemm_f64(c, false, true, r1 * a1, r1, n * r2, 1.0, Z2.p(), r1 * a1, 0, xk, r1, 0, 0.0, Rn,
+             r1 * a1, 0, 1);
+    std::swap(Rk, Rn);
   }
 }
 
