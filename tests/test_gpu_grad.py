@@ -257,3 +257,19 @@ def test_grad_xAx_without_kept_intermediates(ctx):
     for xk, gk in zip(xs, split(G, xs)):
         scale = np.linalg.norm(xk) * np.linalg.norm(gk)
         assert abs(np.vdot(xk, gk) - 2.0 * v) <= GRAD_TOL * scale
+
+
+@pytest.mark.parametrize("r,n,S", [
+    ([1, 33, 32, 1], [3, 2, 5], 129),      # one sample past a tile; narrow and wide outputs
+    ([1, 64, 65, 31, 1], [2, 4, 3, 2], 1025),  # gradient tiles of 512 and one more
+    ([1, 2, 1, 5, 1], [7, 1, 9, 4], 300),  # a mode of one value, ranks of one
+    ([1, 130, 66, 1], [1, 3, 1], 2000)])   # several tiles of outputs
+def test_grad_sampled_tiles(ctx, r, n, S):
+    rng = np.random.default_rng(S)
+    xs = rand_cores(rng, n, r)
+    idx = np.stack([rng.integers(0, nk, S) for nk in n], axis=1)
+    y = rng.standard_normal(S)
+    v, G = ttgpu.grad_sampled(to_tt(xs), idx, y, ctx=ctx)
+    vref, Gref = og.sampled(xs, idx, y)
+    assert abs(v - vref) <= VAL_TOL * abs(vref)
+    assert grad_rel(split(G, xs), Gref) <= GRAD_TOL

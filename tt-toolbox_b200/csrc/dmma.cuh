@@ -29,4 +29,76 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "d"(a), "d"(b));
 }
 
+constexpr int TILE_K = 16;  // k extent of the FP64 operand tiles
+
+// One operand tile of T rows (of C) by TILE_K in shared memory, filled by NT threads, in
+// the order its
+// global layout has: k contiguous (KC) as rows of TILE_K + 4, else k slices of
+// T + 4.  Either pitch is 4 mod 16 doubles, which puts the 16 doubles that a
+// half-warp reads for an mma fragment (4 of k by 4 rows) in different banks.
+template <int T, bool KC, int NT>
+struct TileS {
+  static constexpr int LD = KC ? TILE_K + 4 : T + 4;
+  static constexpr int SIZE = KC ? T * LD : TILE_K * LD;
+  static __device__ __forceinline__ double at(const double* s, int r, int k) {
+    return KC ? s[r * LD + k] : s[k * LD + r];
+  }
+  // Rows r0.. of R, k0.. of K of the operand g (element (r, k) at
+  // g[k + r ld] or g[r + k ld]); zeros outside.
+  static __device__ __forceinline__ void load(double* s, const double* __restrict__ g, int64_t ld,
+                                              int64_t r0, int64_t R, int64_t k0, int64_t K,
+                                              bool vec) {
+    const int tid = threadIdx.x;
+    if (KC) {
+      if (vec) {
+        const int k = (tid & 7) * 2, rb = tid >> 3;
+        const int64_t left = K - (k0 + k);
+        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+#pragma unroll
+        for (int i = 0; i < TILE_K * T / (2 * NT); ++i) {
+          const int r = rb + NT / (TILE_K / 2) * i;
+          const bool ok = bytes && r0 + r < R;
+          cp_async16(s + r * LD + k, ok ? g + (k0 + k) + (r0 + r) * ld : g, ok ? bytes : 0);
+        }
+      } else {
+        const int k = tid & 15, rb = tid >> 4;
+        const bool kok = k0 + k < K;
+#pragma unroll
+        for (int i = 0; i < TILE_K * T / NT; ++i) {
+          const int r = rb + NT / TILE_K * i;
+          const bool ok = kok && r0 + r < R;
+          cp_async8(s + r * LD + k, ok ? g + (k0 + k) + (r0 + r) * ld : g, ok);
+        }
+      }
+    } else {
+      if (vec) {
+        const int r = (tid % (T / 2)) * 2, kb = tid / (T / 2);
+        const int64_t left = R - (r0 + r);
+        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+#pragma unroll
+        for (int i = 0; i < TILE_K * T / (2 * NT); ++i) {
+          const int k = kb + 2 * NT / T * i;
+          const bool ok = bytes && k0 + k < K;
+          cp_async16(s + k * LD + r, ok ? g + (r0 + r) + (k0 + k) * ld : g, ok ? bytes : 0);
+        }
+      } else {
+        const int r = tid % T, kb = tid / T;
+        const bool rok = r0 + r < R;
+#pragma unroll
+        for (int i = 0; i < TILE_K * T / NT; ++i) {
+          const int k = kb + NT / T * i;
+          const bool ok = rok && k0 + k < K;
+          cp_async8(s + k * LD + r, ok ? g + (r0 + r) + (k0 + k) * ld : g, ok);
+        }
+      }
+    }
+  }
+};
+
+// An operand whose columns (or rows, k contiguous) all start on 16 bytes.
+inline bool vec16(const double* p, int64_t ld, int64_t stride = 0, int64_t batch = 1) {
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 2 == 0 &&
+         (batch == 1 || stride % 2 == 0);
+}
+
 }  // namespace ttg

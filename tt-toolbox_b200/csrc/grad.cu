@@ -37,13 +37,13 @@ namespace ttg {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, PADS = 8;
-constexpr int PT = 64;           // samples per propagation tile
+constexpr int PT = 128;          // samples per propagation tile
+constexpr int PROP_THREADS = 256, GRAD_THREADS = 128, GRAD_STAGES = 3;
+// Bytes of intermediates the left sweep of <x, A x> keeps for the right one.
+constexpr int64_t KEEP_MAX = int64_t(1) << 30;
 constexpr int GT = 512;          // samples per gradient (split-K) tile
 constexpr int SORT_CHUNK = 1024; // samples per sorting warp
 constexpr int64_t MAX_BUCKETS = 8192;
-// Bytes of intermediates the left sweep of <x, A x> keeps for the right one.
-constexpr int64_t KEEP_MAX = int64_t(1) << 30;
 
 int blocks_for(int64_t n, int threads = 256) {
   int64_t b = (n + threads - 1) / threads;
@@ -171,7 +171,12 @@ __device__ __forceinline__ int find_bucket(const int* __restrict__ start, int n,
 //   forward  (BWD=false): vout[s, c] = sum_a vin[s, a] * x_k[a, j, c]
 //   backward (BWD=true):  vout[s, a] = sum_c x_k[a, j, c] * vin[s, c]
 // for every sample s of bucket j (i_k(s) = j).  Sample vectors are rows:
-// v[s * ld + a].  CTA = 64 samples x 64 outputs, K in steps of 16.
+// v[s * ld + a].  CTA = 128 samples x BN outputs, eight warps of 32 x BN / 2,
+// K in steps of 16 through a ring of three tiles (the pitches and copies of
+// TileS).  Bound by the FP64 tensor rate next to reading and writing one
+// vector per sample: 1M samples, 64 x 64 slices 279 us forward, 280 backward
+// (29 TFLOP/s with 3.7 TB/s), against 493 and 426 with 64 samples a CTA, two
+// stages, 8-byte copies and conflicting pitches.
 // ---------------------------------------------------------------------------
 struct PropP {
   const double* vin;
@@ -183,13 +188,23 @@ struct PropP {
   int64_t K, N;
   const int* perm;
   const int* meta;  // bucket table (k_bucket_base layout)
+  int vecA, vecB, vecC;  // 16-byte accesses of vin, of the slices and of vout
 };
 
-template <bool BWD>
-__global__ void __launch_bounds__(128) k_prop(PropP p) {
-  __shared__ double As[2][BK][BM + PADS];
-  __shared__ double Bs[2][BK][BN + PADS];
-  __shared__ int64_t rowoff[BM];
+template <int BN, bool BWD>
+constexpr size_t prop_smem() {
+  return sizeof(double) * GRAD_STAGES *
+             (TileS<PT, true, PROP_THREADS>::SIZE + TileS<BN, !BWD, PROP_THREADS>::SIZE) +
+         sizeof(int64_t) * PT;
+}
+
+template <int BN, bool BWD>
+__global__ void __launch_bounds__(PROP_THREADS) k_prop(PropP p) {
+  using SA = TileS<PT, true, PROP_THREADS>;
+  using SB = TileS<BN, !BWD, PROP_THREADS>;
+  constexpr int NI = BN / 16;
+  extern __shared__ __align__(16) double psm[];
+  int64_t* rowoff = reinterpret_cast<int64_t*>(psm + GRAD_STAGES * (SA::SIZE + SB::SIZE));
   const int nb = int(p.n);
   const int* bstart = p.meta;
   const int* tstart = p.meta + nb + 1;
@@ -199,95 +214,90 @@ __global__ void __launch_bounds__(128) k_prop(PropP p) {
   const int64_t s0 = int64_t(bstart[j]) + int64_t(t - tstart[j]) * PT;
   const int64_t cnt = min(int64_t(PT), int64_t(bstart[j + 1]) - s0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < BM) rowoff[tid] = tid < cnt ? int64_t(p.perm[s0 + tid]) : -1;
+  if (tid < PT) rowoff[tid] = tid < cnt ? int64_t(p.perm[s0 + tid]) : -1;
   __syncthreads();
   const double* __restrict__ W = p.core + p.r1 * j;
   const int64_t ldw = p.r1 * p.n;
   const int64_t n0 = int64_t(blockIdx.y) * BN;
   const int64_t K = p.K, N = p.N;
+  const int ktiles = int((K + TILE_K - 1) / TILE_K);
 
-  auto load_tile = [&](int64_t k0, int buf) {
-    {  // A(m, k) = vin[rowoff[m] * ldi + k]   (k contiguous)
-      const int k = tid & 15, mb = tid >> 4;
-      const int64_t gk = k0 + k;
+  auto load_tile = [&](int kt) {
+    if (kt < ktiles) {
+      double* sa = psm + (kt % GRAD_STAGES) * (SA::SIZE + SB::SIZE);
+      const int64_t k0 = int64_t(kt) * TILE_K;
+      // A(m, k) = vin[rowoff[m] * ldi + k]   (k contiguous)
+      if (p.vecA) {
+        const int k = (tid & 7) * 2, mb = tid >> 3;
+        const int64_t left = K - (k0 + k);
+        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int m = mb + 8 * i;
-        const int64_t ro = rowoff[m];
-        const bool ok = ro >= 0 && gk < K;
-        cp_async8(&As[buf][k][m], ok ? p.vin + ro * p.ldi + gk : p.vin, ok);
-      }
-    }
-    if (!BWD) {  // B(k=a, n=c) = W[a + c*ldw]   (k contiguous)
-      const int k = tid & 15, nb2 = tid >> 4;
-      const int64_t gk = k0 + k;
+        for (int i = 0; i < PT * 8 / PROP_THREADS; ++i) {
+          const int m = mb + PROP_THREADS / 8 * i;
+          const int64_t ro = rowoff[m];
+          const bool ok = bytes && ro >= 0;
+          cp_async16(sa + m * SA::LD + k, ok ? p.vin + ro * p.ldi + k0 + k : p.vin,
+                     ok ? bytes : 0);
+        }
+      } else {
+        const int k = tid & 15, mb = tid >> 4;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int nn = nb2 + 8 * i;
-        const int64_t gn = n0 + nn;
-        const bool ok = gn < N && gk < K;
-        cp_async8(&Bs[buf][k][nn], ok ? W + gk + gn * ldw : W, ok);
+        for (int i = 0; i < PT * 16 / PROP_THREADS; ++i) {
+          const int m = mb + PROP_THREADS / 16 * i;
+          const int64_t ro = rowoff[m];
+          const bool ok = ro >= 0 && k0 + k < K;
+          cp_async8(sa + m * SA::LD + k, ok ? p.vin + ro * p.ldi + k0 + k : p.vin, ok);
+        }
       }
-    } else {  // B(k=c, n=a) = W[a + c*ldw]   (n contiguous)
-      const int nn = tid & 63, kb = tid >> 6;
-      const int64_t gn = n0 + nn;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int k = kb + 2 * i;
-        const int64_t gk = k0 + k;
-        const bool ok = gn < N && gk < K;
-        cp_async8(&Bs[buf][k][nn], ok ? W + gn + gk * ldw : W, ok);
-      }
+      // forward B(k=a, n=c) = W[a + c*ldw], backward B(k=c, n=a) = W[a + c*ldw]
+      SB::load(sa + SA::SIZE, W, ldw, n0, N, k0, K, p.vecB);
     }
     cp_async_commit();
   };
 
-  double acc[4][4][2];
+  double acc[4][NI][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) acc[i][jj][0] = acc[i][jj][1] = 0.0;
+    for (int jj = 0; jj < NI; ++jj) acc[i][jj][0] = acc[i][jj][1] = 0.0;
 
   const int g = lane >> 2, tq = lane & 3;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-  const int64_t ktiles = (K + BK - 1) / BK;
-  if (ktiles > 0) load_tile(0, 0);
-  for (int64_t kt = 0; kt < ktiles; ++kt) {
-    const int buf = int(kt & 1);
-    if (kt + 1 < ktiles) {
-      load_tile((kt + 1) * BK, buf ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+  const int wm = (warp & 3) * 32, wn = (warp >> 2) * (BN / 2);
+#pragma unroll
+  for (int s = 0; s < GRAD_STAGES - 1; ++s) load_tile(s);
+  for (int kt = 0; kt < ktiles; ++kt) {
+    cp_async_wait<GRAD_STAGES - 2>();
     __syncthreads();
+    load_tile(kt + GRAD_STAGES - 1);
+    const double* As = psm + (kt % GRAD_STAGES) * (SA::SIZE + SB::SIZE);
+    const double* Bs = As + SA::SIZE;
 #pragma unroll
-    for (int kk = 0; kk < BK / 4; ++kk) {
-      double a[4], b[4];
+    for (int kk = 0; kk < TILE_K / 4; ++kk) {
+      double a[4], b[NI];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk * 4 + tq][wm + i * 8 + g];
+      for (int i = 0; i < 4; ++i) a[i] = SA::at(As, wm + i * 8 + g, kk * 4 + tq);
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) b[jj] = Bs[buf][kk * 4 + tq][wn + jj * 8 + g];
+      for (int jj = 0; jj < NI; ++jj) b[jj] = SB::at(Bs, wn + jj * 8 + g, kk * 4 + tq);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) dmma(acc[i][jj][0], acc[i][jj][1], a[i], b[jj]);
+        for (int jj = 0; jj < NI; ++jj) dmma(acc[i][jj][0], acc[i][jj][1], a[i], b[jj]);
     }
-    __syncthreads();
   }
 
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int m = wm + i * 8 + g;
-    const int64_t ro = rowoff[m];
+    const int64_t ro = rowoff[wm + i * 8 + g];
     if (ro < 0) continue;
     double* dst = p.vout + ro * p.ldo;
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int64_t col = n0 + wn + jj * 8 + 2 * tq + e;
-        if (col < N) dst[col] = acc[i][jj][e];
+    for (int jj = 0; jj < NI; ++jj) {
+      const int64_t col = n0 + wn + jj * 8 + 2 * tq;
+      if (p.vecC && col + 1 < N) {
+        *reinterpret_cast<double2*>(dst + col) = make_double2(acc[i][jj][0], acc[i][jj][1]);
+      } else {
+        if (col < N) dst[col] = acc[i][jj][0];
+        if (col + 1 < N) dst[col + 1] = acc[i][jj][1];
       }
     }
   }
@@ -296,6 +306,7 @@ __global__ void __launch_bounds__(128) k_prop(PropP p) {
 // ---------------------------------------------------------------------------
 // Gradient partials: part[t][a + r1*c] = sum over the <= 512 samples s of
 // gradient tile t of L[s, a] * P[s, c]   (M = r1, N = r2, K = samples)
+// The same ring; 1M samples, 64 x 64: 283 us (315 before).
 // ---------------------------------------------------------------------------
 struct GradP {
   const double* L;
@@ -306,12 +317,53 @@ struct GradP {
   int64_t r1, n, r2;
   const int* perm;
   const int* meta;
+  int vecA, vecB;
 };
 
-__global__ void __launch_bounds__(128) k_grad_tiles(GradP p) {
-  __shared__ double As[2][BK][BM + PADS];
-  __shared__ double Bs[2][BK][BN + PADS];
-  __shared__ int64_t rowoff[GT];
+template <int BM, int BN>
+constexpr size_t grad_smem() {
+  return sizeof(double) * GRAD_STAGES *
+             (TileS<BM, false, GRAD_THREADS>::SIZE + TileS<BN, false, GRAD_THREADS>::SIZE) +
+         sizeof(int64_t) * GT;
+}
+
+// Columns x0.. of the gathered rows k0.. of v into an operand tile (zeros
+// outside): s[k * LD + x] = v[rowoff[k0 + k] * ld + x0 + x].
+template <int T>
+__device__ __forceinline__ void load_gathered(double* s, const double* __restrict__ v, int64_t ld,
+                                              const int64_t* rowoff, int64_t x0, int64_t X,
+                                              int k0, int K, bool vec) {
+  constexpr int LD = TileS<T, false, GRAD_THREADS>::LD;
+  const int tid = threadIdx.x;
+  if (vec) {
+    const int x = (tid % (T / 2)) * 2, kb = tid / (T / 2);
+    const int64_t left = X - (x0 + x);
+    const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+#pragma unroll
+    for (int i = 0; i < TILE_K * T / (2 * GRAD_THREADS); ++i) {
+      const int k = kb + 2 * GRAD_THREADS / T * i;
+      const bool ok = bytes && k0 + k < K;
+      cp_async16(s + k * LD + x, ok ? v + rowoff[k0 + k] * ld + x0 + x : v, ok ? bytes : 0);
+    }
+  } else {
+    const int x = tid % T, kb = tid / T;
+    const bool xok = x0 + x < X;
+#pragma unroll
+    for (int i = 0; i < TILE_K * T / GRAD_THREADS; ++i) {
+      const int k = kb + GRAD_THREADS / T * i;
+      const bool ok = xok && k0 + k < K;
+      cp_async8(s + k * LD + x, ok ? v + rowoff[k0 + k] * ld + x0 + x : v, ok);
+    }
+  }
+}
+
+template <int BM, int BN>
+__global__ void __launch_bounds__(GRAD_THREADS) k_grad_tiles(GradP p) {
+  using SA = TileS<BM, false, GRAD_THREADS>;
+  using SB = TileS<BN, false, GRAD_THREADS>;
+  constexpr int MI = BM / 16, NI = BN / 16;
+  extern __shared__ __align__(16) double gtsm[];
+  int64_t* rowoff = reinterpret_cast<int64_t*>(gtsm + GRAD_STAGES * (SA::SIZE + SB::SIZE));
   const int nb = int(p.n);
   const int* bstart = p.meta;
   const int* gstart = p.meta + 2 * nb + 2;
@@ -319,70 +371,60 @@ __global__ void __launch_bounds__(128) k_grad_tiles(GradP p) {
   if (t >= gstart[nb]) return;
   const int j = find_bucket(gstart, nb, t);
   const int64_t s0 = int64_t(bstart[j]) + int64_t(t - gstart[j]) * GT;
-  const int64_t cnt = min(int64_t(GT), int64_t(bstart[j + 1]) - s0);
+  const int cnt = int(min(int64_t(GT), int64_t(bstart[j + 1]) - s0));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < GT; i += 128) rowoff[i] = i < cnt ? int64_t(p.perm[s0 + i]) : -1;
+  for (int i = tid; i < cnt; i += GRAD_THREADS) rowoff[i] = int64_t(p.perm[s0 + i]);
   __syncthreads();
   const int64_t m0 = int64_t(blockIdx.y) * BM, n0 = int64_t(blockIdx.z) * BN;
-  const int64_t M = p.r1, N = p.r2, K = cnt;
+  const int64_t M = p.r1, N = p.r2;
+  const int ktiles = (cnt + TILE_K - 1) / TILE_K;
 
-  auto load_tile = [&](int64_t k0, int buf) {
-    const int x = tid & 63, kb = tid >> 6;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int k = kb + 2 * i;
-      const int64_t gk = k0 + k;
-      const int64_t ro = gk < K ? rowoff[gk] : -1;
-      const int64_t gm = m0 + x, gn = n0 + x;
-      const bool oka = ro >= 0 && gm < M;
-      const bool okb = ro >= 0 && gn < N;
-      cp_async8(&As[buf][k][x], oka ? p.L + ro * p.ldl + gm : p.L, oka);
-      cp_async8(&Bs[buf][k][x], okb ? p.P + ro * p.ldp + gn : p.P, okb);
+  auto load_tile = [&](int kt) {
+    if (kt < ktiles) {
+      double* s = gtsm + (kt % GRAD_STAGES) * (SA::SIZE + SB::SIZE);
+      load_gathered<BM>(s, p.L, p.ldl, rowoff, m0, M, kt * TILE_K, cnt, p.vecA);
+      load_gathered<BN>(s + SA::SIZE, p.P, p.ldp, rowoff, n0, N, kt * TILE_K, cnt, p.vecB);
     }
     cp_async_commit();
   };
 
-  double acc[4][4][2];
+  double acc[MI][NI][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) acc[i][jj][0] = acc[i][jj][1] = 0.0;
+    for (int jj = 0; jj < NI; ++jj) acc[i][jj][0] = acc[i][jj][1] = 0.0;
 
   const int g = lane >> 2, tq = lane & 3;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-  const int64_t ktiles = (K + BK - 1) / BK;
-  if (ktiles > 0) load_tile(0, 0);
-  for (int64_t kt = 0; kt < ktiles; ++kt) {
-    const int buf = int(kt & 1);
-    if (kt + 1 < ktiles) {
-      load_tile((kt + 1) * BK, buf ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+  const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
+#pragma unroll
+  for (int s = 0; s < GRAD_STAGES - 1; ++s) load_tile(s);
+  for (int kt = 0; kt < ktiles; ++kt) {
+    cp_async_wait<GRAD_STAGES - 2>();
     __syncthreads();
+    load_tile(kt + GRAD_STAGES - 1);
+    const double* As = gtsm + (kt % GRAD_STAGES) * (SA::SIZE + SB::SIZE);
+    const double* Bs = As + SA::SIZE;
 #pragma unroll
-    for (int kk = 0; kk < BK / 4; ++kk) {
-      double a[4], b[4];
+    for (int kk = 0; kk < TILE_K / 4; ++kk) {
+      double a[MI], b[NI];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk * 4 + tq][wm + i * 8 + g];
+      for (int i = 0; i < MI; ++i) a[i] = SA::at(As, wm + i * 8 + g, kk * 4 + tq);
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) b[jj] = Bs[buf][kk * 4 + tq][wn + jj * 8 + g];
+      for (int jj = 0; jj < NI; ++jj) b[jj] = SB::at(Bs, wn + jj * 8 + g, kk * 4 + tq);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) dmma(acc[i][jj][0], acc[i][jj][1], a[i], b[jj]);
+        for (int jj = 0; jj < NI; ++jj) dmma(acc[i][jj][0], acc[i][jj][1], a[i], b[jj]);
     }
-    __syncthreads();
   }
 
   double* dst = p.part + int64_t(t) * (p.r1 * p.r2);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < MI; ++i) {
     const int64_t row = m0 + wm + i * 8 + g;
     if (row >= M) continue;
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
+    for (int jj = 0; jj < NI; ++jj) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int64_t col = n0 + wn + jj * 8 + 2 * tq + e;
@@ -420,6 +462,38 @@ __global__ void k_sample_residual(int64_t S, const double* __restrict__ v,
     e[s] = r;
     rho[s] = 2.0 * r;
   }
+}
+
+template <int BN, bool BWD>
+void prop_launch(Context* c, int64_t tiles, const PropP& p) {
+  constexpr size_t smem = prop_smem<BN, BWD>();
+  ensure_smem_attr(reinterpret_cast<const void*>(k_prop<BN, BWD>), c->device, int(smem));
+  dim3 grid{unsigned(tiles), unsigned((p.N + BN - 1) / BN), 1};
+  k_prop<BN, BWD><<<grid, PROP_THREADS, smem, c->stream>>>(p);
+  c->launches += 1;
+  TTG_CHECK_LAUNCH();
+}
+
+// Outputs up to 32 take the narrow tile: the wide one would multiply padding.
+template <bool BWD>
+void propagate(Context* c, int64_t tiles, PropP p) {
+  p.vecA = vec16(p.vin, p.ldi);
+  p.vecB = vec16(p.core, p.r1);  // slices start r1 apart
+  p.vecC = vec16(p.vout, p.ldo);
+  if (p.N <= 32)
+    prop_launch<32, BWD>(c, tiles, p);
+  else
+    prop_launch<64, BWD>(c, tiles, p);
+}
+
+template <int BM, int BN>
+void grad_launch(Context* c, int64_t tiles, const GradP& p) {
+  constexpr size_t smem = grad_smem<BM, BN>();
+  ensure_smem_attr(reinterpret_cast<const void*>(k_grad_tiles<BM, BN>), c->device, int(smem));
+  dim3 grid{unsigned(tiles), unsigned((p.r1 + BM - 1) / BM), unsigned((p.r2 + BN - 1) / BN)};
+  k_grad_tiles<BM, BN><<<grid, GRAD_THREADS, smem, c->stream>>>(p);
+  c->launches += 1;
+  TTG_CHECK_LAUNCH();
 }
 
 void check_tt_vector(const ttg_tt_s* x, const char* what) {
@@ -645,12 +719,10 @@ void grad_sampled(Context* c, const ttg_tt_s* x, int64_t S, const int* idx, cons
     const int n = int(x->n[k]);
     const int ntiles = hmeta[moff[k] + 2 * n + 1];
     if (ntiles == 0) continue;
-    PropP p{Lv.p() + loff[k], r[k], Lv.p() + loff[k + 1], r[k + 1], x->core + x->ps[k],
-            r[k], x->n[k], r[k + 1], r[k], r[k + 1], perm.p() + k * S, meta.p() + moff[k]};
-    dim3 grid{unsigned(ntiles), unsigned((r[k + 1] + BN - 1) / BN), 1};
-    k_prop<false><<<grid, 128, 0, c->stream>>>(p);
-    c->launches += 1;
-    TTG_CHECK_LAUNCH();
+    propagate<false>(c, ntiles,
+                     PropP{Lv.p() + loff[k], r[k], Lv.p() + loff[k + 1], r[k + 1],
+                           x->core + x->ps[k], r[k], x->n[k], r[k + 1], r[k], r[k + 1],
+                           perm.p() + k * S, meta.p() + moff[k], 0, 0, 0});
   }
   double* rho = rho0.p();
   double* rho_next = rho1.p();
@@ -663,21 +735,25 @@ void grad_sampled(Context* c, const ttg_tt_s* x, int64_t S, const int* idx, cons
     const int ngt = hmeta[moff[k] + 3 * n + 2];
     const int64_t r1 = r[k], r2 = r[k + 1];
     GradP gp{Lv.p() + loff[k], r1, rho, r2, part.p(), r1, x->n[k], r2, perm.p() + k * S,
-             meta.p() + moff[k]};
-    dim3 gg{unsigned(ngt), unsigned((r1 + BM - 1) / BM), unsigned((r2 + BN - 1) / BN)};
-    k_grad_tiles<<<gg, 128, 0, c->stream>>>(gp);
+             meta.p() + moff[k], vec16(Lv.p() + loff[k], r1), vec16(rho, r2)};
+    // narrow tiles for ranks up to 32
+    if (r1 <= 32 && r2 <= 32)
+      grad_launch<32, 32>(c, ngt, gp);
+    else if (r1 <= 32)
+      grad_launch<32, 64>(c, ngt, gp);
+    else if (r2 <= 32)
+      grad_launch<64, 32>(c, ngt, gp);
+    else
+      grad_launch<64, 64>(c, ngt, gp);
     k_grad_reduce<<<blocks_for(r1 * r2 * x->n[k]), 256, 0, c->stream>>>(
         r1, x->n[k], r2, part.p(), meta.p() + moff[k], grad + x->ps[k]);
-    c->launches += 2;
+    c->launches += 1;
     TTG_CHECK_LAUNCH();
     if (k == 0) break;
     const int ntiles = hmeta[moff[k] + 2 * n + 1];
-    PropP p{rho, r2, rho_next, r1, x->core + x->ps[k], r1, x->n[k], r2, r2, r1,
-            perm.p() + k * S, meta.p() + moff[k]};
-    dim3 grid{unsigned(ntiles), unsigned((r1 + BN - 1) / BN), 1};
-    k_prop<true><<<grid, 128, 0, c->stream>>>(p);
-    c->launches += 1;
-    TTG_CHECK_LAUNCH();
+    propagate<true>(c, ntiles,
+                    PropP{rho, r2, rho_next, r1, x->core + x->ps[k], r1, x->n[k], r2, r2, r1,
+                          perm.p() + k * S, meta.p() + moff[k], 0, 0, 0});
     std::swap(rho, rho_next);
   }
 }

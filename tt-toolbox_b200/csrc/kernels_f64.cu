@@ -17,7 +17,7 @@ namespace ttg {
 
 namespace {
 
-constexpr int BK = 16, GEMM_STAGES = 3, GEMM_THREADS = 128;
+constexpr int GEMM_STAGES = 3, GEMM_THREADS = 128;
 // Split-K partial values one CTA may sum in the GEMM kernel itself.
 constexpr int64_t SPLITK_INKERNEL_MAX = 8192;
 
@@ -43,73 +43,10 @@ struct GemmP {
   unsigned* cnt;
 };
 
-// One operand tile of T rows (of C) by BK in shared memory, in the order its
-// global layout has: k contiguous (KC) as rows of BK + 4, else k slices of
-// T + 4.  Either pitch is 4 mod 16 doubles, which puts the 16 doubles that a
-// half-warp reads for an mma fragment (4 of k by 4 rows) in different banks.
-template <int T, bool KC>
-struct TileS {
-  static constexpr int NT = GEMM_THREADS;
-  static constexpr int LD = KC ? BK + 4 : T + 4;
-  static constexpr int SIZE = KC ? T * LD : BK * LD;
-  static __device__ __forceinline__ double at(const double* s, int r, int k) {
-    return KC ? s[r * LD + k] : s[k * LD + r];
-  }
-  // Rows r0.. of R, k0.. of K of the operand g (element (r, k) at
-  // g[k + r ld] or g[r + k ld]); zeros outside.
-  static __device__ __forceinline__ void load(double* s, const double* __restrict__ g, int64_t ld,
-                                              int64_t r0, int64_t R, int64_t k0, int64_t K,
-                                              bool vec) {
-    const int tid = threadIdx.x;
-    if (KC) {
-      if (vec) {
-        const int k = (tid & 7) * 2, rb = tid >> 3;
-        const int64_t left = K - (k0 + k);
-        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
-#pragma unroll
-        for (int i = 0; i < BK * T / (2 * NT); ++i) {
-          const int r = rb + NT / (BK / 2) * i;
-          const bool ok = bytes && r0 + r < R;
-          cp_async16(s + r * LD + k, ok ? g + (k0 + k) + (r0 + r) * ld : g, ok ? bytes : 0);
-        }
-      } else {
-        const int k = tid & 15, rb = tid >> 4;
-        const bool kok = k0 + k < K;
-#pragma unroll
-        for (int i = 0; i < BK * T / NT; ++i) {
-          const int r = rb + NT / BK * i;
-          const bool ok = kok && r0 + r < R;
-          cp_async8(s + r * LD + k, ok ? g + (k0 + k) + (r0 + r) * ld : g, ok);
-        }
-      }
-    } else {
-      if (vec) {
-        const int r = (tid % (T / 2)) * 2, kb = tid / (T / 2);
-        const int64_t left = R - (r0 + r);
-        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
-#pragma unroll
-        for (int i = 0; i < BK * T / (2 * NT); ++i) {
-          const int k = kb + 2 * NT / T * i;
-          const bool ok = bytes && k0 + k < K;
-          cp_async16(s + k * LD + r, ok ? g + (r0 + r) + (k0 + k) * ld : g, ok ? bytes : 0);
-        }
-      } else {
-        const int r = tid % T, kb = tid / T;
-        const bool rok = r0 + r < R;
-#pragma unroll
-        for (int i = 0; i < BK * T / NT; ++i) {
-          const int k = kb + NT / T * i;
-          const bool ok = rok && k0 + k < K;
-          cp_async8(s + k * LD + r, ok ? g + (r0 + r) + (k0 + k) * ld : g, ok);
-        }
-      }
-    }
-  }
-};
-
 template <int BM, int BN, bool TA, bool TB>
 constexpr size_t gemm_smem() {
-  return sizeof(double) * GEMM_STAGES * (TileS<BM, TA>::SIZE + TileS<BN, !TB>::SIZE);
+  return sizeof(double) * GEMM_STAGES *
+         (TileS<BM, TA, GEMM_THREADS>::SIZE + TileS<BN, !TB, GEMM_THREADS>::SIZE);
 }
 
 // Bound by the FP64 tensor rate where the tiles fill the device, by the chain
@@ -125,8 +62,8 @@ TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
   pdl_begin();
   extern __shared__ __align__(16) double gsm[];
   constexpr int NT = GEMM_THREADS;
-  using SA = TileS<BM, TA>;
-  using SB = TileS<BN, !TB>;
+  using SA = TileS<BM, TA, NT>;
+  using SB = TileS<BN, !TB, NT>;
   constexpr int MI = BM / 16, NI = BN / 16;  // 8 x 8 fragments of a warp
   if (p.skip && *p.skip) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -148,12 +85,12 @@ TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
 
   const int g = lane >> 2, t = lane & 3;
   const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
-  const int ktiles = int((K + BK - 1) / BK);
+  const int ktiles = int((K + TILE_K - 1) / TILE_K);
   auto load_tile = [&](int kt) {
     if (kt < ktiles) {
       double* s = gsm + (kt % GEMM_STAGES) * (SA::SIZE + SB::SIZE);
-      SA::load(s, A, p.lda, m0, M, int64_t(kt) * BK, K, p.vecA);
-      SB::load(s + SA::SIZE, B, p.ldb, n0, N, int64_t(kt) * BK, K, p.vecB);
+      SA::load(s, A, p.lda, m0, M, int64_t(kt) * TILE_K, K, p.vecA);
+      SB::load(s + SA::SIZE, B, p.ldb, n0, N, int64_t(kt) * TILE_K, K, p.vecB);
     }
     cp_async_commit();
   };
@@ -175,8 +112,8 @@ TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
     };
     frag(0);
 #pragma unroll
-    for (int kk = 0; kk < BK / 4; ++kk) {
-      if (kk + 1 < BK / 4) frag(kk + 1);
+    for (int kk = 0; kk < TILE_K / 4; ++kk) {
+      if (kk + 1 < TILE_K / 4) frag(kk + 1);
 #pragma unroll
       for (int i = 0; i < MI; ++i)
 #pragma unroll
@@ -574,12 +511,6 @@ int grid_for(Context* c, int64_t n, int threads = 256) {
   return int(b);
 }
 
-// An operand whose columns (or rows, k contiguous) all start on 16 bytes.
-bool vec16(const double* p, int64_t ld, int64_t stride, int64_t batch) {
-  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 2 == 0 &&
-         (batch == 1 || stride % 2 == 0);
-}
-
 template <int BM, int BN, bool TA, bool TB>
 void gemm_launch(Context* c, dim3 grid, const GemmP& p) {
   constexpr size_t smem = gemm_smem<BM, BN, TA, TB>();
@@ -621,7 +552,7 @@ struct GemmPlan {
 // split-K to two 64 x 64 CTAs per SM: 61 x 64 x 67 54 / 83 us, 128 x 64 x 128
 // 136 / 216, 512 x 64 x 512 4.4 / 8.0 ms.
 GemmPlan plan_gemm(Context* c, int64_t M, int64_t N, int64_t K, int64_t batch, bool may_split) {
-  const int64_t ktiles = (K + BK - 1) / BK;
+  const int64_t ktiles = (K + TILE_K - 1) / TILE_K;
   GemmPlan best{};
   double best_t = 0.0;
   for (const GemmTile& t : GEMM_TILES) {
@@ -644,7 +575,7 @@ GemmPlan plan_gemm(Context* c, int64_t M, int64_t N, int64_t K, int64_t batch, b
                (ns * te <= SPLITK_INKERNEL_MAX ? 2500.0 : 4500.0);
       }
       if (best_t == 0.0 || est < best_t) {
-        best = GemmPlan{t, gx, gy, ns, kt * BK};
+        best = GemmPlan{t, gx, gy, ns, kt * TILE_K};
         best_t = est;
       }
     }
