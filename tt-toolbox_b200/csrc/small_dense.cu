@@ -19,6 +19,7 @@
 
 #include <cooperative_groups.h>
 
+#include "dmma.cuh"
 #include "group.cuh"
 #include "small_dense.h"
 
@@ -366,197 +367,358 @@ TTG_BODY(k_jacobi_coop)(TTG_BLOCK, int n, const double* __restrict__ Ain,
 TTG_COOP_KERNEL(k_jacobi_coop, JC_THREADS);
 
 // ---------------------------------------------------------------------------
-// Cluster Jacobi SVD for 113 < n <= 256 (the 256 x 256 R factors of the
-// rounding sweeps): one thread-block cluster of JK_CS CTAs holds A and V in
-// distributed shared memory, JK cols = ceil(n / JK_CS) columns per CTA, one
-// warp per column.  Columns never move: in each round of the round-robin
-// tournament the owners of a pair (P, Q) both read the two columns (one
-// local, one remote over DSMEM), compute the same rotation from the same
-// values in the same order, and each writes its own rotated column into the
-// other of two buffers.  One hardware cluster barrier per round replaces the
-// software grid barrier of k_jacobi_coop (the SVD is bound by the latency of
-// its ~2300 rounds, not by arithmetic): 0.27 us per cluster barrier against
-// several us per grid barrier, while reading the partner's two 256-entry
-// columns over DSMEM costs about 2.4 us per round (measured: per-thread
-// ld.shared::cluster; bulk shared::cta -> shared::cluster pushes of the
-// column blocks completing on the partner's mbarrier measured slower still,
-// and so did a row-partitioned form that sends only the partial inner
-// products and the rotations across the cluster, with two barriers per
-// round: 235 against 195 ms for the SVD sweep of rounding a d = 20, n = 16
-// sum of four rank-64 TTs).  Same rotation formula and stopping
-// rule as k_jacobi_svd; the rotated A and V go to global memory for
-// k_jacobi_finish.  All CTAs of a cluster are co-resident by construction,
-// and every CTA takes the same number of rounds (the stopping decision is
-// read by all from the same published values): the barriers cannot wait
-// for a CTA that is not running.
+// Block Jacobi SVD in one thread-block cluster, for n <= JK_MAX_N columns (the
+// R factors of the rounding sweeps and of AMEn's truncations).  The columns,
+// each A over V, fall into blocks of 8; a round of a round-robin tournament
+// on the blocks gives every CTA one block pair.  A round takes
+//   the Gram matrix of the pair's 16 columns of A (mma.m8n8k4, K split over
+//   the warps),
+//   the 8 x 8 cross pairs of the two blocks rotated on that matrix, one warp,
+//   eight disjoint pairs at a time (in a sweep's first round all 120 pairs),
+//   with the rotations collected in a 16 x 16 orthogonal J,
+//   and [A; V] J for the 16 columns (mma), skipped when nothing rotated.
+// The columns live in L2 (1 MB at n = 256) and are read at the start of a
+// round and written at its end, with one hardware cluster barrier between:
+// distributed shared memory moves 14 bytes per cycle and SM here, L2 four
+// times that.  V arrives while the Gram matrix is rotated.
+// A rotation on the Gram matrix is that of one-sided Jacobi on the columns
+// (al = |a_p|^2, be = |a_q|^2, ga = <a_p, a_q>), whose entries round relative to
+// the columns' norms; each round forms the matrix anew from the columns.  A
+// sweep that rotates no pair ends the iteration: k_jacobi_svd's stopping rule.
+// Bound by the chain of rounds, 7.5 us each at n = 256: the eight rotation steps
+// on one warp 3 us, [A; V] J 1.8, the Gram matrix 1.1, loads and the barrier
+// 1.3.  Whole SVD of a triangular factor, against one column pair per warp and a
+// cluster barrier per column round: 2.75 ms for 9.8 at n = 256, 0.95 for 2.1 at
+// 128, 0.43 for 0.69 at 64, with the same errors against 64 bits.
+// All CTAs of a cluster are co-resident by construction, and every CTA takes
+// the same number of rounds (the stopping decision is read by all from the
+// same published values): the barriers cannot wait for a CTA that is not
+// running.
 // ---------------------------------------------------------------------------
 
-constexpr int JK_CS = 16;
-constexpr int JK_MAX_N = 256;
-constexpr int JK_MAX_COLS = JK_MAX_N / JK_CS;
-constexpr int JK_THREADS = 32 * JK_MAX_COLS;
-constexpr int JK_MAXR = JK_MAX_N / 32;  // column entries per lane
+constexpr int JK_MAX_CS = 16;          // CTAs of a cluster
+constexpr int JK_W = 8;                // columns of a block
+constexpr int JK_COLS = 2 * JK_W;      // columns of a CTA
+constexpr int JK_MAX_N = JK_MAX_CS * JK_COLS;
+constexpr int JK_THREADS = 512;
+constexpr int JK_WARPS = JK_THREADS / 32;
+constexpr int JK_GP = JK_COLS + 1;     // pitch of the Gram matrix
+constexpr int JK_JP = JK_COLS + 4;     // pitch of J (mma operand: 4 mod 16)
 
-// Partner of player p in round r of a circle-method tournament on ne (even)
-// players: player ne - 1 is fixed and meets r; the others pair as
-// p + q = 2 r (mod ne - 1).  Every pair meets once in ne - 1 rounds.
-__device__ __forceinline__ int jk_partner(int p, int r, int ne) {
-  const int m = ne - 1;
-  if (p == m) return r;
-  if (p == r) return m;
-  int q = 2 * r - p;
-  if (q < 0)
-    q += m;
-  else if (q >= m)
-    q -= m;
-  return q;
+// Rows of a column's A (or V) part, and column pitches in global and shared
+// memory (the latter 4 mod 16, so that mma fragments meet no bank twice).
+__host__ __device__ __forceinline__ int jk_rows(int n) { return (n + 7) & ~7; }
+__host__ __device__ __forceinline__ int jk_pitch(int n) {
+  return ((2 * jk_rows(n) + 15) & ~15) + 4;
+}
+int jk_blocks(int64_t n) { return int((n + JK_COLS - 1) / JK_COLS) * 2; }
+int64_t jk_work(int64_t n) {  // columns, then the column norms
+  return int64_t(jk_blocks(n)) * JK_W * (2 * jk_rows(int(n)) + 1);
+}
+size_t jk_smem(int64_t n) {
+  return sizeof(double) * (size_t(JK_COLS) * jk_pitch(int(n)) + JK_WARPS * 192 + JK_COLS * JK_GP +
+                           JK_COLS * JK_JP);
 }
 
-// Load of a double from the shared memory of a CTA of the cluster (address
-// from mapa: the partner's column, which may sit in this CTA too).
-__device__ __forceinline__ double ld_dsmem(uint32_t addr) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr));
-  return v;
+// Blocks of CTA c in round r of a tournament on nb (even) blocks: block nb - 1
+// is fixed and meets r, the others pair as p + q = 2 r (mod nb - 1).
+__device__ __forceinline__ void jk_pair(int c, int r, int nb, int& p, int& q) {
+  const int m = nb - 1;
+  if (c == 0) {
+    p = r;
+    q = m;
+    return;
+  }
+  p = r + c;
+  if (p >= m) p -= m;
+  q = r - c;
+  if (q < 0) q += m;
+}
+
+// Cosine and sine of the rotation that makes a pair orthogonal, the smaller of
+// the two angles: with dd = be - al, g = 2 ga and h = hypot(dd, g),
+// c = sqrt((1 + |dd| / h) / 2) and s = |g| / (2 h c) with the sign of dd g.
+// They are first taken in single precision (dd and g scaled to a common
+// exponent), which leaves 1e-7 of the pair's inner product for the next sweep,
+// then both multiplied by 1 / sqrt(c^2 + s^2) in double precision (two terms
+// of the series: c^2 + s^2 - 1 is 1e-7), which leaves the rounding of c and s
+// alone.  c = 1 / sqrt(1 + t^2) taken directly is biased by 1e-16 for small t,
+// which adds up over a sweep's thousands of rotations.
+__device__ __forceinline__ void jk_rotation(double al, double be, double ga, double& c,
+                                            double& s) {
+  const double dd = be - al, gg = 2.0 * ga;
+  // 2^-e for the exponent e of |dd| + |g|
+  const int field = 0x7fe00000 - (__double2hiint(fabs(dd) + fabs(gg)) & 0x7ff00000);
+  const double scale = __hiloint2double(field, 0);
+  const double y = fabs(gg) * scale;
+  const float x = float(fabs(dd) * scale), yf = float(y);
+  const float rh = rsqrtf(fmaf(x, x, yf * yf));
+  const float v = fmaf(0.5f * x, rh, 0.5f);  // c^2
+  const float rv = rsqrtf(v);
+  const double c0 = double(v * rv);
+  const double s0 = (0.5 * y) * double(rh * rv);
+  const double d = fma(s0, s0, fma(c0, c0, -1.0));
+  const double f = d * fma(0.375, d, -0.5);
+  c = fma(c0, f, c0);
+  s = fma(s0, f, s0);
+  if ((dd >= 0.0) != (gg > 0.0) && dd != 0.0) s = -s;
 }
 
 __global__ void __launch_bounds__(JK_THREADS, 1)
-    k_jacobi_cluster(int n, const double* __restrict__ Ain, int lda, int trans,
-                     double* __restrict__ Aout, double* __restrict__ Vout, int* err,
-                     int max_sweeps) {
+    k_jacobi_cluster(int n, const double* __restrict__ Ain, int lda, int trans, double* X,
+                     double* __restrict__ U, double* __restrict__ S, double* __restrict__ VT,
+                     int* err, int max_sweeps) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ double sm[];  // A[2][cpc][n], then V[2][cpc][n]
-  __shared__ double s_off[2][JK_CS];  // rank 0: per-CTA sweep maxima, by sweep parity
-  __shared__ double s_woff[JK_MAX_COLS];
-  const int rank = int(cl.block_rank());
-  const int ne = (n + 1) & ~1, cpc = (ne + JK_CS - 1) / JK_CS;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int64_t cn = int64_t(cpc) * n;
-  for (int64_t e = tid; e < cn; e += blockDim.x) {
-    const int j = int(e / n), i = int(e % n), p = rank * cpc + j;
-    if (p < n) {
-      sm[e] = trans ? Ain[p + int64_t(i) * lda] : Ain[i + int64_t(p) * lda];
-      sm[2 * cn + e] = (i == p) ? 1.0 : 0.0;
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int s_rot[2][JK_MAX_CS];  // rank 0: whether a CTA found a pair, by sweep parity
+  __shared__ int s_any;                // this round rotated
+  __shared__ __align__(16) double2 s_cs[JK_COLS - 1][JK_W];  // rotations of a round's steps
+  __shared__ int s_rots[JK_COLS - 1];  // whether a step rotates
+  const int rank = int(cl.block_rank()), cs = int(cl.num_blocks());
+  const int np = jk_rows(n), ldx = 2 * np, P = jk_pitch(n);
+  const int nb = 2 * ((n + JK_COLS - 1) / JK_COLS);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const bool work = rank < nb / 2;
+  double* sX = sm;                       // JK_COLS columns of A over V
+  double* sP = sX + JK_COLS * P;         // partial Gram matrices of the warps
+  double* sG = sP + JK_WARPS * 192;
+  double* sJ = sG + JK_COLS * JK_GP;
+  double* norms = X + int64_t(nb) * JK_W * ldx;
+  if (work) {
+    const int c0 = rank * JK_COLS;
+    for (int e = tid; e < JK_COLS * ldx; e += JK_THREADS) {
+      const int col = c0 + e / ldx, i = e % ldx;
+      double v = 0.0;
+      if (col < n) {
+        if (i < n)
+          v = trans ? Ain[col + int64_t(i) * lda] : Ain[i + int64_t(col) * lda];
+        else if (i >= np)
+          v = i - np == col ? 1.0 : 0.0;
+      }
+      X[int64_t(c0) * ldx + e] = v;
     }
   }
   cl.sync();
   const double tol = 4.0 * 2.220446049250313e-16, tol2 = tol * tol;
-  const int p = rank * cpc + w;
-  const bool own = w < cpc && p < n;
-  const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
-  int cur = 0, sweep = 0;
+  int sweep = 0;
   for (sweep = 0; sweep < max_sweeps; ++sweep) {
-    double off = 0.0;
-    for (int r = 0; r < ne - 1; ++r) {
-      if (own) {
-        const int q = jk_partner(p, r, ne);
-        const double* ap = sm + cur * cn + int64_t(w) * n;
-        const double* vp = ap + 2 * cn;
-        double* na = sm + (cur ^ 1) * cn + int64_t(w) * n;
-        double* nv = na + 2 * cn;
-        if (q >= n) {  // dummy partner (odd n): the column stays
-          for (int i = lane; i < n; i += 32) {
-            na[i] = ap[i];
-            nv[i] = vp[i];
-          }
-        } else {
-          const int rq = q / cpc, jq = q - rq * cpc;
-          uint32_t rb;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(sbase), "r"(rq));
-          const uint32_t aq = rb + uint32_t(8 * (cur * cn + int64_t(jq) * n));
-          const uint32_t vq = aq + uint32_t(16 * cn);
-          // own column o (local), partner column t (over DSMEM)
-          double o[JK_MAXR], t[JK_MAXR], vo[JK_MAXR], vt[JK_MAXR];
+    int found = 0;  // warp 0: a pair was rotated in this sweep
+    for (int r = 0; r < nb - 1; ++r) {
+      if (work) {
+        int bp, bq;
+        jk_pair(rank, r, nb, bp, bq);
+        auto column = [&](int k) {
+          return X + int64_t((k < JK_W ? bp * JK_W : bq * JK_W - JK_W) + k) * ldx;
+        };
+        // a column per warp: its A, and later its V (16-byte copies; np is even)
+        const double* src = column(warp);
+        for (int i = 2 * lane; i < np; i += 64) cp_async16(sX + warp * P + i, src + i, 16);
+        cp_async_commit();
+        if (tid < JK_COLS * JK_COLS)
+          sJ[(tid / JK_COLS) * JK_JP + tid % JK_COLS] = tid / JK_COLS == tid % JK_COLS;
+        cp_async_wait<0>();
+        __syncthreads();
+        for (int i = np + 2 * lane; i < ldx; i += 64) cp_async16(sX + warp * P + i, src + i, 16);
+        cp_async_commit();
+        // Gram matrix: 8 x 8 tiles (0,0), (0,1), (1,1)
+        double acc[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        for (int k4 = warp; k4 < np / 4; k4 += JK_WARPS) {
+          const double x0 = sX[g * P + 4 * k4 + t], x1 = sX[(8 + g) * P + 4 * k4 + t];
+          dmma(acc[0][0], acc[0][1], x0, x0);
+          dmma(acc[1][0], acc[1][1], x0, x1);
+          dmma(acc[2][0], acc[2][1], x1, x1);
+        }
 #pragma unroll
-          for (int k = 0; k < JK_MAXR; ++k) {
-            const int i = lane + 32 * k;
-            const bool in = i < n;
-            t[k] = in ? ld_dsmem(aq + 8 * i) : 0.0;
-            vt[k] = in ? ld_dsmem(vq + 8 * i) : 0.0;
-            o[k] = in ? ap[i] : 0.0;
-            vo[k] = in ? vp[i] : 0.0;
-          }
-          // al = |a_P|^2, be = |a_Q|^2, ga = <a_P, a_Q> for P < Q: both
-          // owners of the pair form the same sums in the same order.
-          const bool low = p < q;
-          double sp = 0.0, sq = 0.0, ga = 0.0;
+        for (int q = 0; q < 3; ++q) {
+          sP[warp * 192 + q * 64 + g * 8 + 2 * t] = acc[q][0];
+          sP[warp * 192 + q * 64 + g * 8 + 2 * t + 1] = acc[q][1];
+        }
+        __syncthreads();
+        if (tid < 192) {
+          double v[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-          for (int k = 0; k < JK_MAXR; ++k) {
-            sp = fma(o[k], o[k], sp);
-            sq = fma(t[k], t[k], sq);
-            ga = low ? fma(o[k], t[k], ga) : fma(t[k], o[k], ga);
-          }
-          sp = wsum(sp);
-          sq = wsum(sq);
-          ga = wsum(ga);
-          const double al = low ? sp : sq, be = low ? sq : sp;
-          const double ab = al * be, g2 = ga * ga;
-          if (ab == 0.0 || g2 <= tol2 * ab) {
-#pragma unroll
-            for (int k = 0; k < JK_MAXR; ++k) {
-              const int i = lane + 32 * k;
-              if (i < n) {
-                na[i] = o[k];
-                nv[i] = vo[k];
+          for (int w = 0; w < JK_WARPS; ++w) v[w & 3] += sP[w * 192 + tid];
+          const int q = tid / 64, i = (tid >> 3) & 7, j = tid & 7;
+          const int row = q == 2 ? 8 + i : i, col = q == 0 ? j : 8 + j;
+          if (q == 1 || i <= j)  // one of (i, j), (j, i) where both were formed
+            sG[row * JK_GP + col] = sG[col * JK_GP + row] = (v[0] + v[1]) + (v[2] + v[3]);
+        }
+        __syncthreads();
+        // Rotations, eight disjoint pairs at a time: warp 0 on G, warp 1 behind
+        // it on J (a named barrier per step, at which warp 0 only arrives).
+        if (warp < 2) {
+          const int steps = r == 0 ? JK_COLS - 1 : JK_W;
+          int any = 0;
+          for (int ir = 0; ir < steps; ++ir) {
+            auto pair = [&](int k, int& p, int& q) {
+              if (r == 0) {  // all pairs of 16 columns
+                p = rr_player(k, ir, JK_COLS);
+                q = rr_player(JK_COLS - 1 - k, ir, JK_COLS);
+              } else {  // pairs across the blocks
+                p = k;
+                q = JK_W + ((k + ir) & (JK_W - 1));
               }
-            }
-          } else {
-            off = fmax(off, g2 / ab);
-            const double dd = be - al, gg = 2.0 * ga;
-            const double sg = ((dd >= 0.0) == (gg > 0.0) || dd == 0.0) ? 1.0 : -1.0;
-            const double tt = sg * fabs(gg) / (fabs(dd) + sqrt(fma(dd, dd, gg * gg)));
-            const double c = rsqrt(fma(tt, tt, 1.0)), sn = c * tt;
-            // P' = c P - s Q, Q' = s P + c Q
-            if (low) {
+            };
+            if (warp == 0) {
+              int p, q;
+              pair(lane & 7, p, q);
+              const double al = sG[p * JK_GP + p], be = sG[q * JK_GP + q],
+                           ga = sG[p * JK_GP + q];
+              // the lane's 2 x 2 blocks of G: pair a by pairs b and b + 4
+              const int a = lane >> 2;
+              int pa, qa, pb[2], qb[2];
+              pair(a, pa, qa);
+              pair(lane & 3, pb[0], qb[0]);
+              pair((lane & 3) + 4, pb[1], qb[1]);
+              double x[2][4];
 #pragma unroll
-              for (int k = 0; k < JK_MAXR; ++k) {
-                const int i = lane + 32 * k;
-                if (i < n) {
-                  na[i] = fma(c, o[k], -(sn * t[k]));
-                  nv[i] = fma(c, vo[k], -(sn * vt[k]));
-                }
+              for (int h = 0; h < 2; ++h) {
+                x[h][0] = sG[pa * JK_GP + pb[h]];
+                x[h][1] = sG[pa * JK_GP + qb[h]];
+                x[h][2] = sG[qa * JK_GP + pb[h]];
+                x[h][3] = sG[qa * JK_GP + qb[h]];
               }
+              double c, sn;
+              jk_rotation(al, be, ga, c, sn);
+              const double ab = al * be;
+              const bool rot = ab != 0.0 && ga * ga > tol2 * ab;
+              if (!rot) {
+                c = 1.0;
+                sn = 0.0;
+              }
+              const int rots = __any_sync(0xffffffffu, rot);
+              if (lane < JK_W) s_cs[ir][lane] = make_double2(c, sn);
+              if (lane == 0) s_rots[ir] = rots;
+              const double ca = __shfl_sync(0xffffffffu, c, a);
+              const double sa = __shfl_sync(0xffffffffu, sn, a);
+              // columns p, q <- c p - s q, s p + c q, on both sides of G
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const double cb = __shfl_sync(0xffffffffu, c, (lane & 3) + 4 * h);
+                const double sb = __shfl_sync(0xffffffffu, sn, (lane & 3) + 4 * h);
+                const double y00 = fma(cb, x[h][0], -sb * x[h][1]);
+                const double y01 = fma(sb, x[h][0], cb * x[h][1]);
+                const double y10 = fma(cb, x[h][2], -sb * x[h][3]);
+                const double y11 = fma(sb, x[h][2], cb * x[h][3]);
+                sG[pa * JK_GP + pb[h]] = fma(ca, y00, -sa * y10);
+                sG[pa * JK_GP + qb[h]] = fma(ca, y01, -sa * y11);
+                sG[qa * JK_GP + pb[h]] = fma(sa, y00, ca * y10);
+                sG[qa * JK_GP + qb[h]] = fma(sa, y01, ca * y11);
+              }
+              any |= rots;
+              __syncwarp();
+              asm volatile("bar.arrive %0, 64;" ::"r"(ir + 1) : "memory");
             } else {
+              asm volatile("bar.sync %0, 64;" ::"r"(ir + 1) : "memory");
+              if (!s_rots[ir]) continue;
+              double* row = sJ + (lane & 15) * JK_JP;
 #pragma unroll
-              for (int k = 0; k < JK_MAXR; ++k) {
-                const int i = lane + 32 * k;
-                if (i < n) {
-                  na[i] = fma(sn, t[k], c * o[k]);
-                  nv[i] = fma(sn, vt[k], c * vo[k]);
-                }
+              for (int h = 0; h < 4; ++h) {
+                const int k = (lane >> 4) * 4 + h;
+                int p, q;
+                pair(k, p, q);
+                const double2 rk = s_cs[ir][k];
+                const double xp = row[p], xq = row[q];
+                row[p] = fma(rk.x, xp, -rk.y * xq);
+                row[q] = fma(rk.y, xp, rk.x * xq);
               }
+              __syncwarp();
             }
+          }
+          if (warp == 0) {
+            found |= any;
+            if (lane == 0) s_any = any;
+          }
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        if (s_any) {
+          // [A; V] J, from shared memory straight to the columns in L2
+          double bj[4][2];
+          double* out[2][2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) bj[k][j] = sJ[(4 * k + t) * JK_JP + 8 * j + g];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) out[j][h] = column(8 * j + 2 * t + h) + g;
+          }
+#pragma unroll 4
+          for (int mt = warp; mt < ldx / 8; mt += JK_WARPS) {
+            double o[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const double x = sX[(4 * k + t) * P + 8 * mt + g];
+              dmma(o[0][0], o[0][1], x, bj[k][0]);
+              dmma(o[1][0], o[1][1], x, bj[k][1]);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) out[j][h][8 * mt] = o[j][h];
           }
         }
       }
-      if (r == ne - 2) {  // last round of the sweep: publish this CTA's maximum
-        if (lane == 0 && w < JK_MAX_COLS) s_woff[w] = own ? off : 0.0;
-        __syncthreads();
-        if (tid == 0) {
-          double m = 0.0;
-          for (int j = 0; j < cpc; ++j) m = fmax(m, s_woff[j]);
-          double* so = cl.map_shared_rank(&s_off[sweep & 1][0], 0);
-          so[rank] = m;
-        }
+      if (r == nb - 2 && tid == 0) {
+        int* so = cl.map_shared_rank(&s_rot[sweep & 1][0], 0);
+        so[rank] = found;
       }
       cl.sync();
-      cur ^= 1;
     }
-    const double* so = cl.map_shared_rank(&s_off[sweep & 1][0], 0);
-    double m = 0.0;
-    for (int k = 0; k < JK_CS; ++k) m = fmax(m, so[k]);
-    if (m <= tol2) break;
+    const int* so = cl.map_shared_rank(&s_rot[sweep & 1][0], 0);
+    int any = 0;
+    for (int k = 0; k < cs; ++k) any |= so[k];
+    if (!any) break;
   }
   if (rank == 0 && tid == 0 && sweep >= max_sweeps) atomicExch(err, 5);
-  for (int64_t e = tid; e < cn; e += blockDim.x) {
-    const int j = int(e / n), i = int(e % n), pc = rank * cpc + j;
-    if (pc < n) {
-      Aout[i + int64_t(pc) * n] = sm[cur * cn + e];
-      Vout[i + int64_t(pc) * n] = sm[(2 + cur) * cn + e];
+  // Singular values = column norms, ranked descending (stable on index), and
+  // the factors in that order, as in jacobi_finish.
+  const int c0 = rank * JK_COLS;
+  if (work) {
+    for (int k = warp; k < JK_COLS; k += JK_WARPS) {
+      const double* x = X + int64_t(c0 + k) * ldx;
+      double v = 0.0;
+      for (int i = lane; i < n; i += 32) {
+        const double xi = __ldcg(x + i);
+        v = fma(xi, xi, v);
+      }
+      v = wsum(v);
+      if (lane == 0) norms[c0 + k] = sqrt(v);
     }
   }
-  cl.sync();  // rank 0's published maxima are read until here
+  cl.sync();
+  if (work) {
+    double* sn = sm;
+    int* pos = reinterpret_cast<int*>(sP);
+    for (int k = tid; k < n; k += JK_THREADS) sn[k] = __ldcg(norms + k);
+    __syncthreads();
+    for (int k = warp; k < JK_COLS; k += JK_WARPS) {
+      const int col = c0 + k;
+      int before = 0;
+      if (col < n)
+        for (int i = lane; i < n; i += 32)
+          before += (sn[i] > sn[col]) || (sn[i] == sn[col] && i < col);
+      for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+      if (lane == 0) {
+        pos[k] = before;
+        if (col < n) S[before] = sn[col];
+      }
+    }
+    __syncthreads();
+    for (int e = tid; e < JK_COLS * n; e += JK_THREADS) {
+      const int k = e / n, i = e % n, col = c0 + k;
+      if (col >= n) continue;
+      const double sj = sn[col];
+      const double* x = X + int64_t(col) * ldx;
+      const double ua = sj > 0.0 ? __ldcg(x + i) / sj : (i == pos[k] ? 1.0 : 0.0);
+      const double v = __ldcg(x + np + i);
+      U[i + int64_t(pos[k]) * n] = trans ? v : ua;
+      VT[pos[k] + int64_t(i) * n] = trans ? ua : v;
+    }
+  }
+  cl.sync();  // rank 0's published flags are read until here
 }
 
 // ---------------------------------------------------------------------------
@@ -1324,22 +1486,23 @@ static bool jacobi_block_fits(int64_t n) {
          getenv_flag_on("TTG_JACOBI_BLOCK");
 }
 
-size_t jacobi_cluster_smem(int64_t n) {
-  const int64_t cpc = (((n + 1) & ~int64_t(1)) + JK_CS - 1) / JK_CS;
-  return sizeof(double) * 4 * size_t(cpc) * size_t(n);
+// CTAs of the cluster form: one per pair of blocks, a power of two.
+int jacobi_cluster_size(int64_t n) {
+  int cs = 1;
+  while (2 * cs < jk_blocks(n)) cs *= 2;
+  return cs;
 }
 
 // The cluster form runs where one CTA's shared memory cannot hold both A
-// and V (n > 113) up to JK_MAX_N (measured 2.1x the grid-wide form's speed
-// at n = 120 and 144, 1.2x at 256), unless TTG_JACOBI_CLUSTER=0, when the device
-// can place a 16-CTA cluster with that shared memory (checked once per
-// device and size class: attributes set, cudaOccupancyMaxActiveClusters).
-// Outside a grouped batch it also takes the sizes from
-// TTG_JACOBI_CLUSTER_MIN_N (default 48) up, which the one-CTA kernel could
-// hold: a lone solve waits on each SVD (whole SVD of a Gaussian n x n matrix,
-// cluster against one CTA: 2.0 against 5.7 ms at n = 113, 0.89 against 1.39
-// at 64, 0.68 against 0.84 at 48, even at 32), while a grouped batch fills
-// the GPU with concurrent systems and wants the one-CTA kernel's single SM.
+// and V (n > 113) up to JK_MAX_N, unless TTG_JACOBI_CLUSTER=0, when the device
+// can place a cluster with that shared memory (checked once per device and
+// size class: attributes set, cudaOccupancyMaxActiveClusters).  Outside a
+// grouped batch it also takes the sizes from TTG_JACOBI_CLUSTER_MIN_N (default
+// 48) up, which the one-CTA kernel could hold: a lone solve waits on each SVD
+// (triangular factor, cluster against one CTA: 0.31 against 0.71 ms at n = 47,
+// 0.18 against 0.31 at 32), while a grouped batch fills the GPU with concurrent
+// systems and wants the one-CTA kernel's single SM.  Below 48 both run the
+// one-CTA kernel, so that a grouped batch of such ranks repeats a lone solve.
 int64_t jacobi_cluster_min_n() {
   static const int64_t v = [] {
     const char* e = getenv("TTG_JACOBI_CLUSTER_MIN_N");
@@ -1349,17 +1512,30 @@ int64_t jacobi_cluster_min_n() {
   return v;
 }
 
+cudaLaunchConfig_t jacobi_cluster_config(int64_t n, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(jacobi_cluster_size(n));
+  cfg.blockDim = dim3(JK_THREADS);
+  cfg.dynamicSmemBytes = jk_smem(n);
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = jacobi_cluster_size(n);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
 bool jacobi_cluster_ok(Context* c, int64_t n) {
   static const bool on = [] {
     const char* e = getenv("TTG_JACOBI_CLUSTER");
     return !(e && e[0] == '0');
   }();
   if (!on || n > JK_MAX_N || n < 2) return false;
-  const size_t smem = jacobi_cluster_smem(n);
   static std::mutex mu;
   static std::map<std::pair<int, size_t>, bool> seen;
   std::lock_guard<std::mutex> lk(mu);
-  auto key = std::make_pair(c->device, smem);
+  auto key = std::make_pair(c->device, jk_smem(n) * 32 + jacobi_cluster_size(n));
   auto it = seen.find(key);
   if (it != seen.end()) return it->second;
   // The attribute is set once to the largest size any n takes (setting it
@@ -1367,19 +1543,10 @@ bool jacobi_cluster_ok(Context* c, int64_t n) {
   bool ok = cudaFuncSetAttribute(k_jacobi_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed,
                                  1) == cudaSuccess &&
             cudaFuncSetAttribute(k_jacobi_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(jacobi_cluster_smem(JK_MAX_N))) == cudaSuccess;
+                                 int(jk_smem(JK_MAX_N))) == cudaSuccess;
   if (ok) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(JK_CS);
-    cfg.blockDim = dim3(JK_THREADS);
-    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = JK_CS;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = jacobi_cluster_config(n, attr);
     int clusters = 0;
     ok = cudaOccupancyMaxActiveClusters(&clusters, k_jacobi_cluster, &cfg) == cudaSuccess &&
          clusters >= 1;
@@ -1395,8 +1562,32 @@ void jacobi_svd_f64(Context* c, int64_t n, const double* A, int64_t lda, double*
   TTG_REQUIRE(n >= 1 && n <= 4096, "jacobi_svd: n = %lld out of range", (long long)n);
   const size_t mat = size_t(n * n) * sizeof(double);
   const int mode = 2 * mat <= SMEM_LIMIT ? 2 : (mat <= SMEM_LIMIT ? 1 : 0);
+  const bool block = mode == 0 && jacobi_block_fits(n);
+  if (!block && (mode == 0 || mode == 1 || (!c->rec && n >= jacobi_cluster_min_n())) &&
+      jacobi_cluster_ok(c, n)) {
+    // One cluster, the columns in L2.
+    DBuf<double> X(c, jk_work(n));
+    const int ns = int(n), ilda = int(lda), sweeps = c->jacobi_max_sweeps;
+    double* Xw = X.p();
+    int* err = c->d_err + 3;
+    auto issue = [=](cudaStream_t s) {
+      cudaLaunchAttribute attr[1];
+      cudaLaunchConfig_t cfg = jacobi_cluster_config(ns, attr);
+      cfg.stream = s;
+      TTG_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi_cluster, ns, A, ilda, trans, Xw, U, S, VT, err,
+                                  sweeps));
+    };
+    if (c->rec) {
+      rec_op(c->rec, [issue](cudaStream_t s, cusolverDnHandle_t) { issue(s); });
+    } else {
+      issue(c->stream);
+    }
+    c->launches += 1;
+    TTG_CHECK_LAUNCH();
+    return;
+  }
   DBuf<double> V(c, n * n), work(c, n * n + 2 * n);
-  if (mode == 0 && jacobi_block_fits(n)) {
+  if (block) {
     // Block-cyclic grid-wide rounds: one CTA per block pair.
     const size_t bsm = sizeof(double) * 4 * JB_W * size_t(n);
     ensure_smem_attr(k_jacobi_block.fn(), c->device, int(bsm));
@@ -1411,41 +1602,6 @@ void jacobi_svd_f64(Context* c, int64_t n, const double* A, int64_t lda, double*
     memset_async(c, bar.p(), 0, 2 * sizeof(unsigned));
     launch(c, k_jacobi_block, blocks, JB_THREADS, bsm, int(n), A, int(lda), work.p(), V.p(),
            bar.p(), offmax.p(), c->d_err + 0, c->d_err + 3, trans, c->jacobi_max_sweeps);
-    launch(c, k_jacobi_finish, 1, SD_THREADS, 0, int(n), work.p(), V.p(), U, S, VT,
-           work.p() + int64_t(n) * n, trans);
-    TTG_CHECK_LAUNCH();
-    return;
-  }
-  if ((mode == 0 || mode == 1 || (!c->rec && n >= jacobi_cluster_min_n())) &&
-      jacobi_cluster_ok(c, n)) {
-    // One 16-CTA cluster, A and V in distributed shared memory.
-    const size_t jsm = jacobi_cluster_smem(n);
-    const int ns = int(n), ilda = int(lda), sweeps = c->jacobi_max_sweeps;
-    double* Aw = work.p();
-    double* Vw = V.p();
-    int* err = c->d_err + 3;
-    auto issue = [=](cudaStream_t s) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(JK_CS);
-      cfg.blockDim = dim3(JK_THREADS);
-      cfg.dynamicSmemBytes = jsm;
-      cfg.stream = s;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = JK_CS;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      TTG_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi_cluster, ns, A, ilda, trans, Aw, Vw, err,
-                                  sweeps));
-    };
-    if (c->rec) {
-      rec_op(c->rec, [issue](cudaStream_t s, cusolverDnHandle_t) { issue(s); });
-    } else {
-      issue(c->stream);
-    }
-    c->launches += 1;
     launch(c, k_jacobi_finish, 1, SD_THREADS, 0, int(n), work.p(), V.p(), U, S, VT,
            work.p() + int64_t(n) * n, trans);
     TTG_CHECK_LAUNCH();
