@@ -485,14 +485,16 @@ TTG_BODY(k_collapse_flag)(TTG_BLOCK, int64_t k, const double* G0, int64_t ld0, c
 }
 TTG_KERNEL(k_collapse_flag, 0);
 
-// *flag |= 1 when max |G - I| > tol (G: n x n Gram matrix of a basis).
+// *flag |= 1 when max |G - I| > tol (G: n x n Gram matrix of a basis).  Columns
+// over blocks, rows over threads.
 TTG_BODY(k_orth_check)(TTG_BLOCK, int64_t n, const double* G, double tol, int* flag) {
   pdl_begin();
   int bad = 0;
-  for (int64_t e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const double v = G[e] - ((e % n) == (e / n) ? 1.0 : 0.0);
-    if (!(fabs(v) <= tol)) bad = 1;
-  }
+  for (int64_t j = blockIdx.x; j < n; j += gridDim.x)
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+      const double v = G[i + j * n] - (i == j ? 1.0 : 0.0);
+      if (!(fabs(v) <= tol)) bad = 1;
+    }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 TTG_KERNEL(k_orth_check, 0);
@@ -768,7 +770,8 @@ void collapse_flag(Context* c, int64_t k, const double* G0, int64_t ld0, const d
 }
 
 void orth_check(Context* c, int64_t n, const double* G, double tol, int* flag) {
-  launch(c, k_orth_check, 1, 256, 0, n, G, tol, flag);
+  launch(c, k_orth_check, unsigned(std::min<int64_t>((n + 3) / 4, c->num_sms)), 128, 0, n, G, tol,
+         flag);
   TTG_CHECK_LAUNCH();
 }
 
