@@ -202,15 +202,14 @@ int ttg_local_matvec(ttg_context ctx, int64_t rx1, int64_t n, int64_t rx2, int64
     TTG_CUDA(cudaMemsetAsync(c->d_err + 1, 0, sizeof(int), c->stream));
     nat_to_rev(c, rx1, n, rx2, x, xr.p(), 1.0);
     op.apply(c, xr.p(), yr.p());
-    fill_f64(c, sz, 0.0, y);
-    rev_to_nat_add(c, rx1, n, rx2, yr.p(), y, 1.0);
+    rev_to_nat(c, rx1, n, rx2, yr.p(), y);
   }
-  sync(c);
-  if (precision == TTG_MIXED) {
-    int herr = 0;
-    TTG_CUDA(cudaMemcpy(&herr, c->d_err + 1, sizeof(int), cudaMemcpyDeviceToHost));
-    if (herr) fail(TTG_ERR_TIMEOUT, "tensor-core matvec: a bounded wait timed out");
-  }
+  int herr = 0;
+  if (precision == TTG_MIXED)
+    read_device(c, &herr, c->d_err + 1, sizeof(int));
+  else
+    sync(c);
+  if (herr) fail(TTG_ERR_TIMEOUT, "tensor-core matvec: a bounded wait timed out");
   TTG_API_END
 }
 
@@ -226,15 +225,14 @@ int ttg_next_phi(ttg_context ctx, int32_t dir, int64_t rx1, int64_t n, int64_t r
   TTG_CUDA(cudaSetDevice(c->device));
   const int64_t cnt =
       next_phi_f64(c, dir, rx1, n, rx2, ry1, ry2, ra1, ra2, Phi_prev, x, A, y, Phi_out);
-  if (nrm_out) {
-    double nrm = nrm2_host(c, cnt, Phi_out);
-    if (nrm > 0)
-      axpby_f64(c, cnt, 1.0 / nrm, Phi_out, 0.0, Phi_out);
-    else
-      nrm = 1.0;
-    *nrm_out = nrm;
+  if (nrm_out) {  // normalised on the device: one read, no wait before the scaling
+    DBuf<double> nrm(c, 1);
+    dot_f64(c, cnt, Phi_out, nullptr, nrm.p(), true);
+    normalize_by_dev(c, cnt, Phi_out, nrm.p());
+    read_scalars(c, nrm.p(), nrm_out, 1);
+  } else {
+    sync(c);
   }
-  sync(c);
   TTG_API_END
 }
 

@@ -60,5 +60,8 @@ void nat_to_rev(Context* c, int64_t r1, int64_t n, int64_t r2, const double* x, 
 // x[natural] += scale * y[reversed]
 void rev_to_nat_add(Context* c, int64_t r1, int64_t n, int64_t r2, const float* y, double* x,
                     double scale);
+// x = y, in two launches of half the tiles each (a zero fill and an addition
+// before: a local matvec keeps its number of launches).
+void rev_to_nat(Context* c, int64_t r1, int64_t n, int64_t r2, const float* y, double* x);
 
 }  // namespace ttg
