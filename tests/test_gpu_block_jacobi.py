@@ -1,6 +1,6 @@
-"""Block Jacobi SVD of the cluster (csrc/small_dense.cu) at the edges of its
-blocks of 8 columns, its pairs of 16 and its cluster sizes, on spectra and
-scales that its single-precision angles have to stand."""
+"""Block Jacobi SVDs (csrc/small_dense.cu: one CTA, and a cluster) at the edges of
+their blocks of 8 columns, pairs of 16 and cluster sizes, on spectra and
+scales that their single-precision angles have to stand."""
 import numpy as np
 import pytest
 
@@ -8,7 +8,8 @@ import ttgpu
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [48, 49, 57, 64, 65, 112, 113, 127, 128, 129, 240, 241, 255, 256]
+SIZES = [9, 15, 16, 17, 24, 31, 32, 33, 47, 48, 49, 57, 64, 65, 112, 113, 127, 128, 129, 240,
+         241, 255, 256]
 
 
 def _check(A, U, s, VT):
@@ -31,7 +32,7 @@ def test_gaussian(ctx, n):
     _check(A, *ttgpu.dense_svd(A, ctx=ctx))
 
 
-@pytest.mark.parametrize("n", [48, 100, 200])
+@pytest.mark.parametrize("n", [12, 48, 100, 200])
 def test_tall_and_wide(ctx, n):
     g = np.random.default_rng(n)
     A = g.standard_normal((5 * n + 3, n))
@@ -41,13 +42,13 @@ def test_tall_and_wide(ctx, n):
 
 
 @pytest.mark.parametrize("scale", [1e-60, 1e60])
-@pytest.mark.parametrize("n", [50, 130])
+@pytest.mark.parametrize("n", [20, 50, 130])
 def test_scales(ctx, n, scale):
     A = np.random.default_rng(n).standard_normal((n, n)) * scale
     _check(A, *ttgpu.dense_svd(A, ctx=ctx))
 
 
-@pytest.mark.parametrize("n,decades", [(64, 12), (96, 14), (160, 8)])
+@pytest.mark.parametrize("n,decades", [(24, 14), (40, 12), (64, 12), (96, 14), (160, 8)])
 def test_graded(ctx, n, decades):
     g = np.random.default_rng(7)
     Q1, _ = np.linalg.qr(g.standard_normal((n, n)))
@@ -56,7 +57,7 @@ def test_graded(ctx, n, decades):
     _check(A, *ttgpu.dense_svd(A, ctx=ctx))
 
 
-@pytest.mark.parametrize("n", [56, 140])
+@pytest.mark.parametrize("n", [30, 56, 140])
 def test_columns_of_very_different_size(ctx, n):
     """Norms over 60 decades and two columns almost parallel: angles far below
     what single precision holds by itself."""

@@ -46,60 +46,315 @@ __device__ __forceinline__ int rr_player(int k, int r, int ne) {
   return k == 0 ? 0 : 1 + x;
 }
 
-// Sum over the G lanes of a warp (G = 32) or half-warp (G = 16); all 32
-// lanes take part in every shuffle.
-template <int G>
-__device__ __forceinline__ double gsum(double v) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+// ---------------------------------------------------------------------------
+// Pieces of the block Jacobi SVDs
+// ---------------------------------------------------------------------------
+
+constexpr int JK_MAX_CS = 16;          // CTAs of a cluster
+constexpr int JK_W = 8;                // columns of a block
+constexpr int JK_COLS = 2 * JK_W;      // columns of a CTA
+constexpr int JK_MAX_N = JK_MAX_CS * JK_COLS;
+constexpr int JK_THREADS = 512;
+constexpr int JK_WARPS = JK_THREADS / 32;
+constexpr int JK_GP = JK_COLS + 1;     // pitch of the Gram matrix
+constexpr int JK_JP = JK_COLS + 4;     // pitch of J (mma operand: 4 mod 16)
+
+// Rows of a column's A (or V) part, and column pitches in global and shared
+// memory (the latter 4 mod 16, so that mma fragments meet no bank twice).
+__host__ __device__ __forceinline__ int jk_rows(int n) { return (n + 7) & ~7; }
+__host__ __device__ __forceinline__ int jk_pitch(int n) {
+  return ((2 * jk_rows(n) + 15) & ~15) + 4;
+}
+int jk_blocks(int64_t n) { return int((n + JK_COLS - 1) / JK_COLS) * 2; }
+int64_t jk_work(int64_t n) {  // columns, then the column norms
+  return int64_t(jk_blocks(n)) * JK_W * (2 * jk_rows(int(n)) + 1);
+}
+size_t jk_smem(int64_t n) {
+  return sizeof(double) * (size_t(JK_COLS) * jk_pitch(int(n)) + JK_WARPS * 192 + JK_COLS * JK_GP +
+                           JK_COLS * JK_JP);
 }
 
-// One Jacobi rotation of the column pair p < q of A (n x n, ld n) and of V,
-// on the G lanes gl = 0..G-1 of a warp or half-warp.  live = false keeps the
-// group in the shuffles and touches nothing.  Returns max(off, ga^2/(al be))
-// when the pair is rotated, else off.
-template <int G>
-__device__ __forceinline__ double jacobi_pair(double* A, double* V, int n, int p, int q, int gl,
-                                              bool live, double tol2, double off) {
-  double* ap = A + int64_t(p) * n;
-  double* aq = A + int64_t(q) * n;
-  double al = 0.0, be = 0.0, ga = 0.0;
-  if (live) {
-    for (int i = gl; i < n; i += G) {
-      const double x = ap[i], y = aq[i];
-      al += x * x;
-      be += y * y;
-      ga += x * y;
+// Blocks of CTA c in round r of a tournament on nb (even) blocks: block nb - 1
+// is fixed and meets r, the others pair as p + q = 2 r (mod nb - 1).
+__device__ __forceinline__ void jk_pair(int c, int r, int nb, int& p, int& q) {
+  const int m = nb - 1;
+  if (c == 0) {
+    p = r;
+    q = m;
+    return;
+  }
+  p = r + c;
+  if (p >= m) p -= m;
+  q = r - c;
+  if (q < 0) q += m;
+}
+
+// Cosine and sine of the rotation that makes a pair orthogonal, the smaller of
+// the two angles: with dd = be - al, g = 2 ga and h = hypot(dd, g),
+// c = sqrt((1 + |dd| / h) / 2) and s = |g| / (2 h c) with the sign of dd g.
+// They are first taken in single precision (dd and g scaled to a common
+// exponent), which leaves 1e-7 of the pair's inner product for the next sweep,
+// then both multiplied by 1 / sqrt(c^2 + s^2) in double precision (two terms
+// of the series: c^2 + s^2 - 1 is 1e-7), which leaves the rounding of c and s
+// alone.  c = 1 / sqrt(1 + t^2) taken directly is biased by 1e-16 for small t,
+// which adds up over a sweep's thousands of rotations.
+__device__ __forceinline__ void jk_rotation(double al, double be, double ga, double& c,
+                                            double& s) {
+  const double dd = be - al, gg = 2.0 * ga;
+  // 2^-e for the exponent e of |dd| + |g|
+  const int field = 0x7fe00000 - (__double2hiint(fabs(dd) + fabs(gg)) & 0x7ff00000);
+  const double scale = __hiloint2double(field, 0);
+  const double y = fabs(gg) * scale;
+  const float x = float(fabs(dd) * scale), yf = float(y);
+  const float rh = rsqrtf(fmaf(x, x, yf * yf));
+  const float v = fmaf(0.5f * x, rh, 0.5f);  // c^2
+  const float rv = rsqrtf(v);
+  const double c0 = double(v * rv);
+  const double s0 = (0.5 * y) * double(rh * rv);
+  const double d = fma(s0, s0, fma(c0, c0, -1.0));
+  const double f = d * fma(0.375, d, -0.5);
+  c = fma(c0, f, c0);
+  s = fma(s0, f, s0);
+  if ((dd >= 0.0) != (gg > 0.0) && dd != 0.0) s = -s;
+}
+
+// The rotations of a round on the Gram matrix sG of a block pair, by one warp,
+// collected in sJ (the identity at the start): eight disjoint pairs per step,
+// those across the two blocks in eight steps, or all 120 in fifteen.  Pairs
+// within the tolerance (cosine squared at most tol2) stay.  Returns whether
+// any pair was rotated.
+__device__ __forceinline__ int jk_rotate(double* sG, double* sJ, bool all, double tol2) {
+  const int lane = threadIdx.x & 31;
+  const int steps = all ? JK_COLS - 1 : JK_W;
+  int any = 0;
+  for (int ir = 0; ir < steps; ++ir) {
+    auto pair = [&](int k, int& p, int& q) {
+      if (all) {
+        p = rr_player(k, ir, JK_COLS);
+        q = rr_player(JK_COLS - 1 - k, ir, JK_COLS);
+      } else {
+        p = k;
+        q = JK_W + ((k + ir) & (JK_W - 1));
+      }
+    };
+    int p, q;
+    pair(lane & 7, p, q);
+    const double al = sG[p * JK_GP + p], be = sG[q * JK_GP + q], ga = sG[p * JK_GP + q];
+    // the lane's 2 x 2 blocks of G: pair a by pairs b and b + 4; its rows of J
+    const int a = lane >> 2;
+    int pa, qa, pb[2], qb[2];
+    pair(a, pa, qa);
+    pair(lane & 3, pb[0], qb[0]);
+    pair((lane & 3) + 4, pb[1], qb[1]);
+    double x[2][4], jp[4], jq[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      x[h][0] = sG[pa * JK_GP + pb[h]];
+      x[h][1] = sG[pa * JK_GP + qb[h]];
+      x[h][2] = sG[qa * JK_GP + pb[h]];
+      x[h][3] = sG[qa * JK_GP + qb[h]];
+    }
+    double* row = sJ + (lane & 3) * JK_JP;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      jp[h] = row[4 * h * JK_JP + pa];
+      jq[h] = row[4 * h * JK_JP + qa];
+    }
+    double c, s;
+    jk_rotation(al, be, ga, c, s);
+    const double ab = al * be;
+    const bool rot = ab != 0.0 && ga * ga > tol2 * ab;
+    if (!rot) {
+      c = 1.0;
+      s = 0.0;
+    }
+    any |= __any_sync(0xffffffffu, rot);
+    const double ca = __shfl_sync(0xffffffffu, c, a), sa = __shfl_sync(0xffffffffu, s, a);
+    // columns p, q <- c p - s q, s p + c q, on both sides of G
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double cb = __shfl_sync(0xffffffffu, c, (lane & 3) + 4 * h);
+      const double sb = __shfl_sync(0xffffffffu, s, (lane & 3) + 4 * h);
+      const double y00 = fma(cb, x[h][0], -sb * x[h][1]), y01 = fma(sb, x[h][0], cb * x[h][1]);
+      const double y10 = fma(cb, x[h][2], -sb * x[h][3]), y11 = fma(sb, x[h][2], cb * x[h][3]);
+      sG[pa * JK_GP + pb[h]] = fma(ca, y00, -sa * y10);
+      sG[pa * JK_GP + qb[h]] = fma(ca, y01, -sa * y11);
+      sG[qa * JK_GP + pb[h]] = fma(sa, y00, ca * y10);
+      sG[qa * JK_GP + qb[h]] = fma(sa, y01, ca * y11);
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      row[4 * h * JK_JP + pa] = fma(ca, jp[h], -sa * jq[h]);
+      row[4 * h * JK_JP + qa] = fma(sa, jp[h], ca * jq[h]);
+    }
+    __syncwarp();
+  }
+  return any;
+}
+
+// ---------------------------------------------------------------------------
+// Block Jacobi SVD in one CTA, for n <= JS_MAX_N: the columns, each A over V,
+// in shared memory in blocks of 8.  A round of a round-robin tournament on the
+// blocks takes all block pairs at once: the Gram matrix of each pair's 16
+// columns of A (mma.m8n8k4, its K split over the warps of the pair), the
+// rotations on it by one warp per pair (jk_rotate: the 64 pairs across the
+// blocks, in a sweep's first round all 120), and [A; V] J (mma).  A rotation on
+// the Gram matrix is that of one-sided Jacobi on the columns (al = |a_p|^2, be
+// = |a_q|^2, ga = <a_p, a_q>), whose entries round relative to the columns'
+// norms; each round forms the matrices anew from the columns.  A sweep that
+// rotates no pair ends the iteration (|ga| <= 4 eps sqrt(al be) for all).
+// Bound by the chain of rotation steps, about 700 cycles each, n of them per
+// sweep where one pair per warp took n barriers and as many passes over the
+// columns.  Triangular factor: 0.085 ms for 0.132 at n = 16, 0.155 for 0.306 at
+// 32, 0.32 for 0.71 at 47.
+// Status: *err = 5 if the sweep limit is reached.
+// ---------------------------------------------------------------------------
+
+constexpr int JS_MAX_N = 96;
+
+size_t js_smem(int64_t n) {
+  const int pairs = jk_blocks(n) / 2;
+  return sizeof(double) * (size_t(jk_blocks(n)) * JK_W * jk_pitch(int(n)) + JK_WARPS * 192 +
+                           size_t(pairs) * JK_COLS * (JK_GP + JK_JP));
+}
+
+TTG_BODY(k_jacobi_svd)(TTG_BLOCK, int n, const double* __restrict__ Ain, int lda,
+                       double* __restrict__ U, double* __restrict__ S, double* __restrict__ VT,
+                       int trans, int* err, int max_sweeps) {
+  pdl_begin();
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int s_any[JS_MAX_N / JK_COLS], s_found;
+  const int np = jk_rows(n), ldx = 2 * np, P = jk_pitch(n);
+  const int nb = 2 * ((n + JK_COLS - 1) / JK_COLS), pairs = nb / 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  double* sX = sm;                          // nb * 8 columns of A over V
+  double* sP = sX + nb * JK_W * P;          // partial Gram matrices of the warps
+  double* sG = sP + JK_WARPS * 192;         // per pair
+  double* sJ = sG + pairs * JK_COLS * JK_GP;
+  for (int col = warp; col < nb * JK_W; col += JK_WARPS)
+    for (int i = lane; i < ldx; i += 32) {
+      double v = 0.0;
+      if (col < n) {
+        if (i < n)
+          v = trans ? Ain[col + int64_t(i) * lda] : Ain[i + int64_t(col) * lda];
+        else if (i >= np)
+          v = i - np == col ? 1.0 : 0.0;
+      }
+      sX[col * P + i] = v;
+    }
+  const double tol = 4.0 * 2.220446049250313e-16, tol2 = tol * tol;
+  const int wpp = JK_WARPS / pairs;  // warps per pair in the Gram products
+  int sweep = 0;
+  for (sweep = 0; sweep < max_sweeps; ++sweep) {
+    int found = 0;
+    for (int r = 0; r < nb - 1; ++r) {
+      __syncthreads();  // columns of the previous round are written
+      if (warp < wpp * pairs) {
+        int bp, bq;
+        jk_pair(warp / wpp, r, nb, bp, bq);
+        const double* x0 = sX + (bp * JK_W + g) * P + t;
+        const double* x1 = sX + (bq * JK_W + g) * P + t;
+        double acc[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        for (int k4 = warp % wpp; k4 < np / 4; k4 += wpp) {
+          const double u = x0[4 * k4], v = x1[4 * k4];
+          dmma(acc[0][0], acc[0][1], u, u);
+          dmma(acc[1][0], acc[1][1], u, v);
+          dmma(acc[2][0], acc[2][1], v, v);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          sP[warp * 192 + q * 64 + g * 8 + 2 * t] = acc[q][0];
+          sP[warp * 192 + q * 64 + g * 8 + 2 * t + 1] = acc[q][1];
+        }
+      }
+      __syncthreads();
+      for (int e = tid; e < pairs * 192; e += JK_THREADS) {
+        const int pr = e / 192, el = e % 192;
+        double v = 0.0;
+        for (int w = 0; w < wpp; ++w) v += sP[(pr * wpp + w) * 192 + el];
+        const int q = el / 64, i = (el >> 3) & 7, j = el & 7;
+        const int row = q == 2 ? 8 + i : i, col = q == 0 ? j : 8 + j;
+        double* G = sG + pr * JK_COLS * JK_GP;
+        if (q == 1 || i <= j) G[row * JK_GP + col] = G[col * JK_GP + row] = v;
+      }
+      for (int e = tid; e < pairs * JK_COLS * JK_COLS; e += JK_THREADS) {
+        const int pr = e / (JK_COLS * JK_COLS), i = (e / JK_COLS) % JK_COLS, j = e % JK_COLS;
+        sJ[pr * JK_COLS * JK_JP + i * JK_JP + j] = i == j ? 1.0 : 0.0;
+      }
+      __syncthreads();
+      if (warp < pairs) {
+        const int any = jk_rotate(sG + warp * JK_COLS * JK_GP, sJ + warp * JK_COLS * JK_JP, r == 0,
+                                  tol2);
+        found |= any;
+        if (lane == 0) s_any[warp] = any;
+      }
+      __syncthreads();
+      const int mts = ldx / 8;
+      for (int u = warp; u < pairs * mts; u += JK_WARPS) {
+        const int pr = u / mts, mt = u % mts;
+        if (!s_any[pr]) continue;
+        int bp, bq;
+        jk_pair(pr, r, nb, bp, bq);
+        const double* J = sJ + pr * JK_COLS * JK_JP;
+        double* xp = sX + bp * JK_W * P + 8 * mt + g;
+        double* xq = sX + bq * JK_W * P + 8 * mt + g;
+        double o[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double x = k < 2 ? xp[(4 * k + t) * P] : xq[(4 * (k - 2) + t) * P];
+          dmma(o[0][0], o[0][1], x, J[(4 * k + t) * JK_JP + g]);
+          dmma(o[1][0], o[1][1], x, J[(4 * k + t) * JK_JP + 8 + g]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          xp[(2 * t + h) * P] = o[0][h];
+          xq[(2 * t + h) * P] = o[1][h];
+        }
+      }
+    }
+    if (tid == 0) s_found = 0;
+    __syncthreads();
+    if (found && lane == 0) s_found = 1;
+    __syncthreads();
+    if (!s_found) break;
+  }
+  if (tid == 0 && sweep >= max_sweeps) atomicExch(err, 5);
+  // Singular values = column norms, ranked descending (stable on index), and
+  // the factors in that order.  With trans the rotated matrix is the transpose
+  // of the input (X = In^T = Ux S Vx^T), so the input's factors swap: U = Vx,
+  // VT = Ux^T.
+  double* sn = sP;
+  int* pos = reinterpret_cast<int*>(sn + n);
+  for (int col = warp; col < n; col += JK_WARPS) {
+    double v = 0.0;
+    for (int i = lane; i < n; i += 32) v = fma(sX[col * P + i], sX[col * P + i], v);
+    v = wsum(v);
+    if (lane == 0) sn[col] = sqrt(v);
+  }
+  __syncthreads();
+  for (int col = tid; col < n; col += JK_THREADS) {
+    const double sj = sn[col];
+    int before = 0;
+    for (int k = 0; k < n; ++k) before += (sn[k] > sj) || (sn[k] == sj && k < col);
+    S[before] = sj;
+    pos[col] = before;
+  }
+  __syncthreads();
+  for (int col = warp; col < n; col += JK_WARPS) {
+    const double sj = sn[col];
+    const int at = pos[col];
+    for (int i = lane; i < n; i += 32) {
+      const double ua = sj > 0.0 ? sX[col * P + i] / sj : (i == at ? 1.0 : 0.0);
+      const double v = sX[col * P + np + i];
+      U[i + int64_t(at) * n] = trans ? v : ua;
+      VT[at + int64_t(i) * n] = trans ? ua : v;
     }
   }
-  al = gsum<G>(al);
-  be = gsum<G>(be);
-  ga = gsum<G>(ga);
-  // |ga| <= tol sqrt(al be), compared in squares (no square root on the
-  // path of a pair that needs no rotation)
-  const double ab = al * be, g2 = ga * ga;
-  if (!live || ab == 0.0 || g2 <= tol2 * ab) return off;
-  off = fmax(off, g2 / ab);
-  // t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)), zeta = (be - al) / (2 ga),
-  // written with one division: t = sign(zeta) |g| / (|dd| + hypot(dd, g))
-  // for dd = be - al, g = 2 ga (sign(zeta) = +1 when dd = 0).
-  const double dd = be - al, gg = 2.0 * ga;
-  const double sg = ((dd >= 0.0) == (gg > 0.0) || dd == 0.0) ? 1.0 : -1.0;
-  const double t = sg * fabs(gg) / (fabs(dd) + sqrt(dd * dd + gg * gg));
-  const double c = rsqrt(1.0 + t * t), s = c * t;
-  double* vp = V + int64_t(p) * n;
-  double* vq = V + int64_t(q) * n;
-  for (int i = gl; i < n; i += G) {
-    const double x = ap[i], y = aq[i];
-    ap[i] = c * x - s * y;
-    aq[i] = s * x + c * y;
-    const double vx = vp[i], vy = vq[i];
-    vp[i] = c * vx - s * vy;
-    vq[i] = s * vx + c * vy;
-  }
-  return off;
 }
+TTG_KERNEL(k_jacobi_svd, JK_THREADS);
+
 
 // Singular values = column norms of the rotated A, ranked descending
 // (stable on index); U = A diag(1/s), VT = V^T in that order.  With trans the
@@ -143,86 +398,6 @@ __device__ void jacobi_finish(int n, const double* A, const double* V, double* _
     }
   }
 }
-
-// A: n x n (column-major, lda) input; U (n x n, ld n), S (n), VT (n x n, ld n)
-// outputs.  work: n*n doubles of global scratch used when A does not fit in
-// shared memory.  Status: *err = 5 if the sweep limit is reached.
-TTG_BODY(k_jacobi_svd)(TTG_BLOCK, int n, const double* __restrict__ Ain,
-                                                          int lda, double* __restrict__ U,
-                                                          double* __restrict__ S,
-                                                          double* __restrict__ VT,
-                                                          double* __restrict__ Vg,
-                                                          double* __restrict__ work, int in_smem,
-                                                          int trans, int* err, int max_sweeps) {
-  pdl_begin();
-  extern __shared__ double sm[];
-  __shared__ double s_off[SD_WARPS];
-  __shared__ int s_done;
-  // in_smem: 0 = A and V in global memory, 1 = A in shared memory,
-  // 2 = A and V in shared memory.
-  double* A = in_smem ? sm : work;
-  double* V = in_smem == 2 ? sm + int64_t(n) * n : Vg;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < n * n; e += SD_THREADS) {
-    const int i = e % n, j = e / n;
-    A[e] = trans ? Ain[j + int64_t(i) * lda] : Ain[i + int64_t(j) * lda];
-    V[e] = (i == j) ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  const int ne = (n + 1) & ~1;  // even number of players (dummy column n if odd)
-  const double tol = 4.0 * 2.220446049250313e-16, tol2 = tol * tol;
-  int sweep = 0;
-  for (sweep = 0; sweep < max_sweeps; ++sweep) {
-    double off = 0.0;
-    for (int r = 0; r < ne - 1; ++r) {
-      if (ne / 2 > SD_WARPS && ne / 2 <= 2 * SD_WARPS) {
-        // 32 < pairs <= 64: one half-warp per pair, the whole round at once
-        // (a warp per pair would take two pairs in turn on most warps).
-        const int pr = tid >> 4;
-        int p = 0, q = 0;
-        bool live = false;
-        if (pr < ne / 2) {
-          p = rr_player(pr, r, ne);
-          q = rr_player(ne - 1 - pr, r, ne);
-          if (p > q) {
-            const int t = p;
-            p = q;
-            q = t;
-          }
-          live = q < n;  // else a dummy player
-          if (!live) p = q = 0;
-        }
-        off = jacobi_pair<16>(A, V, n, p, q, lane & 15, live, tol2, off);
-      } else {
-        for (int pr = warp; pr < ne / 2; pr += SD_WARPS) {
-          int p = rr_player(pr, r, ne), q = rr_player(ne - 1 - pr, r, ne);
-          if (p > q) {
-            const int t = p;
-            p = q;
-            q = t;
-          }
-          if (q >= n) continue;  // dummy player
-          off = jacobi_pair<32>(A, V, n, p, q, lane, true, tol2, off);
-        }
-      }
-      __syncthreads();
-    }
-    off = fmax(off, __shfl_xor_sync(0xffffffffu, off, 16));  // both half-warps
-    if (lane == 0) s_off[warp] = off;
-    __syncthreads();
-    if (tid == 0) {
-      double m = 0.0;
-      for (int w = 0; w < SD_WARPS; ++w) m = fmax(m, s_off[w]);
-      s_done = (m <= tol2) ? 1 : 0;
-    }
-    __syncthreads();
-    if (s_done) break;
-  }
-  if (tid == 0 && sweep >= max_sweeps) atomicExch(err, 5);
-  jacobi_finish(n, A, V, U, S, VT, work + int64_t(n) * n, trans);
-}
-TTG_KERNEL(k_jacobi_svd, SD_THREADS);
-
 
 // ---------------------------------------------------------------------------
 // Grid-wide one-sided Jacobi SVD for matrices too large for one CTA's shared
@@ -396,74 +571,6 @@ TTG_COOP_KERNEL(k_jacobi_coop, JC_THREADS);
 // running.
 // ---------------------------------------------------------------------------
 
-constexpr int JK_MAX_CS = 16;          // CTAs of a cluster
-constexpr int JK_W = 8;                // columns of a block
-constexpr int JK_COLS = 2 * JK_W;      // columns of a CTA
-constexpr int JK_MAX_N = JK_MAX_CS * JK_COLS;
-constexpr int JK_THREADS = 512;
-constexpr int JK_WARPS = JK_THREADS / 32;
-constexpr int JK_GP = JK_COLS + 1;     // pitch of the Gram matrix
-constexpr int JK_JP = JK_COLS + 4;     // pitch of J (mma operand: 4 mod 16)
-
-// Rows of a column's A (or V) part, and column pitches in global and shared
-// memory (the latter 4 mod 16, so that mma fragments meet no bank twice).
-__host__ __device__ __forceinline__ int jk_rows(int n) { return (n + 7) & ~7; }
-__host__ __device__ __forceinline__ int jk_pitch(int n) {
-  return ((2 * jk_rows(n) + 15) & ~15) + 4;
-}
-int jk_blocks(int64_t n) { return int((n + JK_COLS - 1) / JK_COLS) * 2; }
-int64_t jk_work(int64_t n) {  // columns, then the column norms
-  return int64_t(jk_blocks(n)) * JK_W * (2 * jk_rows(int(n)) + 1);
-}
-size_t jk_smem(int64_t n) {
-  return sizeof(double) * (size_t(JK_COLS) * jk_pitch(int(n)) + JK_WARPS * 192 + JK_COLS * JK_GP +
-                           JK_COLS * JK_JP);
-}
-
-// Blocks of CTA c in round r of a tournament on nb (even) blocks: block nb - 1
-// is fixed and meets r, the others pair as p + q = 2 r (mod nb - 1).
-__device__ __forceinline__ void jk_pair(int c, int r, int nb, int& p, int& q) {
-  const int m = nb - 1;
-  if (c == 0) {
-    p = r;
-    q = m;
-    return;
-  }
-  p = r + c;
-  if (p >= m) p -= m;
-  q = r - c;
-  if (q < 0) q += m;
-}
-
-// Cosine and sine of the rotation that makes a pair orthogonal, the smaller of
-// the two angles: with dd = be - al, g = 2 ga and h = hypot(dd, g),
-// c = sqrt((1 + |dd| / h) / 2) and s = |g| / (2 h c) with the sign of dd g.
-// They are first taken in single precision (dd and g scaled to a common
-// exponent), which leaves 1e-7 of the pair's inner product for the next sweep,
-// then both multiplied by 1 / sqrt(c^2 + s^2) in double precision (two terms
-// of the series: c^2 + s^2 - 1 is 1e-7), which leaves the rounding of c and s
-// alone.  c = 1 / sqrt(1 + t^2) taken directly is biased by 1e-16 for small t,
-// which adds up over a sweep's thousands of rotations.
-__device__ __forceinline__ void jk_rotation(double al, double be, double ga, double& c,
-                                            double& s) {
-  const double dd = be - al, gg = 2.0 * ga;
-  // 2^-e for the exponent e of |dd| + |g|
-  const int field = 0x7fe00000 - (__double2hiint(fabs(dd) + fabs(gg)) & 0x7ff00000);
-  const double scale = __hiloint2double(field, 0);
-  const double y = fabs(gg) * scale;
-  const float x = float(fabs(dd) * scale), yf = float(y);
-  const float rh = rsqrtf(fmaf(x, x, yf * yf));
-  const float v = fmaf(0.5f * x, rh, 0.5f);  // c^2
-  const float rv = rsqrtf(v);
-  const double c0 = double(v * rv);
-  const double s0 = (0.5 * y) * double(rh * rv);
-  const double d = fma(s0, s0, fma(c0, c0, -1.0));
-  const double f = d * fma(0.375, d, -0.5);
-  c = fma(c0, f, c0);
-  s = fma(s0, f, s0);
-  if ((dd >= 0.0) != (gg > 0.0) && dd != 0.0) s = -s;
-}
-
 __global__ void __launch_bounds__(JK_THREADS, 1)
     k_jacobi_cluster(int n, const double* __restrict__ Ain, int lda, int trans, double* X,
                      double* __restrict__ U, double* __restrict__ S, double* __restrict__ VT,
@@ -473,8 +580,6 @@ __global__ void __launch_bounds__(JK_THREADS, 1)
   extern __shared__ __align__(16) double sm[];
   __shared__ int s_rot[2][JK_MAX_CS];  // rank 0: whether a CTA found a pair, by sweep parity
   __shared__ int s_any;                // this round rotated
-  __shared__ __align__(16) double2 s_cs[JK_COLS - 1][JK_W];  // rotations of a round's steps
-  __shared__ int s_rots[JK_COLS - 1];  // whether a step rotates
   const int rank = int(cl.block_rank()), cs = int(cl.num_blocks());
   const int np = jk_rows(n), ldx = 2 * np, P = jk_pitch(n);
   const int nb = 2 * ((n + JK_COLS - 1) / JK_COLS);
@@ -546,91 +651,10 @@ __global__ void __launch_bounds__(JK_THREADS, 1)
             sG[row * JK_GP + col] = sG[col * JK_GP + row] = (v[0] + v[1]) + (v[2] + v[3]);
         }
         __syncthreads();
-        // Rotations, eight disjoint pairs at a time: warp 0 on G, warp 1 behind
-        // it on J (a named barrier per step, at which warp 0 only arrives).
-        if (warp < 2) {
-          const int steps = r == 0 ? JK_COLS - 1 : JK_W;
-          int any = 0;
-          for (int ir = 0; ir < steps; ++ir) {
-            auto pair = [&](int k, int& p, int& q) {
-              if (r == 0) {  // all pairs of 16 columns
-                p = rr_player(k, ir, JK_COLS);
-                q = rr_player(JK_COLS - 1 - k, ir, JK_COLS);
-              } else {  // pairs across the blocks
-                p = k;
-                q = JK_W + ((k + ir) & (JK_W - 1));
-              }
-            };
-            if (warp == 0) {
-              int p, q;
-              pair(lane & 7, p, q);
-              const double al = sG[p * JK_GP + p], be = sG[q * JK_GP + q],
-                           ga = sG[p * JK_GP + q];
-              // the lane's 2 x 2 blocks of G: pair a by pairs b and b + 4
-              const int a = lane >> 2;
-              int pa, qa, pb[2], qb[2];
-              pair(a, pa, qa);
-              pair(lane & 3, pb[0], qb[0]);
-              pair((lane & 3) + 4, pb[1], qb[1]);
-              double x[2][4];
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                x[h][0] = sG[pa * JK_GP + pb[h]];
-                x[h][1] = sG[pa * JK_GP + qb[h]];
-                x[h][2] = sG[qa * JK_GP + pb[h]];
-                x[h][3] = sG[qa * JK_GP + qb[h]];
-              }
-              double c, sn;
-              jk_rotation(al, be, ga, c, sn);
-              const double ab = al * be;
-              const bool rot = ab != 0.0 && ga * ga > tol2 * ab;
-              if (!rot) {
-                c = 1.0;
-                sn = 0.0;
-              }
-              const int rots = __any_sync(0xffffffffu, rot);
-              if (lane < JK_W) s_cs[ir][lane] = make_double2(c, sn);
-              if (lane == 0) s_rots[ir] = rots;
-              const double ca = __shfl_sync(0xffffffffu, c, a);
-              const double sa = __shfl_sync(0xffffffffu, sn, a);
-              // columns p, q <- c p - s q, s p + c q, on both sides of G
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const double cb = __shfl_sync(0xffffffffu, c, (lane & 3) + 4 * h);
-                const double sb = __shfl_sync(0xffffffffu, sn, (lane & 3) + 4 * h);
-                const double y00 = fma(cb, x[h][0], -sb * x[h][1]);
-                const double y01 = fma(sb, x[h][0], cb * x[h][1]);
-                const double y10 = fma(cb, x[h][2], -sb * x[h][3]);
-                const double y11 = fma(sb, x[h][2], cb * x[h][3]);
-                sG[pa * JK_GP + pb[h]] = fma(ca, y00, -sa * y10);
-                sG[pa * JK_GP + qb[h]] = fma(ca, y01, -sa * y11);
-                sG[qa * JK_GP + pb[h]] = fma(sa, y00, ca * y10);
-                sG[qa * JK_GP + qb[h]] = fma(sa, y01, ca * y11);
-              }
-              any |= rots;
-              __syncwarp();
-              asm volatile("bar.arrive %0, 64;" ::"r"(ir + 1) : "memory");
-            } else {
-              asm volatile("bar.sync %0, 64;" ::"r"(ir + 1) : "memory");
-              if (!s_rots[ir]) continue;
-              double* row = sJ + (lane & 15) * JK_JP;
-#pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                const int k = (lane >> 4) * 4 + h;
-                int p, q;
-                pair(k, p, q);
-                const double2 rk = s_cs[ir][k];
-                const double xp = row[p], xq = row[q];
-                row[p] = fma(rk.x, xp, -rk.y * xq);
-                row[q] = fma(rk.y, xp, rk.x * xq);
-              }
-              __syncwarp();
-            }
-          }
-          if (warp == 0) {
-            found |= any;
-            if (lane == 0) s_any = any;
-          }
+        if (warp == 0) {
+          const int any = jk_rotate(sG, sJ, r == 0, tol2);
+          found |= any;
+          if (lane == 0) s_any = any;
         }
         cp_async_wait<0>();
         __syncthreads();
@@ -1675,10 +1699,9 @@ void jacobi_svd_f64(Context* c, int64_t n, const double* A, int64_t lda, double*
                     double* VT, bool via_transpose) {
   int trans = via_transpose ? 1 : 0;
   TTG_REQUIRE(n >= 1 && n <= 4096, "jacobi_svd: n = %lld out of range", (long long)n);
-  const size_t mat = size_t(n * n) * sizeof(double);
-  const int mode = 2 * mat <= SMEM_LIMIT ? 2 : (mat <= SMEM_LIMIT ? 1 : 0);
-  const bool block = mode == 0 && jacobi_block_fits(n);
-  if (!block && (mode == 0 || mode == 1 || (!c->rec && n >= jacobi_cluster_min_n())) &&
+  const bool one_cta = n <= JS_MAX_N;
+  const bool block = n > 160 && jacobi_block_fits(n);
+  if (!block && (!one_cta || (!c->rec && n >= jacobi_cluster_min_n())) &&
       jacobi_cluster_ok(c, n)) {
     // One cluster, the columns in L2.
     DBuf<double> X(c, jk_work(n));
@@ -1698,6 +1721,13 @@ void jacobi_svd_f64(Context* c, int64_t n, const double* A, int64_t lda, double*
       issue(c->stream);
     }
     c->launches += 1;
+    TTG_CHECK_LAUNCH();
+    return;
+  }
+  if (one_cta) {
+    ensure_smem_attr(k_jacobi_svd.fn(), c->device, int(js_smem(JS_MAX_N)));
+    launch(c, k_jacobi_svd, 1, JK_THREADS, js_smem(n), int(n), A, int(lda), U, S, VT, trans,
+           c->d_err + 3, c->jacobi_max_sweeps);
     TTG_CHECK_LAUNCH();
     return;
   }
@@ -1722,29 +1752,20 @@ void jacobi_svd_f64(Context* c, int64_t n, const double* A, int64_t lda, double*
     TTG_CHECK_LAUNCH();
     return;
   }
-  if (mode != 2) {
-    // Grid-wide rounds: one CTA per column pair (up to what fits at once).
-    int occ = 0;
-    TTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jacobi_coop.plain(),
-                                                           JC_THREADS, 0));
-    const int64_t pairs = (n + 1) / 2;
-    const int blocks = int(std::max<int64_t>(1, std::min<int64_t>(pairs,
-                                                                  int64_t(c->num_sms) * occ)));
-    DBuf<unsigned> bar(c, 2);
-    DBuf<unsigned long long> offmax(c, 3);
-    memset_async(c, bar.p(), 0, 2 * sizeof(unsigned));
-    launch(c, k_jacobi_coop, blocks, JC_THREADS, 0, int(n), A, int(lda), work.p(), V.p(),
-           bar.p(), offmax.p(), c->d_err + 0, c->d_err + 3, trans, c->jacobi_max_sweeps);
-    launch(c, k_jacobi_finish, 1, SD_THREADS, 0, int(n), work.p(), V.p(), U, S, VT,
-           work.p() + int64_t(n) * n, trans);
-    TTG_CHECK_LAUNCH();
-    return;
-  }
-  ensure_smem_attr(k_jacobi_svd.fn(), c->device,
-                   int(SMEM_LIMIT + 1024));
-  const size_t smem = size_t(mode) * mat;
-  launch(c, k_jacobi_svd, 1, SD_THREADS, smem, int(n), A, int(lda), U, S, VT, V.p(), work.p(),
-         mode, trans, c->d_err + 3, c->jacobi_max_sweeps);
+  // Grid-wide rounds: one CTA per column pair (up to what fits at once).
+  int occ = 0;
+  TTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jacobi_coop.plain(), JC_THREADS,
+                                                         0));
+  const int64_t pairs = (n + 1) / 2;
+  const int blocks =
+      int(std::max<int64_t>(1, std::min<int64_t>(pairs, int64_t(c->num_sms) * occ)));
+  DBuf<unsigned> bar(c, 2);
+  DBuf<unsigned long long> offmax(c, 3);
+  memset_async(c, bar.p(), 0, 2 * sizeof(unsigned));
+  launch(c, k_jacobi_coop, blocks, JC_THREADS, 0, int(n), A, int(lda), work.p(), V.p(), bar.p(),
+         offmax.p(), c->d_err + 0, c->d_err + 3, trans, c->jacobi_max_sweeps);
+  launch(c, k_jacobi_finish, 1, SD_THREADS, 0, int(n), work.p(), V.p(), U, S, VT,
+         work.p() + int64_t(n) * n, trans);
   TTG_CHECK_LAUNCH();
 }
 
