@@ -981,6 +981,298 @@ TTG_KERNEL(k_house_qr, SD_THREADS);
 
 
 // ---------------------------------------------------------------------------
+// Blocked Householder QR in one CTA (LAPACK's reflectors and signs), for
+// matrices that fit in shared memory with their rows and columns padded to 8.
+// A panel of 8 columns takes one barrier and one block-wide reduction per
+// column: the inner products of the column with itself and with the panel's
+// later columns are summed in one pass, together with the update by the
+// previous reflector, and give the norm and all coefficients at once (the
+// reflector is x scaled below the diagonal, so v'a = a_j + scal x'a).  The
+// panel's reflectors then act on the columns behind it as I - V T V' (mma),
+// and in reverse order on I's columns to form Q.
+// Bound by the chain of columns, 1.6 us each with Q: 54 x 54 104 us for 178 with
+// one reflector at a time and four barriers each, 198 x 54 125 / 255, 200 x 100
+// 240 / 623, 1600 x 15 72 / 168; residual and orthogonality as before.
+// ---------------------------------------------------------------------------
+
+constexpr int QB_THREADS = 512;
+constexpr int QB_WARPS = QB_THREADS / 32;
+constexpr int QB_WP = 12;  // pitch of the 8-row coefficient columns (mma operand)
+constexpr size_t QB_SMEM = 224 * 1024;  // beside 3 KB of static arrays
+
+// Column pitch: at least m rounded to 8, and 4 mod 16.
+__host__ __device__ __forceinline__ int64_t qb_pitch(int64_t m) {
+  const int64_t mp = (m + 7) & ~int64_t(7);
+  return mp + ((20 - mp % 16) & 15);
+}
+// Columns (and 8 more for the reflectors of a wide matrix, whose last panel may
+// end inside a tile), T, and the coefficients; the partial tiles share the
+// second coefficient array.
+size_t qb_smem(int64_t m, int64_t n) {
+  const int64_t np = (n + 7) & ~int64_t(7), kb = (std::min(m, n) + 7) / 8;
+  return sizeof(double) * size_t((np + (n > m ? 8 : 0)) * qb_pitch(m) + 64 * kb + QB_WP * (np + 8) +
+                                 std::max<int64_t>(QB_WP * (np + 8), 64 * QB_WARPS));
+}
+
+// Sums of eight values over a warp, value 4 b4 + 2 b3 + b2 in the lanes with
+// those bits of their index (b4 highest).
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int half = 4; half >= 1; half >>= 1) {
+    const bool hi = lane & (4 * half);
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double send = hi ? v[i] : v[i + half], keep = hi ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * half);
+    }
+  }
+  double r = v[0];
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  return r;
+}
+
+TTG_BODY(k_house_qr_blk)(TTG_BLOCK, int m, int n, const double* __restrict__ Ain, int lda,
+                         double* __restrict__ Q, double* __restrict__ R, const int* skip) {
+  pdl_begin();
+  if (skip && *skip) return;  // conditional factorization (Context::skip)
+  extern __shared__ __align__(16) double sm[];
+  __shared__ double s_part[2][QB_WARPS][8];
+  __shared__ double s_r[8][8];  // the panel's rows of R
+  __shared__ double s_tau[8];
+  const int k = m < n ? m : n, mp = (m + 7) & ~7, np = (n + 7) & ~7, kb = (k + 7) / 8;
+  const int P = int(qb_pitch(m));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  double* sA = sm;                        // np columns
+  // A panel's reflectors, explicit (unit lower trapezoidal): in their columns'
+  // place, or apart in a wide matrix.
+  const bool apart = n > m;
+  double* sT = sA + (np + (apart ? 8 : 0)) * P;  // T of every panel, 8 x 8 column-major
+  double* sW = sT + 64 * kb;              // V'A: columns of 8 (pitch QB_WP)
+  double* sW2 = sW + QB_WP * (np + 8);    // T'V'A or T V'A
+  double* sK = sW2;                       // partial tiles of the warps
+  double* sV = sA + np * P;
+  for (int c = warp; c < np; c += QB_WARPS)
+    for (int i = lane; i < mp; i += 32)
+      sA[c * P + i] = c < n && i < m ? Ain[i + int64_t(c) * lda] : 0.0;
+
+  auto explicit_v = [&](int j0, int pw) {
+    if (!apart) {  // only the block on the diagonal holds anything else (R)
+      sV = sA + j0 * P;
+      if (tid < 64 && (tid & 7) <= tid >> 3)
+        sV[(tid >> 3) * P + j0 + (tid & 7)] = (tid & 7) == tid >> 3 && tid >> 3 < pw;
+      return;
+    }
+    for (int c = warp >> 1; c < 8; c += QB_WARPS / 2)
+      for (int i = j0 + lane + 32 * (warp & 1); i < mp; i += 64) {
+        const int d = i - j0 - c;
+        sV[c * P + i] = c < pw && d >= 0 ? (d == 0 ? 1.0 : sA[(j0 + c) * P + i]) : 0.0;
+      }
+  };
+  // sW = V' [V | A(:, c0 ..)] over the rows from j0 on: 1 + nt tiles of 8
+  // columns, K split over the warps where there are fewer tiles than warps.
+  auto project = [&](int j0, int c0, int nt) {
+    const int tiles = 1 + nt, wpt = tiles < QB_WARPS ? QB_WARPS / tiles : 1;
+    for (int u = warp; u < tiles * wpt; u += QB_WARPS) {
+      const int tile = u / wpt;
+      const double* b = tile == 0 ? sV : sA + (c0 + 8 * (tile - 1)) * P;
+      // four chains: shorter sums round less, and run side by side
+      double x[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+      for (int k4 = j0 / 4 + u % wpt; k4 < mp / 4; k4 += 4 * wpt)
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (k4 + h * wpt < mp / 4) {
+            const int i = g * P + 4 * (k4 + h * wpt) + t;
+            dmma(x[h][0], x[h][1], sV[i], b[i]);
+          }
+      const double x0 = (x[0][0] + x[1][0]) + (x[2][0] + x[3][0]);
+      const double x1 = (x[0][1] + x[1][1]) + (x[2][1] + x[3][1]);
+      if (wpt == 1) {
+        sW[(8 * tile + 2 * t) * QB_WP + g] = x0;
+        sW[(8 * tile + 2 * t + 1) * QB_WP + g] = x1;
+      } else {  // u == warp: one slot per warp
+        sK[u * 64 + 16 * t + g] = x0;
+        sK[u * 64 + 16 * t + 8 + g] = x1;
+      }
+    }
+    __syncthreads();
+    if (wpt > 1) {
+      for (int e = tid; e < tiles * 64; e += QB_THREADS) {
+        const int tile = e / 64, el = e % 64;
+        double v = 0.0;
+        for (int w = 0; w < wpt; ++w) v += sK[(tile * wpt + w) * 64 + el];
+        sW[(8 * tile + el / 8) * QB_WP + el % 8] = v;
+      }
+      __syncthreads();
+    }
+  };
+  // Tiles of A -= V w2 for the columns from c0 on (nt tiles), rows from j0 on;
+  // with `fresh` the columns start as those of I instead of A's (the panel's
+  // own, where a tile of V is read by the warp that replaces it).
+  auto apply = [&](int j0, int c0, int nt, const double* w2, bool fresh) {
+    const int r0 = j0 / 8, rows = mp / 8 - r0;
+    for (int u = warp; u < nt * rows; u += QB_WARPS) {
+      const int ct = u / rows, rt = r0 + u % rows;
+      double* M = sA + (c0 + 8 * ct) * P + 8 * rt;
+      double x0 = M[2 * t * P + g], x1 = M[(2 * t + 1) * P + g], a[2];
+      if (fresh) {
+        x0 = rt == r0 && g == 2 * t ? 1.0 : 0.0;
+        x1 = rt == r0 && g == 2 * t + 1 ? 1.0 : 0.0;
+      }
+#pragma unroll
+      for (int s = 0; s < 2; ++s) a[s] = -sV[(4 * s + t) * P + 8 * rt + g];
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < 2; ++s) dmma(x0, x1, a[s], w2[(8 * ct + g) * QB_WP + 4 * s + t]);
+      M[2 * t * P + g] = x0;
+      M[(2 * t + 1) * P + g] = x1;
+    }
+  };
+
+  for (int p = 0; p < kb; ++p) {
+    const int j0 = 8 * p, pw = min(8, k - j0);
+    __syncthreads();  // loaded, or updated by the previous panel
+    double* A0 = sA + j0 * P;
+    double v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = 0.0;
+    for (int i = tid; i < m; i += QB_THREADS) {
+      if (i <= j0) continue;
+      const double x = A0[i];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = fma(x, A0[c * P + i], v[c]);
+    }
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) {
+      if (jj >= pw) break;
+      const int j = j0 + jj;
+      // inner products of column jj, below its diagonal, with columns jj .. 7
+      {
+        const double s = warp_sum8(v, lane);
+        const int idx = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+        if ((lane & 3) == 0) s_part[jj & 1][warp][idx] = s;
+      }
+      __syncthreads();  // and the rows updated by reflector jj - 1 are written
+      double d = 0.0;
+#pragma unroll
+      for (int w = 0; w < QB_WARPS; w += 4) d += s_part[jj & 1][w + (lane >> 3)][lane & 7];
+      d += __shfl_xor_sync(0xffffffffu, d, 8);
+      d += __shfl_xor_sync(0xffffffffu, d, 16);
+      const double tt = __shfl_sync(0xffffffffu, d, jj);
+      const double alpha = A0[jj * P + j];
+      double beta = alpha, tau = 0.0, scal = 0.0;
+      if (tt != 0.0) {
+        beta = -copysign(sqrt(alpha * alpha + tt), alpha);
+        scal = 1.0 / (alpha - beta);
+        tau = (beta - alpha) / beta;
+      }
+      double w[8];
+#pragma unroll
+      for (int c = jj + 1; c < 8; ++c) {
+        const double a = A0[c * P + j];
+        w[c] = tau * fma(scal, __shfl_sync(0xffffffffu, d, c), a);
+        if (tid == 0) s_r[jj][c] = a - w[c];
+      }
+      if (tid == 0) {
+        s_r[jj][jj] = beta;
+        s_tau[jj] = tau;
+      }
+      // the reflector, the update of the later columns, and the inner products
+      // of the next column
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = 0.0;
+      for (int i = tid; i < m; i += QB_THREADS) {
+        if (i <= j) continue;
+        const double x = A0[jj * P + i] * scal;
+        A0[jj * P + i] = x;
+        double a[8];
+#pragma unroll
+        for (int c = jj + 1; c < 8; ++c) {
+          a[c] = fma(-w[c], x, A0[c * P + i]);
+          A0[c * P + i] = a[c];
+        }
+        if (jj < 7 && i > j + 1) {
+#pragma unroll
+          for (int c = jj + 1; c < 8; ++c) v[c] = fma(a[jj + 1 < 8 ? jj + 1 : 7], a[c], v[c]);
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < 64) {  // the panel's block of R
+      const int i = tid & 7, c = tid >> 3;
+      if (i < pw && j0 + c < n)
+        R[j0 + i + int64_t(j0 + c) * k] = c >= i ? s_r[i][c] : 0.0;
+    }
+    explicit_v(j0, pw);
+    __syncthreads();
+    const int c0 = j0 + 8, nt = (np - c0) / 8;
+    project(j0, c0, nt);
+    if (warp == 0) {  // T(0:j, j) = -tau_j T(0:j, 0:j) V'v_j, row `lane`
+      double T[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const double tau = j < pw ? s_tau[j] : 0.0;
+        double x = 0.0;
+#pragma unroll
+        for (int l = 0; l < j; ++l) x = fma(T[l], sW[j * QB_WP + l], x);
+        T[j] = lane == j ? tau : (lane < j ? -tau * x : 0.0);
+        if (lane < 8) sT[64 * p + 8 * j + lane] = T[j];
+      }
+    }
+    __syncthreads();
+    for (int e = tid; e < 64 * nt; e += QB_THREADS) {  // T' (V'A)
+      const int c = e / 8, i = e % 8;
+      double x = 0.0;
+#pragma unroll
+      for (int l = 0; l < 8; ++l)
+        if (l <= i) x = fma(sT[64 * p + 8 * i + l], sW[(8 + c) * QB_WP + l], x);
+      sW2[c * QB_WP + i] = x;
+    }
+    __syncthreads();
+    apply(j0, c0, nt, sW2, false);
+  }
+  __syncthreads();
+  // The rest of R: above each panel's block, and zeros below.
+  for (int c = warp; c < n; c += QB_WARPS) {
+    const int b0 = min(c & ~7, 8 * kb);
+    for (int i = lane; i < k; i += 32)
+      if (i < b0 || i >= b0 + 8) R[i + int64_t(c) * k] = i < b0 ? sA[c * P + i] : 0.0;
+  }
+  // Q = (I - V_0 T_0 V_0') ... I, the last panel first: a panel acts on the
+  // columns behind it, which hold Q's already, and replaces its own.
+  const int qc = 8 * kb;
+  for (int p = kb - 1; p >= 0; --p) {
+    const int j0 = 8 * p, pw = min(8, k - j0);
+    __syncthreads();
+    explicit_v(j0, pw);
+    __syncthreads();
+    const int c0 = j0 + 8, nt = (qc - c0) / 8;
+    project(j0, c0, nt);
+    for (int e = tid; e < 64 * (nt + 1); e += QB_THREADS) {
+      const int c = e / 8, i = e % 8;
+      double x = 0.0;
+#pragma unroll
+      for (int l = 0; l < 8; ++l) {
+        const double b = c < 8 ? sV[l * P + j0 + c] : sW[c * QB_WP + l];
+        if (l >= i) x = fma(sT[64 * p + 8 * l + i], b, x);
+      }
+      sW2[c * QB_WP + i] = x;
+    }
+    for (int c = warp; c < 8; c += QB_WARPS)  // Q's rows above the panel's
+      for (int i = lane; i < j0; i += 32) sA[(j0 + c) * P + i] = 0.0;
+    __syncthreads();
+    apply(j0, c0, nt, sW2 + 8 * QB_WP, false);
+    __syncthreads();
+    apply(j0, j0, 1, sW2, true);
+  }
+  __syncthreads();
+  for (int c = warp; c < k; c += QB_WARPS)
+    for (int i = lane; i < m; i += 32) Q[i + int64_t(c) * m] = sA[c * P + i];
+}
+TTG_KERNEL(k_house_qr_blk, QB_THREADS);
+
+// ---------------------------------------------------------------------------
 // Householder QR of a skinny m x n matrix (n <= SK_MAX_N) too tall for shared
 // memory: the work copy W lives in global memory (L2), every thread owns the
 // rows i = tid (mod SD_THREADS), and each reflector needs two block-wide
@@ -1588,6 +1880,15 @@ bool small_qr_fits(int64_t m, int64_t n) {
 
 void small_qr_f64(Context* c, int64_t m, int64_t n, const double* A, int64_t lda, double* Q,
                   double* R) {
+  // The blocked kernel where its padded columns fit (the element-wise one is
+  // left with shapes like 4 x 5000 and 20000 x 1).
+  if (qb_smem(m, n) <= QB_SMEM) {
+    ensure_smem_attr(k_house_qr_blk.fn(), c->device, int(QB_SMEM));
+    launch(c, k_house_qr_blk, 1, QB_THREADS, qb_smem(m, n), int(m), int(n), A, int(lda), Q, R,
+           c->skip);
+    TTG_CHECK_LAUNCH();
+    return;
+  }
   const size_t smem = sizeof(double) * size_t(m * n + std::min(m, n));
   ensure_smem_attr(k_house_qr.fn(), c->device, int(SMEM_LIMIT + 1024));
   launch(c, k_house_qr, 1, SD_THREADS, smem, int(m), int(n), A, int(lda), Q, R, c->skip);
