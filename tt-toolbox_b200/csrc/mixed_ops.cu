@@ -224,6 +224,190 @@ const GroupInfo* umma_info() {
 }
 
 // ---------------------------------------------------------------------------
+// Persistent form of the GEMM for products of many tiles: one CTA per SM walks
+// its tiles of 128 x BN; warp 0 streams TMA tiles into a shared-memory ring
+// across tile boundaries, one thread of warp 1 issues tcgen05.mma into one of
+// two TMEM accumulators, and warps 2-9 drain the other.  The plain form's
+// narrow tiles hide their epilogues behind other CTAs but load (128 + BN)
+// operand rows from L2 for every 128 x BN products, and L2 bounds it: at 512 x
+// 64 x 512, ranks 3, its stages move 1.2, 0.3 and 0.8 GB at 8-9 TB/s.  Tiles of
+// 256 halve that.  127, 127 and 104 us of the plain form become 89, 89 and 60
+// there (865 TFLOP/s for the last stage), bit for bit.
+// Every wait is bounded: a timeout raises the error flag and every role winds
+// down.
+// ---------------------------------------------------------------------------
+
+constexpr int PS_THREADS = 320;
+constexpr int PS_EPI_WARPS = 8;
+template <int BN>
+constexpr int ps_stages() {
+  return 192 * 1024 / (UM_A_BYTES + BN * UM_BK * 2);
+}
+template <int BN>
+constexpr size_t ps_smem_bytes() {
+  return 1024 + size_t(ps_stages<BN>()) * (UM_A_BYTES + BN * UM_BK * 2) +
+         (2 * ps_stages<BN>() + 4) * 8 + 64;
+}
+
+template <int BN, bool OUT_BF16>
+__global__ void __launch_bounds__(PS_THREADS, 1)
+    k_umma_pers(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                int K, int a_rows_pb, int b_rows_pb, OutMap om, int mt, int nt, int ntiles,
+                int* err, const int* skip) {
+  pdl_begin();
+  using namespace umma;
+  if (skip && *skip) return;  // queued Krylov step after convergence (uniform)
+  constexpr int ST = ps_stages<BN>();
+  constexpr int B_BYTES = BN * UM_BK * 2;
+  constexpr uint32_t ACC = BN <= 128 ? 128 : 256;  // TMEM columns of an accumulator
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + ST * UM_A_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sB + ST * B_BYTES);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 4);
+  uint32_t* consumed_slot = tmem_slot + 1;
+  const uint32_t bar_full = smem_u32(bars);
+  const uint32_t bar_empty = smem_u32(bars + ST);
+  const uint32_t bar_accf = smem_u32(bars + 2 * ST);      // 2: accumulator ready
+  const uint32_t bar_acce = smem_u32(bars + 2 * ST + 2);  // 2: accumulator drained
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nk = (K + UM_BK - 1) / UM_BK;
+
+  if (warp == 0) {
+    tmem_alloc(smem_u32(tmem_slot), 2 * ACC);
+    tmem_relinquish();
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(bar_full + 8 * s, 1);
+      mbar_init(bar_empty + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(bar_accf + 8 * b, 1);
+      mbar_init(bar_acce + 8 * b, PS_EPI_WARPS);  // one arrival per epilogue warp
+    }
+    *consumed_slot = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  uint32_t kb_cnt = 0;    // K-blocks issued (producer) / consumed (MMA)
+  uint32_t tile_cnt = 0;  // tiles accumulated (MMA) / drained (epilogue)
+  // Tile t: the column tiles of a row tile follow one another, so that CTAs
+  // that run together share its operand rows.
+  if (warp == 0) {
+    if (lane == 0) {  // TMA producer
+      bool ok = true;
+      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+        const int ni = t % nt, mi = t / nt % mt, bz = t / nt / mt;
+        const int arow = bz * a_rows_pb + mi * UM_BM, brow = bz * b_rows_pb + ni * BN;
+        for (int kb = 0; kb < nk; ++kb, ++kb_cnt) {
+          const uint32_t slot = kb_cnt % ST;
+          if (kb_cnt >= ST && !mbar_wait(bar_empty + 8 * slot, ((kb_cnt / ST) - 1) & 1, err)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(bar_full + 8 * slot, UM_A_BYTES + B_BYTES);
+          tma_load_2d(smem_u32(sA + slot * UM_A_BYTES), &tmA, kb * UM_BK, arow,
+                      bar_full + 8 * slot);
+          tma_load_2d(smem_u32(sB + slot * B_BYTES), &tmB, kb * UM_BK, brow, bar_full + 8 * slot);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {  // MMA issuer
+      const uint32_t idesc = idesc_bf16_f32(UM_BM, BN);
+      bool ok = true;
+      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++tile_cnt) {
+        const uint32_t buf = tile_cnt & 1;
+        if (tile_cnt >= 2 && !mbar_wait(bar_acce + 8 * buf, ((tile_cnt >> 1) - 1) & 1, err)) break;
+        tc_fence_after();
+        const uint32_t tacc = tmem + buf * ACC;
+        for (int kb = 0; kb < nk; ++kb, ++kb_cnt) {
+          const uint32_t slot = kb_cnt % ST;
+          if (!mbar_wait(bar_full + 8 * slot, (kb_cnt / ST) & 1, err)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(sA + slot * UM_A_BYTES), b0 = smem_u32(sB + slot * B_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < UM_BK / 16; ++kk)
+            mma_bf16(tacc, desc_k_sw128(a0 + kk * 32), desc_k_sw128(b0 + kk * 32), idesc,
+                     (kb > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(bar_empty + 8 * slot);
+        }
+        if (ok) mma_commit(bar_accf + 8 * buf);
+      }
+      *consumed_slot = kb_cnt;
+    }
+    __syncwarp();
+  } else {  // epilogue: warp w owns TMEM lanes 32 (w % 4) .., every other 16 columns
+    const int ew = warp & 3, half = (warp - 2) >> 2;
+    const int row = ew * 32 + lane;
+    const unsigned r_s1 = unsigned(om.r_s1), c_s1 = unsigned(om.c_s1);
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tile_cnt) {
+      const uint32_t buf = tile_cnt & 1;
+      const int ni = t % nt, mi = t / nt % mt, bz = t / nt / mt;
+      const unsigned m = unsigned(mi * UM_BM + row);
+      const bool row_ok = m < om.M;
+      const int64_t base = int64_t(bz) * om.batch_stride + int64_t(m % r_s1) * om.r_t1 +
+                           int64_t(m / r_s1) * om.r_t2;
+      const bool ok = mbar_wait(bar_accf + 8 * buf, (tile_cnt >> 1) & 1, err);
+      tc_fence_after();
+      if (!ok) break;
+      const uint32_t tbase = tmem + (uint32_t(ew * 32) << 16) + buf * ACC;
+#pragma unroll 1
+      for (int c0 = 16 * half; c0 < BN; c0 += 32) {
+        const unsigned n0 = unsigned(ni * BN + c0);
+        if (n0 >= om.N) break;  // uniform across the warp
+        float v[16];
+        tmem_ld16(tbase + uint32_t(c0), v);
+        unsigned cr = n0 % c_s1;
+        int64_t off = base + int64_t(cr) * om.c_t1 + int64_t(n0 / c_s1) * om.c_t2;
+        const int left = int(om.N - n0);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (row_ok && j < left) {
+            if (OUT_BF16)
+              static_cast<__nv_bfloat16*>(om.base)[off] = __float2bfloat16_rn(v[j]);
+            else
+              static_cast<float*>(om.base)[off] = v[j];
+          }
+          off += om.c_t1;
+          if (++cr == c_s1) {
+            cr = 0;
+            off += om.c_t2 - om.c_s1 * om.c_t1;
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_acce + 8 * buf);
+    }
+  }
+  __syncthreads();
+  // Wind-down after an error: loads issued but never consumed must land
+  // before the CTA (and its shared memory) goes away.  Bounded.
+  if (threadIdx.x == 0 && *(volatile int*)err) {
+    for (uint32_t k = *consumed_slot; k < kb_cnt; ++k)
+      mbar_wait(bar_full + 8 * (k % ST), (k / ST) & 1, err, 1 << 16);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 2 * ACC);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Fused local matvec: the three GEMM stages in ONE persistent launch.
 //
 // One CTA per SM (cooperative launch, so all CTAs are resident) walks the
@@ -678,10 +862,37 @@ void launch_bn(Context* c, const CUtensorMap& ta, const CUtensorMap& tb, int64_t
   TTG_CHECK_LAUNCH();
 }
 
+// A tile width with this flag names the persistent form (never in a grouped
+// batch, whose launches share the device).
+constexpr int BN_PERS = 1024;
+
+int64_t umma_tiles(int64_t M, int64_t N, int64_t batch, int bn) {
+  return (M + UM_BM - 1) / UM_BM * ((N + bn - 1) / bn) * batch;
+}
+
+template <int BN, bool OB>
+void launch_pers(Context* c, const CUtensorMap& ta, const CUtensorMap& tb, int64_t K,
+                 int64_t a_rows_pb, int64_t b_rows_pb, int64_t M, int64_t N, int64_t batch,
+                 const OutMap& om) {
+  const size_t smem = ps_smem_bytes<BN>();
+  ensure_smem_attr(reinterpret_cast<const void*>(k_umma_pers<BN, OB>), c->device, int(smem));
+  const int64_t tiles = umma_tiles(M, N, batch, BN);
+  launch(c, k_umma_pers<BN, OB>, unsigned(std::min<int64_t>(tiles, c->num_sms)), PS_THREADS, smem,
+         ta, tb, int(K), int(a_rows_pb), int(b_rows_pb), om, int((M + UM_BM - 1) / UM_BM),
+         int((N + BN - 1) / BN), int(tiles), c->d_err + 1, c->skip);
+  TTG_CHECK_LAUNCH();
+}
+
 void umma_gemm(Context* c, const CUtensorMap& ta, const CUtensorMap& tb, int64_t K,
                int64_t a_rows_pb, int64_t b_rows_pb, int64_t M, int64_t N, int64_t batch,
                const OutMap& om, bool out_bf16, int bn) {
   TTG_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && batch <= 65535, "umma gemm too large");
+  if (bn == BN_PERS + 256)
+    return out_bf16 ? launch_pers<256, true>(c, ta, tb, K, a_rows_pb, b_rows_pb, M, N, batch, om)
+                    : launch_pers<256, false>(c, ta, tb, K, a_rows_pb, b_rows_pb, M, N, batch, om);
+  if (bn == BN_PERS + 192)
+    return out_bf16 ? launch_pers<192, true>(c, ta, tb, K, a_rows_pb, b_rows_pb, M, N, batch, om)
+                    : launch_pers<192, false>(c, ta, tb, K, a_rows_pb, b_rows_pb, M, N, batch, om);
   if (out_bf16) {
     if (bn == 64) launch_bn<64, true>(c, ta, tb, K, a_rows_pb, b_rows_pb, M, N, batch, om);
     else if (bn == 128) launch_bn<128, true>(c, ta, tb, K, a_rows_pb, b_rows_pb, M, N, batch, om);
@@ -758,9 +969,9 @@ void MixedOp::prepare(Context* c, const MvDims& dd, const double* Phi1, const do
   bn1 = tuned_bn(c, 1);
   bn2 = tuned_bn(c, 2);
   bn3 = tuned_bn(c, 3);
-  make_map(&mapP2, phi2b.p(), d.rx2, d.ra2 * d.ry2, ldx, bn1);
-  make_map(&mapAT, AT.p(), d.n * d.ra2, d.ra1 * d.n, ld1, bn2);
-  make_map(&mapP1, phi1T.p(), d.rx1 * d.ra1, d.ry1, ld2, bn3);
+  make_map(&mapP2, phi2b.p(), d.rx2, d.ra2 * d.ry2, ldx, bn1 % BN_PERS);
+  make_map(&mapAT, AT.p(), d.n * d.ra2, d.ra1 * d.n, ld1, bn2 % BN_PERS);
+  make_map(&mapP1, phi1T.p(), d.rx1 * d.ra1, d.ry1, ld2, bn3 % BN_PERS);
 }
 
 // ---------------------------------------------------------------------------
@@ -835,7 +1046,7 @@ int MixedOp::tuned_bn(Context* c, int stage) {
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(key);
-    if (it != g_tuned.end()) return it->second;
+    if (it != g_tuned.end()) return c->rec && it->second >= BN_PERS ? fallback : it->second;
   }
   if (c->rec) return fallback;  // recorded stream work cannot be timed
   DBuf<float> ysc;
@@ -845,12 +1056,15 @@ int MixedOp::tuned_bn(Context* c, int stage) {
   cudaEvent_t e0, e1;
   TTG_CUDA(cudaEventCreate(&e0));
   TTG_CUDA(cudaEventCreate(&e1));
-  for (int bn : {64, 128, 256}) {
-    if (bn > 64 && bn / 2 >= N) break;  // wider tiles than N only waste columns
+  for (int bn : {64, 128, 256, BN_PERS + 192, BN_PERS + 256}) {
+    const int w = bn % BN_PERS;
+    if (w > 64 && w / 2 >= N) continue;  // wider tiles than N only waste columns
+    // The persistent form pays where its CTAs walk several tiles each.
+    if (bn >= BN_PERS && umma_tiles(M, N, batch, w) < 2 * c->num_sms) continue;
     CUtensorMap mb;
-    if (stage == 1) make_map(&mb, phi2b.p(), d.rx2, N, ldx, bn);
-    else if (stage == 2) make_map(&mb, AT.p(), K, N, ld1, bn);
-    else make_map(&mb, phi1T.p(), K, N, ld2, bn);
+    if (stage == 1) make_map(&mb, phi2b.p(), d.rx2, N, ldx, w);
+    else if (stage == 2) make_map(&mb, AT.p(), K, N, ld1, w);
+    else make_map(&mb, phi1T.p(), K, N, ld2, w);
     run_stage(c, stage, bn, mb, ysc.p());
     TTG_CUDA(cudaEventRecord(e0, c->stream));
     for (int rep = 0; rep < 3; ++rep) run_stage(c, stage, bn, mb, ysc.p());
