@@ -47,10 +47,79 @@ struct OutMap {
   int64_t r_s1, r_t1, r_t2;
   int64_t c_s1, c_t1, c_t2;
   int64_t batch_stride;    // elements
+  int vec4 = 0;            // BF16: four rows of a column are 8 aligned bytes
 };
+
+// Rows run on in memory and every group of four starts on 8 bytes.
+int bf16_vec4(const OutMap& o) {
+  return o.r_t1 == 1 && (reinterpret_cast<uintptr_t>(o.base) & 7) == 0 && o.M % 4 == 0 &&
+         o.r_s1 % 4 == 0 && o.r_t2 % 4 == 0 && o.c_t1 % 4 == 0 && o.c_t2 % 4 == 0 &&
+         o.batch_stride % 4 == 0;
+}
 
 __device__ __forceinline__ int64_t map2(int64_t i, int64_t s1, int64_t t1, int64_t t2) {
   return (i % s1) * t1 + (i / s1) * t2;
+}
+
+// Stores 16 columns n0 .. of the warp's 32 rows from m0 on (v: the lane's row),
+// `boff` elements into the output.  With vec4 four lanes transpose four rows
+// by four columns among themselves, and a lane stores four rows of one column
+// as 8 bytes, instead of one 2-byte store per element (512 x 64 x 512: 141 us for
+// the two BF16 stages, 178 element by element; 97 x 64 x 83: 7.3 us per launch for
+// 9.1, the 32-bit divisions here included).
+template <bool OUT_BF16>
+__device__ __forceinline__ void store16(const OutMap& om, const float (&v)[16], unsigned m0,
+                                        unsigned n0, int64_t boff) {
+  const unsigned lane = threadIdx.x & 31, r_s1 = unsigned(om.r_s1), c_s1 = unsigned(om.c_s1);
+  if (OUT_BF16 && om.vec4) {
+    const unsigned m = m0 + (lane & ~3u), n = n0 + (lane & 3);
+    const bool ok = m < om.M;
+    const bool odd = lane & 1, hi = lane & 2;
+    int64_t off = boff + int64_t(m % r_s1) + int64_t(m / r_s1) * om.r_t2;
+    unsigned cr = n % c_s1;
+    off += int64_t(cr) * om.c_t1 + int64_t(n / c_s1) * om.c_t2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float* a = v + 4 * q;
+      const float r0 = __shfl_xor_sync(0xffffffffu, odd ? a[0] : a[1], 1);
+      const float r1 = __shfl_xor_sync(0xffffffffu, odd ? a[2] : a[3], 1);
+      const __nv_bfloat162 p0 = odd ? __floats2bfloat162_rn(r0, a[1]) : __floats2bfloat162_rn(a[0], r0);
+      const __nv_bfloat162 p1 = odd ? __floats2bfloat162_rn(r1, a[3]) : __floats2bfloat162_rn(a[2], r1);
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&p0);
+      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(&p1);
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, hi ? w0 : w1, 2);
+      if (ok && n + 4 * q < om.N)
+        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(om.base) + off) =
+            hi ? make_uint2(other, w1) : make_uint2(w0, other);
+      cr += 4;
+      off += 4 * om.c_t1;
+      while (cr >= c_s1) {
+        cr -= c_s1;
+        off += om.c_t2 - om.c_s1 * om.c_t1;
+      }
+    }
+    return;
+  }
+  const unsigned m = m0 + lane;
+  const bool ok = m < om.M;
+  int64_t off = boff + int64_t(m % r_s1) * om.r_t1 + int64_t(m / r_s1) * om.r_t2;
+  unsigned cr = n0 % c_s1;
+  off += int64_t(cr) * om.c_t1 + int64_t(n0 / c_s1) * om.c_t2;
+  const int left = int(om.N - n0);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (ok && j < left) {
+      if (OUT_BF16)
+        static_cast<__nv_bfloat16*>(om.base)[off] = __float2bfloat16_rn(v[j]);
+      else
+        static_cast<float*>(om.base)[off] = v[j];
+    }
+    off += om.c_t1;
+    if (++cr == c_s1) {
+      cr = 0;
+      off += om.c_t2 - om.c_s1 * om.c_t1;
+    }
+  }
 }
 
 template <int BN>
@@ -141,34 +210,13 @@ __device__ __forceinline__ void umma_body(TTG_BLOCK, const CUtensorMap* tmA,
   const bool ok = mbar_wait(bar_done, 0, err);
   tc_fence_after();
   if (ok) {
-    const int row = warp * 32 + lane;
-    const int64_t m = int64_t(m0) + row;
-    const bool row_ok = m < om.M;
-    const int64_t roff = row_ok ? map2(m, om.r_s1, om.r_t1, om.r_t2) : 0;
-    const int64_t boff = int64_t(bz) * om.batch_stride;
-    // Column offsets advance incrementally: (n % c_s1, n / c_s1) -> no
-    // division per element.
-    int64_t cq = (int64_t(n0)) / om.c_s1, cr = (int64_t(n0)) % om.c_s1;
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 16) {
       if (n0 + c0 >= om.N) break;  // uniform across the CTA
       float v[16];
       tmem_ld16(tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0), v);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int64_t n = int64_t(n0) + c0 + j;
-        if (row_ok && n < om.N) {
-          const int64_t off = boff + roff + cr * om.c_t1 + cq * om.c_t2;
-          if (OUT_BF16)
-            static_cast<__nv_bfloat16*>(om.base)[off] = __float2bfloat16_rn(v[j]);
-          else
-            static_cast<float*>(om.base)[off] = v[j];
-        }
-        if (++cr == om.c_s1) {
-          cr = 0;
-          ++cq;
-        }
-      }
+      store16<OUT_BF16>(om, v, unsigned(m0 + warp * 32), unsigned(n0 + c0),
+                        int64_t(bz) * om.batch_stride);
     }
   }
   tc_fence_before();
@@ -231,7 +279,7 @@ const GroupInfo* umma_info() {
 // narrow tiles hide their epilogues behind other CTAs but load (128 + BN)
 // operand rows from L2 for every 128 x BN products, and L2 bounds it: at 512 x
 // 64 x 512, ranks 3, its stages move 1.2, 0.3 and 0.8 GB at 8-9 TB/s.  Tiles of
-// 256 halve that.  127, 127 and 104 us of the plain form become 89, 89 and 60
+// 256 halve that.  127, 127 and 104 us of the plain form become 74, 67 and 60
 // there (865 TFLOP/s for the last stage), bit for bit.
 // Every wait is bounded: a timeout raises the error flag and every role winds
 // down.
@@ -350,15 +398,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     __syncwarp();
   } else {  // epilogue: warp w owns TMEM lanes 32 (w % 4) .., every other 16 columns
     const int ew = warp & 3, half = (warp - 2) >> 2;
-    const int row = ew * 32 + lane;
-    const unsigned r_s1 = unsigned(om.r_s1), c_s1 = unsigned(om.c_s1);
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tile_cnt) {
       const uint32_t buf = tile_cnt & 1;
       const int ni = t % nt, mi = t / nt % mt, bz = t / nt / mt;
-      const unsigned m = unsigned(mi * UM_BM + row);
-      const bool row_ok = m < om.M;
-      const int64_t base = int64_t(bz) * om.batch_stride + int64_t(m % r_s1) * om.r_t1 +
-                           int64_t(m / r_s1) * om.r_t2;
       const bool ok = mbar_wait(bar_accf + 8 * buf, (tile_cnt >> 1) & 1, err);
       tc_fence_after();
       if (!ok) break;
@@ -369,23 +411,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         if (n0 >= om.N) break;  // uniform across the warp
         float v[16];
         tmem_ld16(tbase + uint32_t(c0), v);
-        unsigned cr = n0 % c_s1;
-        int64_t off = base + int64_t(cr) * om.c_t1 + int64_t(n0 / c_s1) * om.c_t2;
-        const int left = int(om.N - n0);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (row_ok && j < left) {
-            if (OUT_BF16)
-              static_cast<__nv_bfloat16*>(om.base)[off] = __float2bfloat16_rn(v[j]);
-            else
-              static_cast<float*>(om.base)[off] = v[j];
-          }
-          off += om.c_t1;
-          if (++cr == c_s1) {
-            cr = 0;
-            off += om.c_t2 - om.c_s1 * om.c_t1;
-          }
-        }
+        store16<OUT_BF16>(om, v, unsigned(mi * UM_BM + ew * 32), n0,
+                          int64_t(bz) * om.batch_stride);
       }
       tc_fence_before();
       __syncwarp();
@@ -1020,9 +1047,11 @@ void MixedOp::run_stage(Context* c, int stage, int bn, const CUtensorMap& mapB, 
   const int64_t rows = d.m * d.rx1;
   if (stage == 1) {
     OutMap o1{T1.p(), rows, d.ra2 * d.ry2, d.m, 1, ld1, d.ra2, d.m, ld1 * d.rx1, 0};
+    o1.vec4 = bf16_vec4(o1);
     umma_gemm(c, mapX, mapB, d.rx2, 0, 0, rows, d.ra2 * d.ry2, 1, o1, true, bn);
   } else if (stage == 2) {
     OutMap o2{T2.p(), d.rx1, d.ra1 * d.n, d.rx1, 1, 0, d.ra1, d.rx1, ld2 * d.ry2, ld2};
+    o2.vec4 = bf16_vec4(o2);
     umma_gemm(c, mapT1, mapB, d.n * d.ra2, d.rx1, 0, d.rx1, d.ra1 * d.n, d.ry2, o2, true, bn);
   } else {
     const int64_t rows3 = d.ry2 * d.n;
