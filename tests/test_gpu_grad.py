@@ -242,6 +242,27 @@ def test_grad_d12_n32_r64_full_size(ctx):
         assert grad_rel(split(G, xc), Gr) <= GRAD_TOL, name
 
 
+@pytest.mark.parametrize("n,r,ra", [
+    ([9], [1, 1], [1, 1]),                            # one core: nothing to pair at its ends
+    ([5, 7], [1, 3, 1], [1, 2, 1]),
+    ([33, 1, 40], [1, 33, 31, 1], [1, 2, 5, 1]),      # edges of the 32 x 32 tiles, n = 1
+    ([16, 700, 16], [1, 16, 15, 1], [1, 3, 2, 1]),    # long k: both products of a launch split
+    ([64, 64, 8], [1, 64, 8, 1], [1, 1, 4, 1]),       # the two sweeps differ in size
+    ([128, 96], [1, 128, 1], [1, 6, 1]),
+])
+def test_grad_xAx_sweeps_share_launches(ctx, n, r, ra):
+    rng = np.random.default_rng(sum(n) + sum(r))
+    xs = rand_cores(rng, n, r)
+    As = [np.asfortranarray(rng.standard_normal((ra[k], n[k], n[k], ra[k + 1])))
+          for k in range(len(n))]
+    v, G = ttgpu.grad_xAx(to_tt(xs), to_mat(As), ctx=ctx)
+    vref, Gref = og.xAx(xs, As)
+    # the value is a sum of products with both signs: relative to |x_k| |g_k|
+    scale = np.linalg.norm(xs[0]) * np.linalg.norm(Gref[0])
+    assert abs(v - vref) <= VAL_TOL * max(abs(vref), scale)
+    assert grad_rel(split(G, xs), Gref) <= GRAD_TOL
+
+
 def test_grad_xAx_without_kept_intermediates(ctx):
     """A core whose left products exceed what the sweep keeps (1 GiB) forms
     them again.  f is quadratic in every core, so <x_k, g_k> = 2 f for all k;

@@ -39,8 +39,8 @@ namespace {
 
 constexpr int PT = 128;          // samples per propagation tile
 constexpr int PROP_THREADS = 256, GRAD_THREADS = 128, GRAD_STAGES = 3;
-// Bytes of intermediates the left sweep of <x, A x> keeps for the right one.
-constexpr int64_t KEEP_MAX = int64_t(1) << 30;
+// Bytes of intermediates that <x, A x> keeps between its sweeps and the gradient.
+constexpr int64_t KEEP_MAX = int64_t(2) << 30;
 constexpr int GT = 512;          // samples per gradient (split-K) tile
 constexpr int SORT_CHUNK = 1024; // samples per sorting warp
 constexpr int64_t MAX_BUCKETS = 8192;
@@ -521,69 +521,102 @@ void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, do
                 (long long)A->n[k], (long long)A->m[k], (long long)x->n[k]);
   const auto& r = x->r;
   const auto& ra = A->r;
-  // Interfaces: L[k] [r_k, r_k, ra_k] (k = 0..d), R [r_k, ra_k, r_k] of the
-  // right sweep's current core.
-  std::vector<int64_t> off(d + 2, 0), woff(d + 1, 0);
-  int64_t nphi = 1, w1max = 1, w2max = 1;
-  for (int64_t k = 0; k <= d; ++k) {
-    off[k + 1] = off[k] + r[k] * r[k] * ra[k];
-    nphi = std::max(nphi, r[k] * r[k] * ra[k]);
-  }
+  // Interfaces L[k] [r_k, r_k, ra_k] and R[k] [r_k, ra_k, r_k], k = 0..d, and the
+  // second products of every core's updates, W2 and Z2.
+  std::vector<int64_t> off(d + 2, 0), woff(d + 1, 0), zoff(d + 1, 0);
+  int64_t w1max = 1, z1max = 1;
+  for (int64_t k = 0; k <= d; ++k) off[k + 1] = off[k] + r[k] * r[k] * ra[k];
   for (int64_t k = 0; k < d; ++k) {
-    const int64_t w2 = r[k] * x->n[k] * ra[k + 1] * r[k + 1];
+    const int64_t w2 = r[k] * x->n[k] * ra[k + 1] * r[k + 1],
+                  z2 = r[k] * ra[k] * x->n[k] * r[k + 1];
     woff[k + 1] = woff[k] + w2;
-    w2max = std::max(w2max, w2);
-    w1max = std::max(w1max, r[k] * ra[k] * x->n[k] * r[k + 1]);
+    zoff[k + 1] = zoff[k] + z2;
+    w1max = std::max(w1max, z2);
+    z1max = std::max(z1max, w2);
   }
-  // The left sweep's W2 of every core serve the right sweep, unless that
-  // would hold too much memory: then each is formed again.
-  const bool keep = woff[d] * int64_t(sizeof(double)) <= KEEP_MAX;
-  DBuf<double> L(c, off[d + 1]), R0(c, nphi), R1(c, nphi);
-  DBuf<double> W1(c, w1max), W2(c, keep ? woff[d] : w2max), Z1(c, w2max), Z2(c, w1max);
-  double* Rk = R0.p();
-  double* Rn = R1.p();
+  // Every core's W2 and Z2 are kept between the sweeps and the gradient, and
+  // the sweeps then run side by side, unless that would hold too much memory:
+  // then the right sweep follows the left one and forms W2 again.
+  const bool keep = (woff[d] + zoff[d]) * int64_t(sizeof(double)) <= KEEP_MAX;
+  DBuf<double> L(c, off[d + 1]), R(c, off[d + 1]);
+  DBuf<double> W1(c, w1max), Z1(c, z1max), W2(c, keep ? woff[d] : z1max),
+      Z2(c, keep ? zoff[d] : w1max);
+  auto W2k = [&](int64_t k) { return W2.p() + (keep ? woff[k] : 0); };
+  auto Z2k = [&](int64_t k) { return Z2.p() + (keep ? zoff[k] : 0); };
   fill_f64(c, 1, 1.0, L.p());
-  fill_f64(c, 1, 1.0, Rk);
-  // W1[(y,al),(j,c)] = L^T x, W2_c[y,(m,be)] = W1_c[y,(al,j)] A[(al,j),(m,be)]
-  auto left_products = [&](int64_t k, double* w2) {
-    const int64_t r1 = r[k], r2 = r[k + 1], a1 = ra[k], a2 = ra[k + 1], n = x->n[k];
-    gemm_f64(c, true, false, r1 * a1, n * r2, r1, 1.0, L.p() + off[k], r1, 0, x->core + x->ps[k],
-             r1, 0, 0.0, W1.p(), r1 * a1, 0, 1);
-    gemm_f64(c, false, false, r1, n * a2, a1 * n, 1.0, W1.p(), r1, r1 * a1 * n,
-             A->core + A->ps[k], a1 * n, 0, 0.0, w2, r1, r1 * n * a2, r2);
-  };
-  for (int64_t k = 0; k < d; ++k) {
-    const int64_t r1 = r[k], r2 = r[k + 1], a2 = ra[k + 1], n = x->n[k];
-    double* w2 = W2.p() + (keep ? woff[k] : 0);
-    left_products(k, w2);
-    // L_{k+1},be [c, e] = W2[(y,m), be, c]^T x[(y,m), e]
-    gemm_f64(c, true, false, r2, r2, r1 * n, 1.0, w2, r1 * n * a2, r1 * n, x->core + x->ps[k],
-             r1 * n, 0, 0.0, L.p() + off[k + 1], r2, r2 * r2, a2);
-  }
-  if (value) copy_f64(c, 1, L.p() + off[d], value);
-  for (int64_t k = d - 1; k >= 0; --k) {
+  fill_f64(c, 1, 1.0, R.p() + off[d]);
+  // left: W1[(y,al),(j,c)] = L_k^T x, W2_c[y,(m,be)] = W1_c[y,(al,j)] A[(al,j),(m,be)],
+  //       L_{k+1},be [c, e] = W2[(y,m), be, c]^T x[(y,m), e]
+  // right: Z1[(y,m),(be,c)] = x R_{k+1}, Z2_c[y,(al,j)] = Z1_c[y,(m,be)] A[(al,j),(m,be)]^T,
+  //       R_k[(y,al), a] = Z2[(y,al),(j,c)] x[a,(j,c)]^T
+  // gradient through the bra copy: G[a,(j,c)] = L_k[a,(y,al)] Z2[(y,al),(j,c)],
+  //       through the ket copy: G[(y,m), e] += W2[(y,m),(be,c)] R_{k+1}[e,(be,c)]^T
+  enum { LEFT1, LEFT2, LEFT3, RIGHT1, RIGHT2, RIGHT3, BRA, KET };
+  auto op = [&](int which, int64_t k) -> GemmOp {
     const int64_t r1 = r[k], r2 = r[k + 1], a1 = ra[k], a2 = ra[k + 1], n = x->n[k];
     const double* xk = x->core + x->ps[k];
+    const double* Ak = A->core + A->ps[k];
     double* gk = grad + x->ps[k];
-    double* w2 = W2.p() + (keep ? woff[k] : 0);
-    // Z1[(y,m),(be,c)] = x R_{k+1}, Z2_c[y,(al,j)] = Z1_c[y,(m,be)] A[(al,j),(m,be)]^T
-    gemm_f64(c, false, false, r1 * n, a2 * r2, r2, 1.0, xk, r1 * n, 0, Rk, r2, 0, 0.0, Z1.p(),
-             r1 * n, 0, 1);
-    gemm_f64(c, false, true, r1, a1 * n, n * a2, 1.0, Z1.p(), r1, r1 * n * a2,
-             A->core + A->ps[k], a1 * n, 0, 0.0, Z2.p(), r1, r1 * a1 * n, r2);
-    // through the bra copy: G[a,(j,c)] = L_k[a,(y,al)] Z2[(y,al),(j,c)]
-    gemm_f64(c, false, false, r1, n * r2, r1 * a1, 1.0, L.p() + off[k], r1, 0, Z2.p(), r1 * a1, 0,
-             0.0, gk, r1, 0, 1);
-    // through the ket copy: G[(y,m), e] += W2[(y,m),(be,c)] R_{k+1}[e,(be,c)]^T
-    if (!keep) left_products(k, w2);
-    gemm_f64(c, false, true, r1 * n, r2, a2 * r2, 1.0, w2, r1 * n, 0, Rk, r2, 0, 1.0, gk, r1 * n,
-             0, 1);
-    if (k == 0) break;
-    // R_k[(y,al), a] = Z2[(y,al),(j,c)] x[a,(j,c)]^T
-    gemm_f64(c, false, true, r1 * a1, r1, n * r2, 1.0, Z2.p(), r1 * a1, 0, xk, r1, 0, 0.0, Rn,
-             r1 * a1, 0, 1);
-    std::swap(Rk, Rn);
+    const double* Lk = L.p() + off[k];
+    const double* Rn = R.p() + off[k + 1];
+    switch (which) {
+      case LEFT1:
+        return {true, false, r1 * a1, n * r2, r1, Lk, r1, 0, xk, r1, 0, 0.0, W1.p(), r1 * a1, 0, 1};
+      case LEFT2:
+        return {false, false, r1, n * a2, a1 * n, W1.p(), r1, r1 * a1 * n, Ak, a1 * n, 0, 0.0,
+                W2k(k), r1, r1 * n * a2, r2};
+      case LEFT3:
+        return {true, false, r2, r2, r1 * n, W2k(k), r1 * n * a2, r1 * n, xk, r1 * n, 0, 0.0,
+                L.p() + off[k + 1], r2, r2 * r2, a2};
+      case RIGHT1:
+        return {false, false, r1 * n, a2 * r2, r2, xk, r1 * n, 0, Rn, r2, 0, 0.0, Z1.p(), r1 * n,
+                0, 1};
+      case RIGHT2:
+        return {false, true, r1, a1 * n, n * a2, Z1.p(), r1, r1 * n * a2, Ak, a1 * n, 0, 0.0,
+                Z2k(k), r1, r1 * a1 * n, r2};
+      case RIGHT3:
+        return {false, true, r1 * a1, r1, n * r2, Z2k(k), r1 * a1, 0, xk, r1, 0, 0.0,
+                R.p() + off[k], r1 * a1, 0, 1};
+      case BRA:
+        return {false, false, r1, n * r2, r1 * a1, Lk, r1, 0, Z2k(k), r1 * a1, 0, 0.0, gk, r1, 0,
+                1};
+      default:
+        return {false, true, r1 * n, r2, a2 * r2, W2k(k), r1 * n, 0, Rn, r2, 0, 1.0, gk, r1 * n, 0,
+                1};
+    }
+  };
+  auto one = [&](int which, int64_t k) {
+    const GemmOp o = op(which, k);
+    gemm_f64(c, o.tA, o.tB, o.M, o.N, o.K, 1.0, o.A, o.lda, o.sA, o.B, o.ldb, o.sB, o.beta, o.C,
+             o.ldc, o.sC, o.batch);
+  };
+  if (keep) {
+    for (int64_t k = 0; k < d; ++k) {
+      const int64_t l = d - 1 - k;
+      gemm_pair_f64(c, op(LEFT1, k), op(RIGHT1, l));
+      gemm_pair_f64(c, op(LEFT2, k), op(RIGHT2, l));
+      if (l > 0)
+        gemm_pair_f64(c, op(LEFT3, k), op(RIGHT3, l));
+      else
+        one(LEFT3, k);
+    }
+    for (int64_t k = 0; k <= d; ++k) {  // a core's ket product follows its bra product
+      if (k == 0)
+        one(BRA, 0);
+      else if (k < d)
+        gemm_pair_f64(c, op(BRA, k), op(KET, k - 1));
+      else
+        one(KET, d - 1);
+    }
+  } else {
+    for (int64_t k = 0; k < d; ++k)
+      for (int which : {LEFT1, LEFT2, LEFT3}) one(which, k);
+    for (int64_t k = d - 1; k >= 0; --k) {
+      for (int which : {RIGHT1, RIGHT2, BRA, LEFT1, LEFT2, KET}) one(which, k);
+      if (k > 0) one(RIGHT3, k);
+    }
   }
+  if (value) copy_f64(c, 1, L.p() + off[d], value);
 }
 
 // ---------------------------------------------------------------------------

@@ -15,6 +15,22 @@ void gemm_f64(Context* c, bool tA, bool tB, int64_t M, int64_t N, int64_t K, dou
               const double* A, int64_t lda, int64_t sA, const double* B, int64_t ldb,
               int64_t sB, double beta, double* C, int64_t ldc, int64_t sC, int64_t batch = 1);
 
+// Two independent products C = op(A) op(B) + beta C (arguments as gemm_f64's), in
+// one launch for the combinations of transpositions (T,N)+(N,N), (N,N)+(N,T) and
+// (T,N)+(N,T), one after the other for the rest and in a grouped batch.
+struct GemmOp {
+  bool tA, tB;
+  int64_t M, N, K;
+  const double* A;
+  int64_t lda, sA;
+  const double* B;
+  int64_t ldb, sB;
+  double beta;
+  double* C;
+  int64_t ldc, sC, batch;
+};
+void gemm_pair_f64(Context* c, const GemmOp& a, const GemmOp& b);
+
 // out = sum(x.*y) (or sum(x.^2) when y == nullptr) into a device scalar;
 // deterministic one-launch reduction (block partials summed in block order
 // by the last block).  If do_sqrt, stores sqrt of the sum.

@@ -58,7 +58,7 @@ constexpr size_t gemm_smem() {
 // TFLOP/s).  Four stages, eight warps per tile and the larger mma shapes
 // measure the same or slower.
 template <int BM, int BN, bool TA, bool TB>
-TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
+__device__ __forceinline__ void gemm_body(TTG_BLOCK, const GemmP& p) {
   pdl_begin();
   extern __shared__ __align__(16) double gsm[];
   constexpr int NT = GEMM_THREADS;
@@ -207,7 +207,33 @@ TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
   }
 }
 template <int BM, int BN, bool TA, bool TB>
+TTG_BODY(k_gemm_f64)(TTG_BLOCK, GemmP p) {
+  gemm_body<BM, BN, TA, TB>(blockIdx, gridDim, p);
+}
+template <int BM, int BN, bool TA, bool TB>
 TTG_KERNEL_T(k_gemm_f64, GEMM_THREADS, BM, BN, TA, TB);
+
+// Two independent products in one launch: the first n1 blocks are the first
+// product's grid g1, the others the second's.  For chains of short products
+// that run side by side (the left and right sweeps of a gradient), which are
+// bound by each launch's chain of first loads, k loop and stores: sharing the
+// launches takes the gradient of <x, A x> at d = 12, n = 32, rank 64 from 721 to
+// 580 us (six cores of 8, rank 16: 177 to 134).  Up to 198 registers a thread: at 128 (twice the CTAs an SM) the
+// next launch's waiting CTAs take the places of this one's last ones, 660 us.
+template <int BM, int BN, bool TA1, bool TB1, bool TA2, bool TB2>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+    k_gemm_pair(GemmP p, GemmP q, dim3 g1, dim3 g2) {
+  pdl_begin();
+  const unsigned n1 = g1.x * g1.y * g1.z;
+  const bool first = blockIdx.x < n1;
+  const unsigned b = first ? blockIdx.x : blockIdx.x - n1;
+  const dim3 g = first ? g1 : g2;
+  const uint3 at = {b % g.x, b / g.x % g.y, b / (g.x * g.y)};
+  if (first)
+    gemm_body<BM, BN, TA1, TB1>(at, g, p);
+  else
+    gemm_body<BM, BN, TA2, TB2>(at, g, q);
+}
 
 // ---------------------------------------------------------------------------
 // Reductions
@@ -559,25 +585,30 @@ struct GemmPlan {
 // last CTA's sum or a second kernel.  Interface update with this rule, against
 // split-K to two 64 x 64 CTAs per SM: 61 x 64 x 67 54 / 83 us, 128 x 64 x 128
 // 136 / 216, 512 x 64 x 512 4.4 / 8.0 ms.
-GemmPlan plan_gemm(Context* c, int64_t M, int64_t N, int64_t K, int64_t batch, bool may_split) {
+// `sms`: the SMs the product may count on; `only`: plan for this tile; partials
+// of one tile stay within `most`.
+GemmPlan plan_gemm(int64_t sms, int64_t M, int64_t N, int64_t K, int64_t batch, bool may_split,
+                   const GemmTile* only = nullptr, int64_t most = INT64_MAX) {
   const int64_t ktiles = (K + TILE_K - 1) / TILE_K;
   GemmPlan best{};
   double best_t = 0.0;
   for (const GemmTile& t : GEMM_TILES) {
     const int64_t gx = (M + t.bm - 1) / t.bm, gy = (N + t.bn - 1) / t.bn, ctas = gx * gy * batch;
-    if (&t != GEMM_TILES && (gy > 65535 || gx > 0x7fffffff)) continue;  // the grid's limits
+    if (only && only->bm * only->bn != t.bm * t.bn) continue;
+    if (!only && &t != GEMM_TILES && (gy > 65535 || gx > 0x7fffffff)) continue;  // the grid's limits
     int64_t smax = 1;
-    if (may_split && ctas < 4 * c->num_sms && ktiles >= 8 && ctas <= GEMM_TILE_COUNTERS)
-      smax = std::min({ktiles / 4, 8 * c->num_sms / ctas + 1, 65535 / batch});
+    if (may_split && ctas < 4 * sms && ktiles >= 8 && ctas <= GEMM_TILE_COUNTERS)
+      smax = std::min({ktiles / 4, 8 * sms / ctas + 1, 65535 / batch});
     int64_t prev = 0;
     for (int64_t s = 1; s <= smax; s = s < 8 ? s + 1 : s + s / 4) {
       const int64_t kt = (ktiles + s - 1) / s, ns = (ktiles + kt - 1) / kt;
       if (ns == prev) continue;
       prev = ns;
-      const int64_t per_sm = (ctas * ns + c->num_sms - 1) / c->num_sms;
+      const int64_t per_sm = (ctas * ns + sms - 1) / sms;
       const double idle = per_sm == 1 ? 2.2 : per_sm == 2 ? 1.45 : per_sm == 3 ? 1.15 : 1.0;
       double est = double(per_sm * kt) * (t.bm * t.bn / 4) * t.cost * idle;
       if (ns > 1) {
+        if (ns * std::min<int64_t>(M, t.bm) * std::min<int64_t>(N, t.bn) > most) break;
         const int64_t te = std::min<int64_t>(M, t.bm) * std::min<int64_t>(N, t.bn);
         est += 16.0 * double(ns * M * N * batch) / 2600.0 +
                (ns * te <= SPLITK_INKERNEL_MAX ? 2500.0 : 4500.0);
@@ -618,7 +649,7 @@ void gemm_f64(Context* c, bool tA, bool tB, int64_t M, int64_t N, int64_t K, dou
   // reading many partials is latency-bound).
   // (A context without an allocator -- the caller-scratch entry point -- runs
   // every product unsplit.)
-  const GemmPlan pl = plan_gemm(c, M, N, K, batch, c->alloc && c->d_tile_cnt);
+  const GemmPlan pl = plan_gemm(c->num_sms, M, N, K, batch, c->alloc && c->d_tile_cnt);
   GemmP p{M,  N,     K,       A,  lda, sA, B, ldb, sB, C, ldc, sC, alpha, beta, c->skip,
           vec16(A, lda, sA, batch), vec16(B, ldb, sB, batch), 1, 0, nullptr, nullptr};
   dim3 grid{unsigned(pl.gx), unsigned(pl.gy), unsigned(batch * pl.split)};
@@ -643,6 +674,78 @@ void gemm_f64(Context* c, bool tA, bool tB, int64_t M, int64_t N, int64_t K, dou
            part.p(), alpha, beta, C, ldc, sC, c->skip);
     TTG_CHECK_LAUNCH();
   }
+}
+
+namespace {
+
+template <int BM, int BN, bool TA1, bool TB1, bool TA2, bool TB2>
+void pair_launch(Context* c, const GemmP& p, const GemmP& q, dim3 g1, dim3 g2) {
+  constexpr size_t s1 = gemm_smem<BM, BN, TA1, TB1>(), s2 = gemm_smem<BM, BN, TA2, TB2>();
+  constexpr size_t smem = s1 > s2 ? s1 : s2;
+  const void* fn = reinterpret_cast<const void*>(k_gemm_pair<BM, BN, TA1, TB1, TA2, TB2>);
+  if (smem > 48 * 1024) ensure_smem_attr(fn, c->device, int(smem));
+  const unsigned blocks = g1.x * g1.y * g1.z + g2.x * g2.y * g2.z;
+  launch(c, k_gemm_pair<BM, BN, TA1, TB1, TA2, TB2>, blocks, GEMM_THREADS, smem, p, q, g1, g2);
+  TTG_CHECK_LAUNCH();
+}
+
+// Partials of one tile that the last slice of a pair sums: 12 slices of 32 x 32
+// (615 us in the gradient above with 8, 640 with 16 or more: one CTA reads them).
+constexpr int64_t PAIR_SPLITK_MAX = 12288;
+
+template <bool TA1, bool TB1, bool TA2, bool TB2>
+bool pair_f64(Context* c, const GemmOp& a, const GemmOp& b) {
+  if (c->rec || !c->alloc || !c->d_tile_cnt) return false;
+  for (const GemmOp* o : {&a, &b})  // gemm_f64 refuses these
+    if (o->batch > 65535 || (o->N + 63) / 64 > 65535 || (o->M + 63) / 64 > 0x7fffffff) return false;
+  // Each product plans for half the device, with the first one's tile, and
+  // sums its slices in the kernel.
+  const int64_t sms = std::max(1, c->num_sms / 2);
+  const GemmPlan pa = plan_gemm(sms, a.M, a.N, a.K, a.batch, true, nullptr, PAIR_SPLITK_MAX);
+  const GemmPlan pb = plan_gemm(sms, b.M, b.N, b.K, b.batch, true, &pa.tile, PAIR_SPLITK_MAX);
+  const int64_t ta = pa.gx * pa.gy * a.batch, tb = pb.gx * pb.gy * b.batch;
+  // (products of more tiles than counters fill the device one by one)
+  if (ta * pa.split + tb * pb.split > 0x7fffffff || ta + tb > GEMM_TILE_COUNTERS) return false;
+  DBuf<double> part1, part2;
+  auto params = [&](const GemmOp& o, const GemmPlan& pl, DBuf<double>& part, unsigned* cnt) {
+    GemmP p{o.M,   o.N,     o.K,   o.A,  o.lda, o.sA,   o.B,     o.ldb,    o.sB,
+            o.C,   o.ldc,   o.sC,  1.0,  o.beta, c->skip, vec16(o.A, o.lda, o.sA, o.batch),
+            vec16(o.B, o.ldb, o.sB, o.batch), 1, 0, nullptr, nullptr};
+    if (pl.split > 1) {
+      part.reset(c, o.batch * pl.split * o.M * o.N);
+      p.nsplit = pl.split;
+      p.kc = pl.kc;
+      p.part = part.p();
+      p.cnt = cnt;
+    }
+    return p;
+  };
+  const GemmP p = params(a, pa, part1, c->d_tile_cnt), q = params(b, pb, part2, c->d_tile_cnt + ta);
+  const dim3 g1{unsigned(pa.gx), unsigned(pa.gy), unsigned(a.batch * pa.split)};
+  const dim3 g2{unsigned(pb.gx), unsigned(pb.gy), unsigned(b.batch * pb.split)};
+  if (pa.tile.bm == 64)
+    pair_launch<64, 64, TA1, TB1, TA2, TB2>(c, p, q, g1, g2);
+  else if (pa.tile.bn == 64)
+    pair_launch<32, 64, TA1, TB1, TA2, TB2>(c, p, q, g1, g2);
+  else
+    pair_launch<32, 32, TA1, TB1, TA2, TB2>(c, p, q, g1, g2);
+  return true;
+}
+
+}  // namespace
+
+void gemm_pair_f64(Context* c, const GemmOp& a, const GemmOp& b) {
+  bool done = false;
+  if (a.M > 0 && a.N > 0 && a.K > 0 && a.batch > 0 && b.M > 0 && b.N > 0 && b.K > 0 &&
+      b.batch > 0) {
+    if (a.tA && !a.tB && !b.tA && !b.tB) done = pair_f64<true, false, false, false>(c, a, b);
+    if (!a.tA && !a.tB && !b.tA && b.tB) done = pair_f64<false, false, false, true>(c, a, b);
+    if (a.tA && !a.tB && !b.tA && b.tB) done = pair_f64<true, false, false, true>(c, a, b);
+  }
+  if (done) return;
+  for (const GemmOp* o : {&a, &b})
+    gemm_f64(c, o->tA, o->tB, o->M, o->N, o->K, 1.0, o->A, o->lda, o->sA, o->B, o->ldb, o->sB,
+             o->beta, o->C, o->ldc, o->sC, o->batch);
 }
 
 void dot_f64(Context* c, int64_t n, const double* x, const double* y, double* out, bool do_sqrt) {
