@@ -233,8 +233,8 @@ TTG_COOP_KERNEL(k_hh_init, HH_THREADS);
 // (u_{j+1} = (w2 + alpha e_{j+1}) / nu there).  v_{j+1} has unit norm by
 // construction.  Bound by the four reads of U a step (41 columns of 64 x 64 x
 // 64 are 86 MB, mostly L2 hits): a local solve of two restarts of 40 at that
-// size takes 7.0 ms, 40 us of it this kernel per step, against 22.3 ms with
-// one grid barrier per reflector (225 us per step).
+// size takes 5.8 ms, 40 us of it this kernel per step, against 20.3 ms with
+// one grid barrier per reflector (225 us per step) and the same matvec.
 TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
   if (*(volatile int*)a.stop) return;  // queued after convergence
   extern __shared__ double hsm[];
@@ -412,7 +412,7 @@ TTG_KERNEL(k_hh_correct, HH_THREADS);
 
 // Blocks of the cooperative kernels: contiguous row ranges of at least HH_ROWS
 // rows, at most two blocks per SM.  Two keep twice the loads of U in flight
-// (64 x 64 x 64, 80 steps: 7.04 against 7.66 ms with one); small systems take
+// (64 x 64 x 64, 80 steps: one block an SM takes 8 us a step longer); small systems take
 // few blocks, and 256 or 512 rows as the least share measure the same.
 constexpr int64_t HH_ROWS = 256;
 int coop_blocks(Context* c, const void* kernel, size_t smem, int64_t sz) {

@@ -218,8 +218,8 @@ TTG_KERNEL_T(k_gemm_f64, GEMM_THREADS, BM, BN, TA, TB);
 // that run side by side (the left and right sweeps of a gradient), which are
 // bound by each launch's chain of first loads, k loop and stores: sharing the
 // launches takes the gradient of <x, A x> at d = 12, n = 32, rank 64 from 721 to
-// 580 us (six cores of 8, rank 16: 177 to 134).  Up to 198 registers a thread: at 128 (twice the CTAs an SM) the
-// next launch's waiting CTAs take the places of this one's last ones, 660 us.
+// 580 us (six cores of 8, rank 16: 177 to 134).  Up to 198 registers a thread:
+// at 128, with more CTAs on an SM, the gradient takes 9% longer.
 template <int BM, int BN, bool TA1, bool TB1, bool TA2, bool TB2>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     k_gemm_pair(GemmP p, GemmP q, dim3 g1, dim3 g2) {
@@ -359,17 +359,11 @@ TTG_BODY(k_copy)(TTG_BLOCK, int64_t n, const double* __restrict__ x, double* __r
 }
 TTG_KERNEL(k_copy, 0);
 
-// Pairs, from the first 16-byte boundary on (134 MB: 22 us, against 39 one by one).
 TTG_BODY(k_fill)(TTG_BLOCK, int64_t n, double v, double* y) {
   pdl_begin();
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t head = (reinterpret_cast<uintptr_t>(y) >> 3) & 1, pairs = (n - head) / 2;
-  if (t == 0) {
-    if (head) y[0] = v;
-    if (head + 2 * pairs < n) y[n - 1] = v;
-  }
-  double2* y2 = reinterpret_cast<double2*>(y + head);
-  for (int64_t i = t; i < pairs; i += int64_t(gridDim.x) * blockDim.x) y2[i] = make_double2(v, v);
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x)
+    y[i] = v;
 }
 TTG_KERNEL(k_fill, 0);
 
@@ -690,7 +684,7 @@ void pair_launch(Context* c, const GemmP& p, const GemmP& q, dim3 g1, dim3 g2) {
 }
 
 // Partials of one tile that the last slice of a pair sums: 12 slices of 32 x 32
-// (615 us in the gradient above with 8, 640 with 16 or more: one CTA reads them).
+// (the gradient above takes 3% longer with 8, 5% with 16: one CTA reads them).
 constexpr int64_t PAIR_SPLITK_MAX = 12288;
 
 template <bool TA1, bool TB1, bool TA2, bool TB2>
@@ -819,7 +813,7 @@ void scale_dev_f64(Context* c, int64_t n, const double* x, double* y, const doub
 
 void fill_f64(Context* c, int64_t n, double v, double* y) {
   if (n <= 0) return;
-  launch(c, k_fill, grid_for(c, (n + 1) / 2), 256, 0, n, v, y);
+  launch(c, k_fill, grid_for(c, n), 256, 0, n, v, y);
   TTG_CHECK_LAUNCH();
 }
 

@@ -2,15 +2,18 @@
 // and rounding sweeps (replacing library calls whose host-side sequencing
 // cost milliseconds on 64x64 inputs):
 //
-//   k_jacobi_svd : one-sided (Hestenes) Jacobi SVD of a square n x n matrix,
-//                  round-robin pairing, one warp per column pair, the matrix
-//                  held in shared memory (global memory above ~160 columns),
-//                  V accumulated in global memory.  Singular values sorted
-//                  descending.  One launch, no host round trip.
-//   k_house_qr   : Householder QR (LAPACK sign convention: beta =
-//                  -sign(alpha) ||x||, as geqrf/orgqr and MATLAB's qr(A,0))
-//                  of an m x n matrix that fits in shared memory; forms the
-//                  thin Q and R.
+//   k_jacobi_svd :     one-sided block Jacobi SVD of a square n x n matrix,
+//                      n <= 96, in one CTA: A and V in shared memory, blocks
+//                      of eight columns rotated by 16 x 16 Gram matrices.
+//   k_jacobi_cluster : the same for n <= 256 on a cluster, a pair of blocks a
+//                      CTA; k_jacobi_coop column pairs over the grid beyond.
+//   k_house_qr_blk :   Householder QR (LAPACK sign convention: beta =
+//                      -sign(alpha) ||x||, as geqrf/orgqr and MATLAB's qr(A,0))
+//                      of an m x n matrix in shared memory, in panels of
+//                      eight columns; forms the thin Q and R.  k_house_qr, a
+//                      column at a time, takes the shapes that fit only
+//                      without the panel's workspace.
+// Singular values descend.  One launch each, no host round trip.
 #include <cmath>
 #include <cstdlib>
 
@@ -1934,13 +1937,13 @@ int jacobi_cluster_size(int64_t n) {
 }
 
 // The cluster form runs where one CTA's shared memory cannot hold both A
-// and V (n > 113) up to JK_MAX_N, unless TTG_JACOBI_CLUSTER=0, when the device
+// and V (n > JS_MAX_N) up to JK_MAX_N, unless TTG_JACOBI_CLUSTER=0, when the device
 // can place a cluster with that shared memory (checked once per device and
 // size class: attributes set, cudaOccupancyMaxActiveClusters).  Outside a
 // grouped batch it also takes the sizes from TTG_JACOBI_CLUSTER_MIN_N (default
 // 48) up, which the one-CTA kernel could hold: a lone solve waits on each SVD
-// (triangular factor, cluster against one CTA: 0.31 against 0.71 ms at n = 47,
-// 0.18 against 0.31 at 32), while a grouped batch fills the GPU with concurrent
+// (triangular factor, cluster against one CTA: 0.18 / 0.16 ms at n = 32, 0.31 /
+// 0.31 at 47, 0.40 / 0.53 at 64, 0.58 / 1.18 at 96), while a grouped batch fills the GPU with concurrent
 // systems and wants the one-CTA kernel's single SM.  Below 48 both run the
 // one-CTA kernel, so that a grouped batch of such ranks repeats a lone solve.
 int64_t jacobi_cluster_min_n() {
