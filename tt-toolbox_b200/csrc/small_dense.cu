@@ -1943,9 +1943,10 @@ int jacobi_cluster_size(int64_t n) {
 // grouped batch it also takes the sizes from TTG_JACOBI_CLUSTER_MIN_N (default
 // 48) up, which the one-CTA kernel could hold: a lone solve waits on each SVD
 // (triangular factor, cluster against one CTA: 0.18 / 0.16 ms at n = 32, 0.31 /
-// 0.31 at 47, 0.40 / 0.53 at 64, 0.58 / 1.18 at 96), while a grouped batch fills the GPU with concurrent
-// systems and wants the one-CTA kernel's single SM.  Below 48 both run the
-// one-CTA kernel, so that a grouped batch of such ranks repeats a lone solve.
+// 0.31 at 47, 0.40 / 0.53 at 64, 0.58 / 1.18 at 96), while a grouped batch
+// fills the GPU with concurrent systems and wants the one-CTA kernel's single
+// SM.  Below 48 both run the one-CTA kernel, so that a grouped batch of such
+// ranks repeats a lone solve.
 int64_t jacobi_cluster_min_n() {
   static const int64_t v = [] {
     const char* e = getenv("TTG_JACOBI_CLUSTER_MIN_N");
