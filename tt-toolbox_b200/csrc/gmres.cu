@@ -220,7 +220,7 @@ TTG_BODY(k_hh_init)(TTG_BLOCK, HhArgs a, int it) {
     }
   }
 }
-TTG_COOP_KERNEL(k_hh_init, HH_THREADS);
+TTG_COOP_KERNEL(k_hh_init, HH_THREADS, COOP_CTAS);
 
 // One Arnoldi step around the matvec w2 = B v_j:
 //   w2 = P_j ... P_0 w2 = w2 - U T' (U' w2)                     (:421-427)
@@ -359,7 +359,7 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
       a.R[k + j * a.nrestart] = k <= j ? wl[k] : 0.0;
   }
 }
-TTG_COOP_KERNEL(k_hh_step, HH_THREADS);
+TTG_COOP_KERNEL(k_hh_step, HH_THREADS, COOP_CTAS);
 
 // y = R^{-1} tau, then sol += P_0 ... P_j (sum_i y_i e_i)
 //                        = sol + y - U T (U' y)                 (:487-507)
@@ -411,13 +411,13 @@ TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t ni) {
 TTG_KERNEL(k_hh_correct, HH_THREADS);
 
 // Blocks of the cooperative kernels: contiguous row ranges of at least HH_ROWS
-// rows, at most two blocks per SM.  Two keep twice the loads of U in flight
+// rows, at most two blocks per SM (Context::coop_ctas).  Two keep twice the loads of U in flight
 // (64 x 64 x 64, 80 steps: one block an SM takes 8 us a step longer); small systems take
 // few blocks, and 256 or 512 rows as the least share measure the same.
 constexpr int64_t HH_ROWS = 256;
 int coop_blocks(Context* c, const void* kernel, size_t smem, int64_t sz) {
-  const int64_t cap =
-      int64_t(c->num_sms) * std::max(1, std::min(max_active_blocks(kernel, HH_THREADS, smem), 2));
+  const int occ = std::max(1, max_active_blocks(kernel, HH_THREADS, smem));
+  const int64_t cap = int64_t(c->num_sms) * std::min(occ, c->coop_ctas);
   return int(std::max<int64_t>(1, std::min((sz + HH_ROWS - 1) / HH_ROWS, cap)));
 }
 

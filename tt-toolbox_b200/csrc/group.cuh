@@ -15,7 +15,11 @@
 // Helpers that read blockIdx/gridDim take them as parameters in the same way.
 // Cooperative bodies (bounded grid barriers on a per-launch counter) are
 // grouped into cooperative launches whose CTAs are all resident, so every
-// launch's barrier completes as in its own grid.
+// launch's barrier completes as in its own grid.  A solve sizes such a grid
+// with the plain entry's occupancy, so both entries are bound to the same
+// number of CTAs per SM: left to itself the compiler gives the grouped entry,
+// whose arguments come from memory, up to twice the registers, and half the
+// CTAs of the grid would fit.
 #pragma once
 
 #include <cstddef>
@@ -85,12 +89,20 @@ template <auto Body, int LB, class... A>
 __global__ void __launch_bounds__(LB) k_plain_lb(A... a) {
   Body(blockIdx, gridDim, a...);
 }
+template <auto Body, int LB, int CTAS, class... A>
+__global__ void __launch_bounds__(LB, CTAS) k_plain_coop(A... a) {
+  Body(blockIdx, gridDim, a...);
+}
 template <auto Body, class... A>
 __global__ void k_plain_nolb(A... a) {
   Body(blockIdx, gridDim, a...);
 }
 template <auto Body, int LB, class... A>
 __global__ void __launch_bounds__(LB) k_group_lb(GroupArgs g) {
+  group_call<Body, A...>(g, std::index_sequence_for<A...>{});
+}
+template <auto Body, int LB, int CTAS, class... A>
+__global__ void __launch_bounds__(LB, CTAS) k_group_coop(GroupArgs g) {
   group_call<Body, A...>(g, std::index_sequence_for<A...>{});
 }
 template <auto Body, class... A>
@@ -145,30 +157,36 @@ void rec_group(Recorder* r, const GroupInfo* info, dim3 grid, dim3 block, size_t
 // FLOPs (counted, and timed on request, by the executor).
 void rec_note_flop(Recorder* r, double flop);
 
-template <auto Body, int LB, bool COOP, class... A>
+// COOP: 0, or a cooperative kernel: the CTAs per SM that both entries are
+// bound to (-1: as many as their registers leave).
+template <auto Body, int LB, int COOP, class... A>
 struct Kern {
   using plain_t = void (*)(A...);
   using pack_t = Pack<A...>;
 #ifdef __CUDACC__
   static plain_t plain() {
-    if constexpr (LB > 0)
+    if constexpr (COOP > 0)
+      return &k_plain_coop<Body, LB, COOP, A...>;
+    else if constexpr (LB > 0)
       return &k_plain_lb<Body, LB, A...>;
     else
       return &k_plain_nolb<Body, A...>;
   }
   static const void* group() {
-    if constexpr (LB > 0)
+    if constexpr (COOP > 0)
+      return reinterpret_cast<const void*>(&k_group_coop<Body, LB, COOP, A...>);
+    else if constexpr (LB > 0)
       return reinterpret_cast<const void*>(&k_group_lb<Body, LB, A...>);
     else
       return reinterpret_cast<const void*>(&k_group_nolb<Body, A...>);
   }
   static void issue(const void* pack, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                     bool pdl) {
-    issue_plain<COOP, A...>(reinterpret_cast<const void*>(plain()), pack, grid, block, smem, s,
+    issue_plain<COOP != 0, A...>(reinterpret_cast<const void*>(plain()), pack, grid, block, smem, s,
                             pdl);
   }
   static const GroupInfo* info() {
-    static const GroupInfo gi{reinterpret_cast<const void*>(plain()), group(), COOP,
+    static const GroupInfo gi{reinterpret_cast<const void*>(plain()), group(), COOP != 0,
                               uint32_t(sizeof(pack_t)), uint32_t(alignof(pack_t)), &issue};
     return &gi;
   }
@@ -177,9 +195,9 @@ struct Kern {
 #endif
 };
 
-template <auto Body, int LB, bool COOP, class F>
+template <auto Body, int LB, int COOP, class F>
 struct KernOfT;
-template <auto Body, int LB, bool COOP, class... A>
+template <auto Body, int LB, int COOP, class... A>
 struct KernOfT<Body, LB, COOP, void (*)(uint3, dim3, A...)> {
   using type = Kern<Body, LB, COOP, A...>;
 };
@@ -190,13 +208,13 @@ struct KernOfT<Body, LB, COOP, void (*)(uint3, dim3, A...)> {
 #define TTG_BLOCK const uint3 blockIdx, const dim3 gridDim
 #define TTG_BODY(name) __device__ __forceinline__ void name##_body
 #define TTG_KERNEL(name, LB)                                                          \
-  constexpr typename ::ttg::KernOfT<name##_body, LB, false, decltype(&name##_body)>::type \
+  constexpr typename ::ttg::KernOfT<name##_body, LB, 0, decltype(&name##_body)>::type \
       name {}
-#define TTG_COOP_KERNEL(name, LB)                                                    \
-  constexpr typename ::ttg::KernOfT<name##_body, LB, true, decltype(&name##_body)>::type \
+#define TTG_COOP_KERNEL(name, LB, CTAS)                                              \
+  constexpr typename ::ttg::KernOfT<name##_body, LB, CTAS, decltype(&name##_body)>::type \
       name {}
 #define TTG_KERNEL_T(name, LB, ...)                                                   \
-  constexpr typename ::ttg::KernOfT<name##_body<__VA_ARGS__>, LB, false,             \
+  constexpr typename ::ttg::KernOfT<name##_body<__VA_ARGS__>, LB, 0,                 \
                                     decltype(&name##_body<__VA_ARGS__>)>::type name {}
 
 template <class... A, class... Args, size_t... I>
@@ -218,7 +236,7 @@ void run_grouped(Context* owner, int width, int64_t count,
 #ifdef __CUDACC__
 // Launch of a TTG_KERNEL on the context's stream, or its record when the
 // context belongs to a grouped batch.
-template <auto Body, int LB, bool COOP, class... A, class... Args>
+template <auto Body, int LB, int COOP, class... A, class... Args>
 void launch(Context* c, Kern<Body, LB, COOP, A...> k, dim3 grid, dim3 block, size_t smem,
             Args&&... args) {
   static_assert(sizeof...(A) == sizeof...(Args), "argument count");
@@ -229,7 +247,7 @@ void launch(Context* c, Kern<Body, LB, COOP, A...> k, dim3 grid, dim3 block, siz
     rec_group(c->rec, k.info(), grid, block, smem, &p);
     return;
   }
-  if constexpr (COOP) {
+  if constexpr (COOP != 0) {
     Pack<A...> p{};
     fill_pack(p, std::index_sequence_for<A...>{}, std::forward<Args>(args)...);
     void* kargs[sizeof...(A) + 1];

@@ -57,6 +57,9 @@ struct Error {
     if (!(cond)) ::ttg::fail(TTG_ERR_INVALID, __VA_ARGS__);                         \
   } while (0)
 
+// CTAs per SM of the cooperative Krylov grids.
+constexpr int COOP_CTAS = 2;
+
 // Number of per-tile arrival counters a context holds for split-K GEMMs.
 constexpr int64_t GEMM_TILE_COUNTERS = int64_t(1) << 16;
 
@@ -175,6 +178,8 @@ struct Context {
   int jacobi_max_sweeps = 40;
   // SM count the solves of a grouped batch size their grids with (0: share).
   int group_sms = 0;
+  // CTAs per SM (of num_sms) that the cooperative Krylov grids may take.
+  int coop_ctas = COOP_CTAS;
   // Per-output-tile arrival counters of split-K GEMMs (GEMM_TILE_COUNTERS,
   // zero between launches: the last slice of a tile resets its counter).
   unsigned* d_tile_cnt = nullptr;

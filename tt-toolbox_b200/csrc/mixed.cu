@@ -344,7 +344,7 @@ TTG_BODY(k_arnoldi)(TTG_BLOCK, ArArgs a, int j) {
   double* Hj = a.H + int64_t(m + 1) * j;
   for (int c = tid; c <= j + 1; c += 32) Hj[c] = ht[c];
 }
-TTG_COOP_KERNEL(k_arnoldi, AR_THREADS);
+TTG_COOP_KERNEL(k_arnoldi, AR_THREADS, COOP_CTAS);
 
 // V(:,0) = r / ||r||, g = [||r||, 0, ...]; scal[2] = ||r||.  On the first
 // restart (first != 0) r is the right-hand side: scal[3] = ||r||.  The stop
@@ -402,7 +402,7 @@ TTG_BODY(k_ar_init)(TTG_BLOCK, ArArgs a, const float* r, int first) {
     }
   }
 }
-TTG_COOP_KERNEL(k_ar_init, AR_THREADS);
+TTG_COOP_KERNEL(k_ar_init, AR_THREADS, COOP_CTAS);
 
 // x += V(:, 0:k) y with H(0:k,0:k) y = g(0:k) (upper triangular after Givens).
 TTG_BODY(k_ar_update)(TTG_BLOCK, ArArgs a, int k, float* x) {
@@ -494,7 +494,7 @@ struct Gmres32 {
     occ = max_active_blocks(k_arnoldi.fn(), AR_THREADS, arnoldi_smem());
     if (occ < 1) occ = 1;
     const int64_t want = (sz + AR_ROWS - 1) / AR_ROWS;
-    const int64_t cap = int64_t(c->num_sms) * std::min(occ, 2);
+    const int64_t cap = int64_t(c->num_sms) * std::min(occ, c->coop_ctas);
     blocks = int(std::max<int64_t>(1, std::min(want, cap)));
     part.reset(c, size_t(2) * (m + 2) * blocks);
     bar.reset(c, 4);

@@ -542,7 +542,7 @@ TTG_BODY(k_jacobi_coop)(TTG_BLOCK, int n, const double* __restrict__ Ain,
   }
   if (blockIdx.x == 0 && tid == 0 && sweep >= max_sweeps) atomicExch(sweep_err, 5);
 }
-TTG_COOP_KERNEL(k_jacobi_coop, JC_THREADS);
+TTG_COOP_KERNEL(k_jacobi_coop, JC_THREADS, -1);
 
 // ---------------------------------------------------------------------------
 // Block Jacobi SVD in one thread-block cluster, for n <= JK_MAX_N columns (the
@@ -878,7 +878,7 @@ TTG_BODY(k_jacobi_block)(TTG_BLOCK, int n, const double* __restrict__ Ain,
   }
   if (blockIdx.x == 0 && tid == 0 && sweep >= max_sweeps) atomicExch(sweep_err, 5);
 }
-TTG_COOP_KERNEL(k_jacobi_block, JB_THREADS);
+TTG_COOP_KERNEL(k_jacobi_block, JB_THREADS, -1);
 
 TTG_BODY(k_jacobi_finish)(TTG_BLOCK, int n, const double* A,
                                                              const double* V, double* U,
