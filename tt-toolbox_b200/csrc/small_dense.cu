@@ -93,27 +93,27 @@ __device__ __forceinline__ void jk_pair(int c, int r, int nb, int& p, int& q) {
 }
 
 // Cosine and sine of the rotation that makes a pair orthogonal, the smaller of
-// the two angles: with dd = be - al, g = 2 ga and h = hypot(dd, g),
-// c = sqrt((1 + |dd| / h) / 2) and s = |g| / (2 h c) with the sign of dd g.
-// They are first taken in single precision (dd and g scaled to a common
-// exponent), which leaves 1e-7 of the pair's inner product for the next sweep,
-// then both multiplied by 1 / sqrt(c^2 + s^2) in double precision (two terms
-// of the series: c^2 + s^2 - 1 is 1e-7), which leaves the rounding of c and s
-// alone.  c = 1 / sqrt(1 + t^2) taken directly is biased by 1e-16 for small t,
-// which adds up over a sweep's thousands of rotations.
+// the two angles: with dd = be - al, g = 2 ga (scaled to a common exponent) and
+// h = hypot(dd, g), c = sqrt((1 + |dd| / h) / 2) and s = |g| / (2 h c) with the
+// sign of dd g: two reciprocal roots, where the tangent takes a root, a quotient
+// and a reciprocal root.  Both are then multiplied by 1 / sqrt(c^2 + s^2) (two
+// terms of the series): a bias of 1e-16 in c^2 + s^2 adds up over a sweep's
+// thousands of rotations.
+// The angle takes double precision throughout: from single precision, the 1e-7
+// of a pair's inner product that it leaves comes to rest below the stopping
+// threshold in the last sweep, and the left factors of graded matrices lose
+// 10-45% of their orthogonality.
 __device__ __forceinline__ void jk_rotation(double al, double be, double ga, double& c,
                                             double& s) {
   const double dd = be - al, gg = 2.0 * ga;
-  // 2^-e for the exponent e of |dd| + |g|
-  const int field = 0x7fe00000 - (__double2hiint(fabs(dd) + fabs(gg)) & 0x7ff00000);
+  // 2^-e for the exponent e of |dd| + |g| (2^-1022 at the top of the range)
+  const int field = max(0x7fe00000 - (__double2hiint(fabs(dd) + fabs(gg)) & 0x7ff00000), 0x00100000);
   const double scale = __hiloint2double(field, 0);
-  const double y = fabs(gg) * scale;
-  const float x = float(fabs(dd) * scale), yf = float(y);
-  const float rh = rsqrtf(fmaf(x, x, yf * yf));
-  const float v = fmaf(0.5f * x, rh, 0.5f);  // c^2
-  const float rv = rsqrtf(v);
-  const double c0 = double(v * rv);
-  const double s0 = (0.5 * y) * double(rh * rv);
+  const double x = fabs(dd) * scale, y = fabs(gg) * scale;
+  const double rh = rsqrt(fma(x, x, y * y));
+  const double v = fma(0.5 * x, rh, 0.5);  // c^2
+  const double rv = rsqrt(v);
+  const double c0 = v * rv, s0 = 0.5 * y * rh * rv;
   const double d = fma(s0, s0, fma(c0, c0, -1.0));
   const double f = d * fma(0.375, d, -0.5);
   c = fma(c0, f, c0);
