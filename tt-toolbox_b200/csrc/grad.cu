@@ -534,13 +534,11 @@ void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, do
     w1max = std::max(w1max, z2);
     z1max = std::max(z1max, w2);
   }
-  // Every core's W2 and Z2 are kept between the sweeps and the gradient, and
-  // the sweeps then run side by side, unless that would hold too much memory:
-  // then the right sweep follows the left one and forms W2 again.
-  const bool keep = (woff[d] + zoff[d]) * int64_t(sizeof(double)) <= KEEP_MAX;
   DBuf<double> L(c, off[d + 1]), R(c, off[d + 1]);
-  DBuf<double> W1(c, w1max), Z1(c, z1max), W2(c, keep ? woff[d] : z1max),
-      Z2(c, keep ? zoff[d] : w1max);
+  DBuf<double> W1, Z1, W2, Z2;
+  bool keep = false;
+  auto W1p = [&] { return keep ? W1.p() : Z2.p(); };
+  auto Z1p = [&] { return keep ? Z1.p() : W2.p(); };
   auto W2k = [&](int64_t k) { return W2.p() + (keep ? woff[k] : 0); };
   auto Z2k = [&](int64_t k) { return Z2.p() + (keep ? zoff[k] : 0); };
   fill_f64(c, 1, 1.0, L.p());
@@ -561,18 +559,18 @@ void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, do
     const double* Rn = R.p() + off[k + 1];
     switch (which) {
       case LEFT1:
-        return {true, false, r1 * a1, n * r2, r1, Lk, r1, 0, xk, r1, 0, 0.0, W1.p(), r1 * a1, 0, 1};
+        return {true, false, r1 * a1, n * r2, r1, Lk, r1, 0, xk, r1, 0, 0.0, W1p(), r1 * a1, 0, 1};
       case LEFT2:
-        return {false, false, r1, n * a2, a1 * n, W1.p(), r1, r1 * a1 * n, Ak, a1 * n, 0, 0.0,
+        return {false, false, r1, n * a2, a1 * n, W1p(), r1, r1 * a1 * n, Ak, a1 * n, 0, 0.0,
                 W2k(k), r1, r1 * n * a2, r2};
       case LEFT3:
         return {true, false, r2, r2, r1 * n, W2k(k), r1 * n * a2, r1 * n, xk, r1 * n, 0, 0.0,
                 L.p() + off[k + 1], r2, r2 * r2, a2};
       case RIGHT1:
-        return {false, false, r1 * n, a2 * r2, r2, xk, r1 * n, 0, Rn, r2, 0, 0.0, Z1.p(), r1 * n,
+        return {false, false, r1 * n, a2 * r2, r2, xk, r1 * n, 0, Rn, r2, 0, 0.0, Z1p(), r1 * n,
                 0, 1};
       case RIGHT2:
-        return {false, true, r1, a1 * n, n * a2, Z1.p(), r1, r1 * n * a2, Ak, a1 * n, 0, 0.0,
+        return {false, true, r1, a1 * n, n * a2, Z1p(), r1, r1 * n * a2, Ak, a1 * n, 0, 0.0,
                 Z2k(k), r1, r1 * a1 * n, r2};
       case RIGHT3:
         return {false, true, r1 * a1, r1, n * r2, Z2k(k), r1 * a1, 0, xk, r1, 0, 0.0,
@@ -590,7 +588,14 @@ void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, do
     gemm_f64(c, o.tA, o.tB, o.M, o.N, o.K, 1.0, o.A, o.lda, o.sA, o.B, o.ldb, o.sB, o.beta, o.C,
              o.ldc, o.sC, o.batch);
   };
-  if (keep) {
+  // Every core's W2 and Z2 are kept between the sweeps and the gradient, and
+  // the sweeps then run side by side.
+  auto side_by_side = [&] {
+    keep = true;
+    W1.reset(c, w1max);
+    Z1.reset(c, z1max);
+    W2.reset(c, woff[d]);
+    Z2.reset(c, zoff[d]);
     for (int64_t k = 0; k < d; ++k) {
       const int64_t l = d - 1 - k;
       gemm_pair_f64(c, op(LEFT1, k), op(RIGHT1, l));
@@ -608,14 +613,33 @@ void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, do
       else
         one(KET, d - 1);
     }
-  } else {
+  };
+  // The right sweep follows the left one and forms W2 again: two buffers of
+  // the largest core, W1 in Z2's and Z1 in W2's.
+  auto one_by_one = [&] {
+    keep = false;
+    for (DBuf<double>* b : {&W1, &Z1, &W2, &Z2}) b->release();
+    W2.reset(c, z1max);
+    Z2.reset(c, w1max);
     for (int64_t k = 0; k < d; ++k)
       for (int which : {LEFT1, LEFT2, LEFT3}) one(which, k);
     for (int64_t k = d - 1; k >= 0; --k) {
-      for (int which : {RIGHT1, RIGHT2, BRA, LEFT1, LEFT2, KET}) one(which, k);
+      for (int which : {RIGHT1, RIGHT2, BRA}) one(which, k);
       if (k > 0) one(RIGHT3, k);
+      for (int which : {LEFT1, LEFT2, KET}) one(which, k);
+    }
+  };
+  // Side by side up to KEEP_MAX, where the device has the memory for it.
+  bool done = false;
+  if ((woff[d] + zoff[d]) * int64_t(sizeof(double)) <= KEEP_MAX) {
+    try {
+      side_by_side();
+      done = true;
+    } catch (const Error& e) {
+      if (e.code != TTG_ERR_ALLOC) throw;
     }
   }
+  if (!done) one_by_one();
   if (value) copy_f64(c, 1, L.p() + off[d], value);
 }
 
