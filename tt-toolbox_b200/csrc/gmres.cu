@@ -53,9 +53,9 @@ struct HhArgs {
   const double* rhs;
   double* tau;   // nrestart+1
   double* J;     // 2 x nrestart
-  double* R;     // nrestart x nrestart
-  double* T;     // (nrestart+1)^2: the WY factor, and its transpose
-  double* TT;
+  // (nrestart+1)^2: R in the upper triangle, and below it the transpose of the
+  // WY factor T, whose diagonal is 2: element (q, r) of T, q < r, at r + q ld.
+  double* RT;
   double* scal;  // [0] nrmrhs [1] curres [2] nrmr [3] exact-flag [4] w[j+1]
   double* part;  // 2 x (nrestart+2) x gridDim.x partial sums
   unsigned* bar; // [0] count [1] generation
@@ -214,10 +214,7 @@ TTG_BODY(k_hh_init)(TTG_BLOCK, HhArgs a, int it) {
   if (b == 0) {
     for (int64_t k = threadIdx.x; k <= a.nrestart; k += blockDim.x) a.tau[k] = 0.0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      a.tau[0] = -beta;
-      a.T[0] = a.TT[0] = 2.0;
-    }
+    if (threadIdx.x == 0) a.tau[0] = -beta;
   }
 }
 TTG_COOP_KERNEL(k_hh_init, HH_THREADS, COOP_CTAS);
@@ -254,7 +251,7 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
   hh_gather(a.part, nb, nr, sd);
   for (int64_t r = warp; r < nr; r += HH_WARPS) {  // T' (U' w2)
     double s = 0.0;
-    for (int64_t q = lane; q <= r; q += 32) s = fma(a.T[q + r * m1], sd[q], s);
+    for (int64_t q = lane; q <= r; q += 32) s = fma(q < r ? a.RT[r + q * m1] : 2.0, sd[q], s);
     s = warp_sum(s);
     if (lane == 0) sy[r] = s;
   }
@@ -297,7 +294,7 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
       for (int64_t q = warp; q < nr; q += HH_WARPS) {
         double t = 0.0, y = 0.0;
         for (int64_t r = q + lane; r < nr; r += 32) {
-          const double Tqr = a.TT[r + q * m1];
+          const double Tqr = r > q ? a.RT[r + q * m1] : 2.0;
           t = fma(Tqr, sd[r], t);
           y = fma(Tqr, su[r], y);
         }
@@ -305,10 +302,9 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
         y = warp_sum(y);
         if (lane == 0) {
           sy[q] = fma(t, uj1, y);
-          if (b == 0) a.T[q + nr * m1] = a.TT[nr + q * m1] = t;
+          if (b == 0) a.RT[nr + q * m1] = t;
         }
       }
-      if (b == 0 && tid == 0) a.T[nr + nr * m1] = a.TT[nr + nr * m1] = 2.0;
       __syncthreads();
       double* Un = a.U + nr * sz;
       const double yn = 2.0 * uj1;
@@ -355,8 +351,7 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
       }
     }
     __syncthreads();
-    for (int64_t k = tid; k < a.nrestart; k += blockDim.x)
-      a.R[k + j * a.nrestart] = k <= j ? wl[k] : 0.0;
+    for (int64_t k = tid; k <= j; k += blockDim.x) a.RT[k + j * m1] = wl[k];
   }
 }
 TTG_COOP_KERNEL(k_hh_step, HH_THREADS, COOP_CTAS);
@@ -375,12 +370,12 @@ TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t ni) {
   double* Rs = st + ni;
   if (staged)
     for (int64_t e = tid; e < ni * ni; e += blockDim.x)
-      Rs[e] = a.R[(e % ni) + (e / ni) * a.nrestart];
+      Rs[e] = a.RT[(e % ni) + (e / ni) * m1];
   for (int64_t e = tid; e < ni; e += blockDim.x) y[e] = a.tau[e];
   __syncthreads();
   if (warp == 0) {  // back-substitution, one column at a time
-    const double* R = staged ? Rs : a.R;
-    const int64_t ldr = staged ? ni : a.nrestart;
+    const double* R = staged ? Rs : a.RT;
+    const int64_t ldr = staged ? ni : m1;
     for (int64_t c = ni - 1; c >= 0; --c) {
       const double v = y[c] / R[c + c * ldr];
       __syncwarp();
@@ -399,7 +394,8 @@ TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t ni) {
   __syncthreads();
   for (int64_t q = warp; q < ni; q += HH_WARPS) {
     double s = 0.0;
-    for (int64_t r = q + lane; r < ni; r += 32) s = fma(a.TT[r + q * m1], sc[r], s);
+    for (int64_t r = q + lane; r < ni; r += 32)
+      s = fma(r > q ? a.RT[r + q * m1] : 2.0, sc[r], s);
     s = warp_sum(s);
     if (lane == 0) st[q] = s;
   }
@@ -430,7 +426,7 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
               (long long)nrestart);
   DBuf<double> U(c, size_t(sz) * (nrestart + 1)), w(c, sz), w2(c, sz);
   const int64_t m1 = nrestart + 1;
-  DBuf<double> small(c, m1 + 2 * nrestart + nrestart * nrestart + 2 * m1 * m1 + 8);
+  DBuf<double> small(c, m1 + 2 * nrestart + m1 * m1 + 8);
   const size_t step_smem = hh_step_smem(nrestart);
   ensure_smem_attr(k_hh_step.fn(), c->device, int(hh_step_smem(4096)));
   ensure_smem_attr(k_hh_correct.fn(), c->device, int(hh_correct_smem(4096, 4096)));
@@ -452,10 +448,8 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
   a.rhs = rhs;
   a.tau = small.p();
   a.J = a.tau + (nrestart + 1);
-  a.R = a.J + 2 * nrestart;
-  a.T = a.R + nrestart * nrestart;
-  a.TT = a.T + m1 * m1;
-  a.scal = a.TT + m1 * m1;
+  a.RT = a.J + 2 * nrestart;
+  a.scal = a.RT + m1 * m1;
   a.part = part.p();
   a.bar = bar.p();
   a.err = c->d_err;
