@@ -25,8 +25,10 @@
 #include <cuda_bf16.h>
 
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <mutex>
+#include <utility>
 
 #include "group.cuh"
 #include "mixed_ops.h"
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   if (skip && *skip) return;  // queued Krylov step after convergence (uniform)
   constexpr int ST = ps_stages<BN>();
   constexpr int B_BYTES = BN * UM_BK * 2;
-  constexpr uint32_t ACC = BN <= 128 ? 128 : 256;  // TMEM columns of an accumulator
+  constexpr uint32_t ACC = 256;  // TMEM columns of an accumulator
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
@@ -1010,9 +1012,7 @@ void MixedOp::prepare(Context* c, const MvDims& dd, const double* Phi1, const do
 // whatever the intermediates hold -- the values do not change the work) and
 // the fastest is kept for the life of the process.  The width only decides
 // which CTA computes which output columns; every output element is still
-// the same K-ordered sequence of MMA steps.  TTG_AUTOTUNE=0 turns tuning off
-// (the CTA-count heuristic pick_bn is used instead), e.g. for runs that must
-// repeat the same launch configuration.
+// the same K-ordered sequence of MMA steps.
 // ---------------------------------------------------------------------------
 
 namespace {
@@ -1033,12 +1033,27 @@ struct TuneKey {
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tuned;
 
-bool autotune_enabled() {
-  static const bool on = [] {
+// TTG_AUTOTUNE: 0 takes pick_bn's width (a CTA-count heuristic) without timing,
+// for runs that must repeat the same launch configuration; 64, 128, 256, p192
+// or p256 takes that tile for every stage (p: the persistent form, outside a
+// grouped batch), so that each form can be compared with the others.
+struct Tuning {
+  bool on = true;
+  int tile = 0;
+};
+const Tuning& tuning() {
+  static const Tuning t = [] {
+    Tuning v;
     const char* e = getenv("TTG_AUTOTUNE");
-    return !(e && e[0] == '0');
+    if (!e) return v;
+    v.on = e[0] != '0';
+    const std::pair<const char*, int> names[] = {
+        {"64", 64}, {"128", 128}, {"256", 256}, {"p192", BN_PERS + 192}, {"p256", BN_PERS + 256}};
+    for (const auto& n : names)
+      if (!strcmp(e, n.first)) v.tile = n.second;
+    return v;
   }();
-  return on;
+  return t;
 }
 
 }  // namespace
@@ -1070,7 +1085,8 @@ int MixedOp::tuned_bn(Context* c, int stage) {
     M = d.ry2 * d.n; N = d.ry1; K = d.rx1 * d.ra1;
   }
   const int fallback = pick_bn(c, M, N, batch);
-  if (!autotune_enabled() || c->skip) return fallback;
+  if (const int bn = tuning().tile) return c->rec && bn >= BN_PERS ? fallback : bn;
+  if (!tuning().on || c->skip) return fallback;
   const TuneKey key{c->device, stage, M, N, K, batch};
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
