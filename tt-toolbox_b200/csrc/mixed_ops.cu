@@ -1293,12 +1293,13 @@ void rev_to_nat_add(Context* c, int64_t r1, int64_t n, int64_t r2, const float* 
 }
 
 void rev_to_nat(Context* c, int64_t r1, int64_t n, int64_t r2, const float* y, double* x) {
-  const int64_t tiles = rev_tiles(r1, n, r2), half = tiles / 2;
-  launch(c, k_rev_to_nat<false>, rev_blocks(c, half), dim3(32, 8), 0, r1, n, r2, y, x, 1.0,
-         int64_t(0), half);
-  launch(c, k_rev_to_nat<false>, rev_blocks(c, tiles - half), dim3(32, 8), 0, r1, n, r2, y, x, 1.0,
-         half, tiles);
-  TTG_CHECK_LAUNCH();
+  const int64_t tiles = rev_tiles(r1, n, r2);
+  for (int64_t t0 = 0, t1 = tiles / 2; t0 < tiles; t0 = t1, t1 = tiles) {
+    if (t1 == t0) continue;  // a single tile
+    launch(c, k_rev_to_nat<false>, rev_blocks(c, t1 - t0), dim3(32, 8), 0, r1, n, r2, y, x, 1.0,
+           t0, t1);
+    TTG_CHECK_LAUNCH();
+  }
 }
 
 namespace {
