@@ -217,9 +217,11 @@ TTG_KERNEL_T(k_gemm_f64, GEMM_THREADS, BM, BN, TA, TB);
 // product's grid g1, the others the second's.  For chains of short products
 // that run side by side (the left and right sweeps of a gradient), which are
 // bound by each launch's chain of first loads, k loop and stores: sharing the
-// launches takes the gradient of <x, A x> at d = 12, n = 32, rank 64 from 721 to
-// 580 us (six cores of 8, rank 16: 177 to 134).  Up to 198 registers a thread:
-// at 128, with more CTAs on an SM, the gradient takes 9% longer.
+// launches takes the gradient of <x, A x> at d = 12, n = 32, rank 64 from 696 to
+// 580 us (six cores of 8, rank 16: 167 to 128; twenty of 4, rank 24: 514 to 366).
+// 189-190 registers a thread with 32 x 32 tiles, 212-214 with 32 x 64, 255 with
+// 64 x 64: at 128, with more CTAs on an SM, the first of these takes 646 us (the
+// others 129 and 361).
 template <int BM, int BN, bool TA1, bool TB1, bool TA2, bool TB2>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     k_gemm_pair(GemmP p, GemmP q, dim3 g1, dim3 g2) {
@@ -683,15 +685,28 @@ void pair_launch(Context* c, const GemmP& p, const GemmP& q, dim3 g1, dim3 g2) {
   TTG_CHECK_LAUNCH();
 }
 
-// Partials of one tile that the last slice of a pair sums: 12 slices of 32 x 32
-// (the gradient above takes 3% longer with 8, 5% with 16: one CTA reads them).
+// Partials of one tile that the last slice of a pair sums: 12 slices of 32 x 32.
+// The first gradient above takes 656, 593, 580, 622 us with 4, 8, 12, 16 (one CTA
+// reads them); d = 8, n = 24, rank 50 285, 274, 273, 273; six cores of 8, rank 16,
+// d = 8, n = 16, rank 32 and ranks from 128 on do not move by more than 2% (rank
+// 128 with 4: 8%).
 constexpr int64_t PAIR_SPLITK_MAX = 12288;
+// Work of the two products up to which they share a launch: 7 us at the FP64
+// tensor rate, about a launch's own chain.  Longer ones fill the device by
+// themselves, with more CTAs on an SM than the pair kernel's registers leave:
+// gradient of <x, A x>, shared / apart, d = 12, n = 32, rank 64 (150 MFLOP a
+// pair) 580 / 696 us, d = 10, n = 32, rank 80 (130) 594 / 632; d = 6, n = 32, rank
+// 100, operator rank 3 (380) 643 / 610; d = 5, n = 64, rank 128 (1600) 1194 /
+// 1172; d = 4, n = 48, rank 200 (3100) 1513 / 1235.
+constexpr double PAIR_FLOP_MAX = 256e6;
 
 template <bool TA1, bool TB1, bool TA2, bool TB2>
 bool pair_f64(Context* c, const GemmOp& a, const GemmOp& b) {
   if (c->rec || !c->alloc || !c->d_tile_cnt) return false;
   for (const GemmOp* o : {&a, &b})  // gemm_f64 refuses these
     if (o->batch > 65535 || (o->N + 63) / 64 > 65535 || (o->M + 63) / 64 > 0x7fffffff) return false;
+  auto flop = [](const GemmOp& o) { return 2.0 * double(o.M) * double(o.N) * double(o.K) * double(o.batch); };
+  if (flop(a) + flop(b) > PAIR_FLOP_MAX) return false;
   // Each product plans for half the device, with the first one's tile, and
   // sums its slices in the kernel.
   const int64_t sms = std::max(1, c->num_sms / 2);
