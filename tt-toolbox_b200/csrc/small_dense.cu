@@ -110,7 +110,9 @@ __device__ __forceinline__ void jk_rotation(double al, double be, double ga, dou
   const int field = max(0x7fe00000 - (__double2hiint(fabs(dd) + fabs(gg)) & 0x7ff00000), 0x00100000);
   const double scale = __hiloint2double(field, 0);
   const double x = fabs(dd) * scale, y = fabs(gg) * scale;
-  const double rh = rsqrt(fma(x, x, y * y));
+  // (a pair of zero columns keeps clear of rsqrt's special cases, which take a
+  // call: 18% of an SVD whose last block is padded)
+  const double rh = rsqrt(fmax(fma(x, x, y * y), 0.25));
   const double v = fma(0.5 * x, rh, 0.5);  // c^2
   const double rv = rsqrt(v);
   const double c0 = v * rv, s0 = 0.5 * y * rh * rv;
