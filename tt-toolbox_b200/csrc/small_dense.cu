@@ -11,8 +11,9 @@
 //                      -sign(alpha) ||x||, as geqrf/orgqr and MATLAB's qr(A,0))
 //                      of an m x n matrix in shared memory, in panels of
 //                      eight columns; forms the thin Q and R.  k_house_qr, a
-//                      column at a time, takes the shapes that fit only
-//                      without the panel's workspace.
+//                      column at a time, takes the shapes of two or three
+//                      reflectors and those that fit only without the panel's
+//                      workspace.
 // Singular values descend.  One launch each, no host round trip.
 #include <cmath>
 #include <cstdlib>
@@ -1886,8 +1887,14 @@ bool small_qr_fits(int64_t m, int64_t n) {
 void small_qr_f64(Context* c, int64_t m, int64_t n, const double* A, int64_t lda, double* Q,
                   double* R) {
   // The blocked kernel where its padded columns fit (the element-wise one is
-  // left with shapes like 4 x 5000 and 20000 x 1).
-  if (qb_smem(m, n) <= QB_SMEM) {
+  // left with shapes like 4 x 5000) and there are more than a few reflectors:
+  // its panel takes eight columns' steps whatever their number.  Blocked
+  // against one reflector at a time: 64 x 1 30.0 / 20.9 us, 1 x 512 41 / 19, 2048
+  // x 2 40 / 32, 2 x 512 43 / 30, 3 x 256 40 / 31, 3 x 512 43 / 40; but 1024 x 3
+  // 30 / 40, 4 x 512 44 / 53, 512 x 4 28 / 33; the same (28) at 4 x 4, 64 x 3 and
+  // between.
+  const int64_t k = std::min(m, n);
+  if (k > (n > m ? 3 : 2) && qb_smem(m, n) <= QB_SMEM) {
     ensure_smem_attr(k_house_qr_blk.fn(), c->device, int(QB_SMEM));
     launch(c, k_house_qr_blk, 1, QB_THREADS, qb_smem(m, n), int(m), int(n), A, int(lda), Q, R,
            c->skip);
