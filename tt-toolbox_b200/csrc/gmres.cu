@@ -34,6 +34,11 @@ constexpr long long BAR_SPIN_LIMIT = 1LL << 24;
 // Restart lengths up to which k_hh_correct stages R in shared memory.
 constexpr int64_t HH_CORRECT_STAGE_MAX = 64;
 
+// Restart lengths up to which T is kept a second time (34 MB at most) in the
+// order that T' (U' w2) reads it; beyond, those reads are strided.  64 x 64 x 64, a
+// restart of 250: 67.8 ms for 68.5; of 900: 774 for 822; of 120 and less the same.
+constexpr int64_t HH_OWN_T_MAX = 2048;
+
 // Shared memory of k_hh_step: three vectors over the reflectors and the
 // per-warp partial inner products (the Givens section reuses the space).
 size_t hh_step_smem(int64_t nrestart) {
@@ -53,9 +58,13 @@ struct HhArgs {
   const double* rhs;
   double* tau;   // nrestart+1
   double* J;     // 2 x nrestart
-  // (nrestart+1)^2: R in the upper triangle, and below it the transpose of the
-  // WY factor T, whose diagonal is 2: element (q, r) of T, q < r, at r + q ld.
-  double* RT;
+  // R (upper triangle, ld nrestart + 2) and, from the row below its diagonal on, the
+  // transpose TT of the WY factor (lower triangle) in one array; T itself, element
+  // (q, r) at q tq + r tr: the same entries, or for short restarts an array of its own.
+  double* R;
+  double* TT;
+  double* T;
+  int64_t tq, tr;
   double* scal;  // [0] nrmrhs [1] curres [2] nrmr [3] exact-flag [4] w[j+1]
   double* part;  // 2 x (nrestart+2) x gridDim.x partial sums
   unsigned* bar; // [0] count [1] generation
@@ -214,7 +223,10 @@ TTG_BODY(k_hh_init)(TTG_BLOCK, HhArgs a, int it) {
   if (b == 0) {
     for (int64_t k = threadIdx.x; k <= a.nrestart; k += blockDim.x) a.tau[k] = 0.0;
     __syncthreads();
-    if (threadIdx.x == 0) a.tau[0] = -beta;
+    if (threadIdx.x == 0) {
+      a.tau[0] = -beta;
+      a.T[0] = a.TT[0] = 2.0;
+    }
   }
 }
 TTG_COOP_KERNEL(k_hh_init, HH_THREADS, COOP_CTAS);
@@ -235,7 +247,7 @@ TTG_COOP_KERNEL(k_hh_init, HH_THREADS, COOP_CTAS);
 TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
   if (*(volatile int*)a.stop) return;  // queued after convergence
   extern __shared__ double hsm[];
-  const int64_t sz = a.sz, m1 = a.nrestart + 1, nr = j + 1;
+  const int64_t sz = a.sz, m1 = a.nrestart + 1, ld = m1 + 1, nr = j + 1;
   const int64_t nb = gridDim.x, b = blockIdx.x;
   const int64_t i0 = row_at(sz, b, nb), i1 = row_at(sz, b + 1, nb);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -251,7 +263,7 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
   hh_gather(a.part, nb, nr, sd);
   for (int64_t r = warp; r < nr; r += HH_WARPS) {  // T' (U' w2)
     double s = 0.0;
-    for (int64_t q = lane; q <= r; q += 32) s = fma(q < r ? a.RT[r + q * m1] : 2.0, sd[q], s);
+    for (int64_t q = lane; q <= r; q += 32) s = fma(a.T[q * a.tq + r * a.tr], sd[q], s);
     s = warp_sum(s);
     if (lane == 0) sy[r] = s;
   }
@@ -294,7 +306,7 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
       for (int64_t q = warp; q < nr; q += HH_WARPS) {
         double t = 0.0, y = 0.0;
         for (int64_t r = q + lane; r < nr; r += 32) {
-          const double Tqr = r > q ? a.RT[r + q * m1] : 2.0;
+          const double Tqr = a.TT[r + q * ld];
           t = fma(Tqr, sd[r], t);
           y = fma(Tqr, su[r], y);
         }
@@ -302,9 +314,10 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
         y = warp_sum(y);
         if (lane == 0) {
           sy[q] = fma(t, uj1, y);
-          if (b == 0) a.RT[nr + q * m1] = t;
+          if (b == 0) a.T[q * a.tq + nr * a.tr] = a.TT[nr + q * ld] = t;
         }
       }
+      if (b == 0 && tid == 0) a.T[nr * a.tq + nr * a.tr] = a.TT[nr + nr * ld] = 2.0;
       __syncthreads();
       double* Un = a.U + nr * sz;
       const double yn = 2.0 * uj1;
@@ -351,7 +364,7 @@ TTG_BODY(k_hh_step)(TTG_BLOCK, HhArgs a, int64_t j) {
       }
     }
     __syncthreads();
-    for (int64_t k = tid; k <= j; k += blockDim.x) a.RT[k + j * m1] = wl[k];
+    for (int64_t k = tid; k <= j; k += blockDim.x) a.R[k + j * ld] = wl[k];
   }
 }
 TTG_COOP_KERNEL(k_hh_step, HH_THREADS, COOP_CTAS);
@@ -362,7 +375,7 @@ TTG_COOP_KERNEL(k_hh_step, HH_THREADS, COOP_CTAS);
 TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t ni) {
   pdl_begin();
   extern __shared__ double y[];  // y (ni), U' y (ni), T U' y (ni), R when staged (ld ni)
-  const int64_t sz = a.sz, m1 = a.nrestart + 1;
+  const int64_t sz = a.sz, ld = a.nrestart + 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool staged = a.nrestart <= HH_CORRECT_STAGE_MAX;
   double* sc = y + ni;
@@ -370,12 +383,12 @@ TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t ni) {
   double* Rs = st + ni;
   if (staged)
     for (int64_t e = tid; e < ni * ni; e += blockDim.x)
-      Rs[e] = a.RT[(e % ni) + (e / ni) * m1];
+      Rs[e] = a.R[(e % ni) + (e / ni) * ld];
   for (int64_t e = tid; e < ni; e += blockDim.x) y[e] = a.tau[e];
   __syncthreads();
   if (warp == 0) {  // back-substitution, one column at a time
-    const double* R = staged ? Rs : a.RT;
-    const int64_t ldr = staged ? ni : m1;
+    const double* R = staged ? Rs : a.R;
+    const int64_t ldr = staged ? ni : ld;
     for (int64_t c = ni - 1; c >= 0; --c) {
       const double v = y[c] / R[c + c * ldr];
       __syncwarp();
@@ -394,8 +407,7 @@ TTG_BODY(k_hh_correct)(TTG_BLOCK, HhArgs a, int64_t ni) {
   __syncthreads();
   for (int64_t q = warp; q < ni; q += HH_WARPS) {
     double s = 0.0;
-    for (int64_t r = q + lane; r < ni; r += 32)
-      s = fma(r > q ? a.RT[r + q * m1] : 2.0, sc[r], s);
+    for (int64_t r = q + lane; r < ni; r += 32) s = fma(a.TT[r + q * ld], sc[r], s);
     s = warp_sum(s);
     if (lane == 0) st[q] = s;
   }
@@ -426,7 +438,9 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
               (long long)nrestart);
   DBuf<double> U(c, size_t(sz) * (nrestart + 1)), w(c, sz), w2(c, sz);
   const int64_t m1 = nrestart + 1;
-  DBuf<double> small(c, m1 + 2 * nrestart + m1 * m1 + 8);
+  const int64_t ld = m1 + 1, square = ld * m1;
+  const bool own_t = nrestart <= HH_OWN_T_MAX;
+  DBuf<double> small(c, m1 + 2 * nrestart + (own_t ? 2 : 1) * square + 8);
   const size_t step_smem = hh_step_smem(nrestart);
   ensure_smem_attr(k_hh_step.fn(), c->device, int(hh_step_smem(4096)));
   ensure_smem_attr(k_hh_correct.fn(), c->device, int(hh_correct_smem(4096, 4096)));
@@ -448,8 +462,12 @@ GmresResult gmres_hh_f64(Context* c, const ApplyFn& apply, const double* rhs, in
   a.rhs = rhs;
   a.tau = small.p();
   a.J = a.tau + (nrestart + 1);
-  a.RT = a.J + 2 * nrestart;
-  a.scal = a.RT + m1 * m1;
+  a.R = a.J + 2 * nrestart;
+  a.TT = a.R + 1;
+  a.T = own_t ? a.R + square : a.TT;
+  a.tq = own_t ? 1 : ld;
+  a.tr = own_t ? m1 : 1;
+  a.scal = a.R + (own_t ? 2 : 1) * square;
   a.part = part.p();
   a.bar = bar.p();
   a.err = c->d_err;
