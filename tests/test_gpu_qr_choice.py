@@ -13,9 +13,9 @@ import ttgpu
 pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-SINGLE = [(1, 1), (64, 1), (512, 1), (1, 64), (1, 512), (2, 2), (2, 300), (2000, 2), (3, 4),
-          (3, 256)]
-BLOCKED = [(3, 3), (4, 3), (1000, 3), (4, 4), (4, 64), (64, 4), (9, 9)]
+SINGLE = [(1, 1), (64, 1), (512, 1), (1, 64), (1, 512), (2, 2), (2, 300), (2000, 2), (3, 3),
+          (3, 4), (4, 3), (3, 256), (256, 3)]
+BLOCKED = [(257, 3), (1000, 3), (4, 4), (4, 64), (64, 4), (9, 9)]
 
 CHILD = r"""
 import os, sys

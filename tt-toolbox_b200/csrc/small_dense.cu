@@ -1888,13 +1888,14 @@ void small_qr_f64(Context* c, int64_t m, int64_t n, const double* A, int64_t lda
                   double* R) {
   // The blocked kernel where its padded columns fit (the element-wise one is
   // left with shapes like 4 x 5000) and there are more than a few reflectors:
-  // its panel takes eight columns' steps whatever their number.  Blocked
-  // against one reflector at a time: 64 x 1 30.0 / 20.9 us, 1 x 512 41 / 19, 2048
-  // x 2 40 / 32, 2 x 512 43 / 30, 3 x 256 40 / 31, 3 x 512 43 / 40; but 1024 x 3
-  // 30 / 40, 4 x 512 44 / 53, 512 x 4 28 / 33; the same (28) at 4 x 4, 64 x 3 and
-  // between.
+  // its panel takes eight columns' steps whatever their number.  Device time,
+  // blocked / one reflector at a time: 2 x 2 6.8 / 4.9 us, 400 x 2 9.1 / 6.8, 2 x
+  // 400 21.3 / 11.5, 3 x 3 7.9 / 6.9, 200 x 3 9.3 / 8.8, 3 x 400 22.3 / 20.3; but
+  // 400 x 3 10.3 / 10.8, 1600 x 3 18.1 / 22.4, 4 x 4 8.9 / 8.9, 100 x 4 10.1 / 10.7,
+  // 4 x 400 23.4 / 28.8.
   const int64_t k = std::min(m, n);
-  if (k > (n > m ? 3 : 2) && qb_smem(m, n) <= QB_SMEM) {
+  const bool few = k <= 2 || (k == 3 && m <= 256);
+  if (!few && qb_smem(m, n) <= QB_SMEM) {
     ensure_smem_attr(k_house_qr_blk.fn(), c->device, int(QB_SMEM));
     launch(c, k_house_qr_blk, 1, QB_THREADS, qb_smem(m, n), int(m), int(n), A, int(lda), Q, R,
            c->skip);
