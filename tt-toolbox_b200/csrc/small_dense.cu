@@ -94,12 +94,11 @@ __device__ __forceinline__ void jk_pair(int c, int r, int nb, int& p, int& q) {
 }
 
 // Cosine and sine of the rotation that makes a pair orthogonal, the smaller of
-// the two angles: with dd = be - al, g = 2 ga (scaled to a common exponent) and
-// h = hypot(dd, g), c = sqrt((1 + |dd| / h) / 2) and s = |g| / (2 h c) with the
+// the two angles: with dd = be - al, g = 2 ga (scaled by the exponent of al + be)
+// and h = hypot(dd, g), c = sqrt((1 + |dd| / h) / 2) and s = |g| / (2 h c) with the
 // sign of dd g: two reciprocal roots, where the tangent takes a root, a quotient
-// and a reciprocal root.  Both are then multiplied by 1 / sqrt(c^2 + s^2) (two
-// terms of the series): a bias of 1e-16 in c^2 + s^2 adds up over a sweep's
-// thousands of rotations.
+// and a reciprocal root.  Both are then multiplied by 1 / sqrt(c^2 + s^2): a bias
+// of 1e-16 in c^2 + s^2 adds up over a sweep's thousands of rotations.
 // The angle takes double precision throughout: from single precision, the 1e-7
 // of a pair's inner product that it leaves comes to rest below the stopping
 // threshold in the last sweep, and the left factors of graded matrices lose
@@ -107,20 +106,19 @@ __device__ __forceinline__ void jk_pair(int c, int r, int nb, int& p, int& q) {
 __device__ __forceinline__ void jk_rotation(double al, double be, double ga, double& c,
                                             double& s) {
   const double dd = be - al, gg = 2.0 * ga;
-  // 2^-e for the exponent e of |dd| + |g| (2^-1022 at the top of the range)
-  const int field = max(0x7fe00000 - (__double2hiint(fabs(dd) + fabs(gg)) & 0x7ff00000), 0x00100000);
+  // 2^-e for the exponent e of al + be (2^-1022 at the top of the range)
+  const int field = max(0x7fe00000 - (__double2hiint(al + be) & 0x7ff00000), 0x00100000);
   const double scale = __hiloint2double(field, 0);
   const double x = fabs(dd) * scale, y = fabs(gg) * scale;
   // (a pair of zero columns keeps clear of rsqrt's special cases, which take a
   // call: 18% of an SVD whose last block is padded)
-  const double rh = rsqrt(fmax(fma(x, x, y * y), 0.25));
+  const double rh = rsqrt(fmax(fma(x, x, y * y), 1e-200));
   const double v = fma(0.5 * x, rh, 0.5);  // c^2
   const double rv = rsqrt(v);
   const double c0 = v * rv, s0 = 0.5 * y * rh * rv;
-  const double d = fma(s0, s0, fma(c0, c0, -1.0));
-  const double f = d * fma(0.375, d, -0.5);
-  c = fma(c0, f, c0);
-  s = fma(s0, f, s0);
+  const double d = fma(s0, s0, fma(c0, c0, -1.0));  // some 1e-16
+  c = fma(-0.5 * c0, d, c0);
+  s = fma(-0.5 * s0, d, s0);
   if ((dd >= 0.0) != (gg > 0.0) && dd != 0.0) s = -s;
 }
 
