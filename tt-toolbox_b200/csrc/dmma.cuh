@@ -31,10 +31,9 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
 
 constexpr int TILE_K = 16;  // k extent of the FP64 operand tiles
 
-// One operand tile of T rows (of C) by TILE_K in shared memory, filled by NT threads, in
-// the order its
-// global layout has: k contiguous (KC) as rows of TILE_K + 4, else k slices of
-// T + 4.  Either pitch is 4 mod 16 doubles, which puts the 16 doubles that a
+// One operand tile of T rows (of C) by TILE_K in shared memory, filled by NT
+// threads in the order of its global layout: k contiguous (KC) as rows of
+// TILE_K + 4, else k slices of T + 4.  Either pitch is 4 mod 16 doubles, which puts the 16 doubles that a
 // half-warp reads for an mma fragment (4 of k by 4 rows) in different banks.
 template <int T, bool KC, int NT>
 struct TileS {

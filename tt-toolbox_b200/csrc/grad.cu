@@ -25,7 +25,7 @@
 //   core k at slice j is sum over samples with i_k = j of l_k(s)^T rho_k(s)^T.
 //   Samples are bucketed by i_k (stable counting sort, deterministic), and
 //   every product becomes a gathered GEMM on the FP64 tensor cores: the CTA
-//   owns 64 samples of one bucket, stages their vectors (gathered rows) and
+//   owns 128 samples of one bucket, stages their vectors (gathered rows) and
 //   the bucket's slice in shared memory and multiplies with mma.m8n8k4.  The
 //   gradient is a split-K GEMM per bucket (512 samples per CTA) whose
 //   partials are summed in a fixed order, so results are bitwise repeatable.
@@ -505,9 +505,10 @@ void check_tt_vector(const ttg_tt_s* x, const char* what) {
 
 // ---------------------------------------------------------------------------
 // <x, A x>: eight products per core (three each way for the interfaces, two
-// for the gradient).  Bound by the chain of some 120 dependent launches of
-// 5-10 us: d = 12, n = 32, rank 64 721 us, against 1151 us with two whole local
-// matvecs and three permutations per core.
+// for the gradient), shared by the two sweeps two to a launch where they are
+// short.  Bound by the chain of 49 dependent launches of 11-12 us: d = 12, n = 32,
+// rank 64 580 us, against 1151 us with two whole local matvecs and three
+// permutations per core and 696 us with one launch per product.
 // ---------------------------------------------------------------------------
 void grad_xAx(Context* c, const ttg_tt_s* x, const ttg_tt_s* A, double* grad, double* value) {
   check_tt_vector(x, "x");

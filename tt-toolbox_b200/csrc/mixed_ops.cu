@@ -15,11 +15,15 @@
 //   stage 3  y[(k,j), i] = T2[(k,j),(a,al)] * Phi1T[i,(a,al)]        K = rx1*ra1
 //            written straight into the reversed vector layout (FP32).
 //
-// One CTA computes a 128 x BN tile: warp 0 issues TMA loads into a 3-stage
-// shared-memory ring, one thread of warp 1 issues tcgen05.mma (M=128, N=BN,
-// K=16) and commits to mbarriers, and all four warps drain the FP32
-// accumulator from tensor memory (tcgen05.ld) in the epilogue.  All waits
-// are bounded; a timeout sets the context error flag.
+// A GEMM runs in one of two forms, by a timing of each stage's shape.  In the
+// plain one a CTA computes a 128 x BN tile, BN = 64, 128 or 256: warp 0 issues
+// TMA loads into a 3-stage shared-memory ring, one thread of warp 1 issues
+// tcgen05.mma (M=128, N=BN, K=16) and commits to mbarriers, and all four warps
+// drain the FP32 accumulator from tensor memory (tcgen05.ld) in the epilogue.
+// In the persistent one (products of many tiles) one CTA per SM walks tiles of
+// 128 x 192 or 128 x 256 with two accumulators, so that eight warps drain one
+// while the next is formed.  All waits are bounded; a timeout sets the context
+// error flag.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>

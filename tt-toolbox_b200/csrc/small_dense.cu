@@ -209,8 +209,8 @@ __device__ __forceinline__ int jk_rotate(double* sG, double* sJ, bool all, doubl
 // rotates no pair ends the iteration (|ga| <= 4 eps sqrt(al be) for all).
 // Bound by the chain of rotation steps, about 700 cycles each, n of them per
 // sweep where one pair per warp took n barriers and as many passes over the
-// columns.  Triangular factor: 0.085 ms for 0.132 at n = 16, 0.155 for 0.306 at
-// 32, 0.32 for 0.71 at 47.
+// columns.  Triangular factors (mean of six): 0.066 ms for 0.107 at n = 16, 0.244
+// for 0.318 at 33, 0.264 for 0.547 at 47.
 // Status: *err = 5 if the sweep limit is reached.
 // ---------------------------------------------------------------------------
 
@@ -406,8 +406,9 @@ __device__ void jacobi_finish(int n, const double* A, const double* V, double* _
 // ---------------------------------------------------------------------------
 // Grid-wide one-sided Jacobi SVD for matrices too large for one CTA's shared
 // memory: one CTA per column pair of a round-robin round, a bounded grid
-// barrier between rounds (cooperative launch), the same rotation and
-// stopping rule as k_jacobi_svd.
+// barrier between rounds (cooperative launch).  The rotation of a pair is that of
+// k_jacobi_svd, taken from the columns' own inner products by the tangent, with
+// the same stopping rule.
 // ---------------------------------------------------------------------------
 
 constexpr int JC_THREADS = 256;
@@ -566,9 +567,9 @@ TTG_COOP_KERNEL(k_jacobi_coop, JC_THREADS, -1);
 // sweep that rotates no pair ends the iteration: k_jacobi_svd's stopping rule.
 // Bound by the chain of rounds, 7.5 us each at n = 256: the eight rotation steps
 // on one warp 3 us, [A; V] J 1.8, the Gram matrix 1.1, loads and the barrier
-// 1.3.  Whole SVD of a triangular factor, against one column pair per warp and a
-// cluster barrier per column round: 2.75 ms for 9.8 at n = 256, 0.95 for 2.1 at
-// 128, 0.43 for 0.69 at 64, with the same errors against 64 bits.
+// 1.3.  Whole SVD of triangular factors (mean of six), against one column pair per
+// warp and a cluster barrier per column round: 2.26 ms for 7.98 at n = 256, 0.99 for
+// 1.93 at 130, 0.46 for 0.68 at 65, with the same errors against 64 bits.
 // All CTAs of a cluster are co-resident by construction, and every CTA takes
 // the same number of rounds (the stopping decision is read by all from the
 // same published values): the barriers cannot wait for a CTA that is not
