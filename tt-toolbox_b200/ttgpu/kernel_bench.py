@@ -301,7 +301,7 @@ def _kernel_table(run, top=30, top_shapes=25):
                 name = name[:i]
                 break
         # grouped / plain entries of a kernel body: name the body
-        m = re.match(r"k_(plain|group)_(?:no)?lb<&\(?(\w+?)_body(<[^>]*>)?", name)
+        m = re.match(r"k_(plain|group)_(?:lb|nolb|coop)<&\(?(?:void )?(\w+?)_body(<[^>]*>)?", name)
         if m:
             return "%s%s%s" % (m.group(2), m.group(3) or "", " [grouped]" if m.group(1) == "group"
                                 else "")
