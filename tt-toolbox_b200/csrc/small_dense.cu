@@ -11,9 +11,9 @@
 //                      -sign(alpha) ||x||, as geqrf/orgqr and MATLAB's qr(A,0))
 //                      of an m x n matrix in shared memory, in panels of
 //                      eight columns; forms the thin Q and R.  k_house_qr, a
-//                      column at a time, takes the shapes of two or three
-//                      reflectors and those that fit only without the panel's
-//                      workspace.
+//                      column at a time, takes the shapes of one or two
+//                      reflectors, of three with up to 256 rows, and those
+//                      that fit only without the panel's workspace.
 // Singular values descend.  One launch each, no host round trip.
 #include <cmath>
 #include <cstdlib>
